@@ -23,14 +23,14 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-fopenmp,-O3",
           "-I" + os.path.join(HERE, "..", "include")]
-SOURCES = ["topology.cpp", "basis.cpp", "kernels_assemble.cu", "kernels_pcg.cu", "capi.cu",
+SOURCES = ["topology.cpp", "basis.cpp", "kernels_assemble.cu", "kernels_pcg.cu", "kernels_pcg_resident.cu", "capi.cu",
            "noalloc.cu", "topology_gpu.cu", "kernels_ad.cu",
            "kernels_probe.cu", "kernels_pml.cu",
            "kernels_dist.cu", "kernels_weighted.cu", "kernels_tc.cu", "kernels_oriented.cu"]
 
 
 def _headers():
-    return [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".inc"))] + \
+    return [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh", ".inc"))] + \
         [os.path.join(HERE, "..", "include", "fortfem_gpu.h")]
 
 

@@ -149,6 +149,13 @@ struct DeviceSell {
   int2 *inc_range = nullptr; // per SELL row: its column's incidence range (the
                              // slice gather's, built on its first use)
   int grid = 0;
+  // largest share of a CTA of the grid under cta_slice (sell_shares)
+  int share_slices = 0;
+  int64_t share_entries = 0;
+  // slice cuts over 8 and 16 CTAs (9 + 17 ints, set by sell_shares) and the
+  // largest count of slices of a CTA under each
+  int *cluster_slice = nullptr;
+  int cluster_share[2] = {0, 0};
 };
 
 // Upload the slice structure (values left zero) and the CTA partition.
@@ -158,6 +165,9 @@ int upload_sell(const HostSell &h, int grid, DeviceSell &d);
 // warp, CTA-major) and woff (grid * 32 + 1) where each warp's list starts.
 void sell_partition(const int64_t *soff, int64_t n_slices, int grid, std::vector<int> &cs,
                     std::vector<int> &wslice, std::vector<int> &woff, int slice_cost = 256);
+// Record the largest CTA share of a partition in d, and cut the slices for the
+// cluster solves.
+int sell_shares(const int64_t *soff, const std::vector<int> &cs, DeviceSell &d);
 // Re-deal an uploaded operator's slices to CTAs and warps with another slice cost.
 int sell_repartition(DeviceSell &d, int slice_cost);
 void free_sell(DeviceSell &d);

@@ -35,7 +35,6 @@
 // solve continues in the FP64 loop from the current x; if the FP32 p^T A p is
 // not positive (condition number beyond FP32 reach, as for curl-curl
 // operators with a small mass term) the FP64 loop starts again from x = 0.
-#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -43,7 +42,7 @@
 #include <cstring>
 #include <mutex>
 
-#include "ffg_internal.h"
+#include "pcg_common.cuh"
 
 namespace ffg {
 
@@ -53,9 +52,6 @@ constexpr int kThreads = 1024;
 constexpr int kWarps = kThreads / 32;
 constexpr int kSlots = 4;
 constexpr int kPartialBatch = 8;   // partial loads in flight per lane
-constexpr int kResultDoubles = 16;
-constexpr int kMinWindow = 256;  // iterations before a plateau forces a reliable update
-constexpr unsigned long long kBarrierLimitNs = 4000000000ull;  // 4 s per barrier wait
 // Staged SpMV: every warp streams its slices through kStages shared-memory
 // buffers of kStageBytes (32 rows by as many columns as fit: values, then
 // column indices).  Measured on the 48^3 P2 system (FP32 + int16): 2 x 10
@@ -65,40 +61,6 @@ constexpr int kStageBytes = 10 * 32 * (4 + 2);                 // 1920 B
 constexpr int kStages = 2;                                   // chunks in flight per warp
 constexpr int kStageSmem = kWarps * kStages * kStageBytes;   // 120 KB per CTA
 constexpr unsigned long long kCopyLimitNs = 1000000000ull;   // 1 s per copy wait
-
-struct PcgParams {
-  int64_t n;
-  const int64_t *soff;
-  const int16_t *dcol;
-  const int *col;
-  const float *v32;
-  const __half *v16;  // FFG_PRECISION_MIXED16: FP16 operator, row r scaled by rs[r]
-  const float *rs;
-  const double *v64;
-  const float *d32;
-  const double *d64;
-  const int *cta_slice;
-  const int *wslice, *woff;  // per-warp slice lists of the cooperative grid
-  const double *b;
-  double *x;
-  double *r64;
-  float *rf, *zf, *pf, *qf;  // mixed mode: r, z = D^-1 r, p, q = A p
-  float *xf;                 // mixed mode: increment of x since it was last folded in
-  float2 *zpf0, *zpf1;       // mixed mode after a switch to direct A p: (z, p) pairs
-  double *rd, *qd;
-  double2 *zpd0, *zpd1;
-  double *partial;  // [2][kSlots][grid]
-  unsigned int *bar;
-  int *control;     // [0] error status
-  double *result;   // kResultDoubles
-  int precision, relative, max_it, max_updates, guard;
-  double tol, delta;
-  unsigned long long limit_ns;
-  // CTAs that solve this system: blockIdx.x - cta0 in [0, ncta).  With one
-  // CTA the system's slices are [0, n_slices) and barriers are CTA barriers.
-  int cta0, ncta, n_slices;
-  int staged;  // launched with kStageSmem bytes of dynamic shared memory
-};
 
 // Set when a warp's staged copy did not complete in time; every barrier
 // checks it, so the solve ends on the next one.
@@ -111,20 +73,10 @@ __shared__ unsigned g_mparity[kWarps];
 
 __device__ __forceinline__ int cta_of(const PcgParams &P) { return (int)blockIdx.x - P.cta0; }
 
-__device__ __forceinline__ unsigned long long globaltimer() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
-
 __device__ __forceinline__ unsigned int ld_acquire(const unsigned int *p) {
   unsigned int v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
-}
-
-__device__ __forceinline__ int ld_volatile_int(const int *p) {
-  return *reinterpret_cast<const volatile int *>(p);
 }
 
 // Bounded grid barrier.  Every CTA calls it the same number of times; the
@@ -300,10 +252,6 @@ __device__ __noinline__ double spmv_pairs(const PcgParams &P, const V *__restric
 }
 
 // ------------------------------------------------------ staged FP32 SpMV
-__device__ __forceinline__ unsigned smem_addr(const void *p) {
-  return (unsigned)__cvta_generic_to_shared(p);
-}
-
 __device__ __forceinline__ void mbar_init(unsigned long long *m) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(m)) : "memory");
 }
@@ -550,21 +498,6 @@ __device__ __forceinline__ void for_rows_even_batched(const PcgParams &P, L load
     }
   }
 }
-
-__device__ __forceinline__ bool is_finite_d(double x) { return isfinite(x); }
-
-struct Outcome {
-  int iterations = 0, updates = 0, converged = 0, status = FFG_OK, stagnated = 0, aborted = 0;
-  int restart = 0;  // the FP32 phase broke down: the FP64 loop starts again from x = 0
-  double true_res = 0.0, final_res = 0.0, bnorm = 0.0;
-};
-
-// Device time of the phases seen by CTA 0 (the others are symmetric):
-// SpMV work, wait at the following barrier, vector work, wait, and the
-// residual-replacement phases.
-struct Timing {
-  unsigned long long a = 0, aw = 0, b = 0, bw = 0, u = 0;
-};
 
 __device__ __forceinline__ unsigned long long stamp(const PcgParams &P) {
   return (cta_of(P) == 0 && threadIdx.x == 0) ? globaltimer() : 0ull;
@@ -1278,6 +1211,7 @@ int upload_sell(const HostSell &h, int grid, DeviceSell &d) {
   A((void **)&d.iperm, sizeof(int) * N);
   std::vector<int> cs, wslice, woff;
   sell_partition(h.soff.data(), h.n_slices, grid, cs, wslice, woff);
+  if (sell_shares(h.soff.data(), cs, d)) bad = true;
   A((void **)&d.cta_slice, sizeof(int) * (grid + 1));
   A((void **)&d.wslice, sizeof(int) * wslice.size());
   A((void **)&d.woff, sizeof(int) * woff.size());
@@ -1345,6 +1279,40 @@ void sell_partition(const int64_t *soff, int64_t n_slices, int grid, std::vector
   woff[(size_t)grid * kWarps] = (int)wslice.size();
 }
 
+int sell_shares(const int64_t *soff, const std::vector<int> &cs, DeviceSell &d) {
+  d.share_slices = 0;
+  d.share_entries = 0;
+  for (size_t b = 0; b + 1 < cs.size(); ++b) {
+    d.share_slices = std::max(d.share_slices, cs[b + 1] - cs[b]);
+    d.share_entries = std::max(d.share_entries, soff[cs[b + 1]] - soff[cs[b]]);
+  }
+  // contiguous ranges of about equal cost, a row weighing as much as eight
+  // entries (its share of the vector phases)
+  std::vector<int> cuts;
+  for (int k = 0; k < 2; ++k) {
+    const int c = 8 << k;
+    const int64_t ns = d.n_slices, weight = 8 * kSliceRows, total = soff[ns] + weight * ns;
+    int s = 0;
+    d.cluster_share[k] = 0;
+    for (int b = 0; b <= c; ++b) {
+      const int first = s;
+      while (s < ns && soff[s] + weight * s < total * b / c) ++s;
+      if (b == c) s = (int)ns;
+      cuts.push_back(s);
+      if (b > 0) d.cluster_share[k] = std::max(d.cluster_share[k], s - first);
+    }
+  }
+  if (!d.cluster_slice && cudaMalloc((void **)&d.cluster_slice, sizeof(int) * cuts.size()) != cudaSuccess) {
+    cudaGetLastError();
+    d.cluster_slice = nullptr;
+    return FFG_OUT_OF_MEMORY;
+  }
+  return cudaMemcpy(d.cluster_slice, cuts.data(), sizeof(int) * cuts.size(),
+                    cudaMemcpyHostToDevice) == cudaSuccess
+             ? FFG_OK
+             : FFG_CUDA_ERROR;
+}
+
 namespace {
 // val16 = FP16(val32 / s_r) with s_r the row's largest |val32| (1 for an
 // empty row); one thread per row walks the row's entries in its slice.
@@ -1406,6 +1374,7 @@ int sell_repartition(DeviceSell &d, int slice_cost) {
     return FFG_CUDA_ERROR;
   std::vector<int> cs, ws, wo;
   sell_partition(soff.data(), d.n_slices, d.grid, cs, ws, wo, slice_cost);
+  if (int st = sell_shares(soff.data(), cs, d)) return st;
   bool ok = cudaMemcpy(d.cta_slice, cs.data(), sizeof(int) * cs.size(), cudaMemcpyHostToDevice) ==
             cudaSuccess;
   if (!ws.empty())
@@ -1419,10 +1388,16 @@ int sell_repartition(DeviceSell &d, int slice_cost) {
 void free_sell(DeviceSell &d) {
   void *ptrs[] = {d.soff, d.dcol, d.col, d.val64, d.val32, d.val16, d.rscale, d.dinv64, d.dinv32,
                   d.perm, d.iperm,
-                  d.cta_slice, d.wslice, d.woff, d.inc_range};
+                  d.cta_slice, d.wslice, d.woff, d.inc_range, d.cluster_slice};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   d = DeviceSell();
+}
+
+// Partial sums of pcg_kernel ([2][kSlots][grid] doubles) or messages of the
+// resident kernel.
+static size_t partial_bytes(int grid) {
+  return std::max(2 * kSlots * (size_t)grid * sizeof(double), pcg_resident_message_bytes(grid));
 }
 
 int solve_work_alloc(SolveWork &w, int64_t n, int grid) {
@@ -1446,7 +1421,7 @@ int solve_work_alloc(SolveWork &w, int64_t n, int grid) {
   A((void **)&w.xf, N * sizeof(float));
   A((void **)&w.zpf0, N * sizeof(float2));
   A((void **)&w.zpf1, N * sizeof(float2));
-  A((void **)&w.partial, 2 * kSlots * (size_t)grid * sizeof(double));
+  A((void **)&w.partial, partial_bytes(grid));
   A((void **)&w.barrier, 64);
   A((void **)&w.control, 64);
   A((void **)&w.result, kResultDoubles * sizeof(double));
@@ -1520,6 +1495,10 @@ PcgParams make_params(const DeviceSell &A, const double *b, double *x,
   P.ncta = A.grid;
   P.n_slices = (int)A.n_slices;
   P.staged = 0;
+  P.cluster_slice = A.cluster_slice;
+  P.cluster_share[0] = A.cluster_share[0];
+  P.cluster_share[1] = A.cluster_share[1];
+  P.share_slices = A.share_slices;
   return P;
 }
 }  // namespace
@@ -1531,17 +1510,26 @@ int pcg_launch(const DeviceSell &A, const double *b, double *x, const ffg_solver
     return FFG_INVALID_INPUT;
   }
   PcgParams P = make_params(A, b, x, opts, w);
-  P.staged = staged_smem_ready() ? 1 : 0;
-  if (cudaMemsetAsync(w.barrier, 0, 64, stream) != cudaSuccess) return FFG_CUDA_ERROR;
   if (cudaMemsetAsync(w.control, 0, 64, stream) != cudaSuccess) return FFG_CUDA_ERROR;
   if (cudaMemsetAsync(w.result, 0, kResultDoubles * sizeof(double), stream) != cudaSuccess)
     return FFG_CUDA_ERROR;
-  void *args[] = {&P};
-  cudaError_t e = cudaLaunchCooperativeKernel((const void *)pcg_kernel, dim3(w.grid),
-                                              dim3(kThreads), args,
-                                              P.staged ? kStageSmem : 0, stream);
+  cudaError_t e;
+  const int cluster = pcg_cluster_size(A, opts.precision, false);
+  if (cluster) {
+    e = pcg_launch_cluster(1, &P, cluster, false, false, stream);
+  } else if (const size_t pool = pcg_grid_resident(A, opts.precision)) {
+    if (cudaMemsetAsync(w.partial, 0, pcg_resident_message_bytes(w.grid), stream) != cudaSuccess)
+      return FFG_CUDA_ERROR;
+    e = pcg_launch_resident(P, pool, stream);
+  } else {
+    if (cudaMemsetAsync(w.barrier, 0, 64, stream) != cudaSuccess) return FFG_CUDA_ERROR;
+    P.staged = staged_smem_ready() ? 1 : 0;
+    void *args[] = {&P};
+    e = cudaLaunchCooperativeKernel((const void *)pcg_kernel, dim3(w.grid), dim3(kThreads), args,
+                                    P.staged ? kStageSmem : 0, stream);
+  }
   if (e != cudaSuccess) {
-    msg = std::string("cooperative launch failed: ") + cudaGetErrorString(e);
+    msg = std::string("solve launch failed: ") + cudaGetErrorString(e);
     cudaGetLastError();
     return FFG_CUDA_ERROR;
   }
@@ -1563,13 +1551,37 @@ int pcg_launch_batch(int count, const DeviceSell *const *A, const double *const 
     }
   static_assert(sizeof(PcgBatch) <= 32000, "kernel parameter block too large");
   const int staged = staged_smem_ready() ? 1 : 0;
+  // systems by kernel: a cluster each, or one CTA each; the largest first, so
+  // that the longest solves start first
+  std::vector<int> order((size_t)count);
+  for (int i = 0; i < count; ++i) order[i] = i;
+  std::stable_sort(order.begin(), order.end(),
+                   [&](int i, int j) { return A[i]->padded > A[j]->padded; });
+  std::vector<PcgParams> clustered[2], single;
+  for (int i : order) {
+    const PcgParams P = make_params(*A[i], b[i], x[i], opts, *w[i]);
+    const int c = pcg_cluster_size(*A[i], opts.precision, true);
+    w[i]->control_host[0] = 0;
+    (c == 16 ? clustered[0] : c == 8 ? clustered[1] : single).push_back(P);
+  }
+  bool overlap = false;
+  for (int k = 0; k < 2; ++k) {
+    if (clustered[k].empty()) continue;
+    const cudaError_t e = pcg_launch_cluster((int)clustered[k].size(), clustered[k].data(),
+                                             k ? 8 : 16, true, overlap, stream);
+    overlap = true;
+    if (e != cudaSuccess) {
+      msg = std::string("batch launch failed: ") + cudaGetErrorString(e);
+      cudaGetLastError();
+      return FFG_CUDA_ERROR;
+    }
+  }
   PcgBatch B;
-  for (int c0 = 0; c0 < count; c0 += kMaxBatch) {
-    const int m = std::min(kMaxBatch, count - c0);
+  for (int c0 = 0; c0 < (int)single.size(); c0 += kMaxBatch) {
+    const int m = std::min(kMaxBatch, (int)single.size() - c0);
     for (int i = 0; i < m; ++i) {
-      B.sys[i] = make_params(*A[c0 + i], b[c0 + i], x[c0 + i], opts, *w[c0 + i]);
+      B.sys[i] = single[c0 + i];
       B.sys[i].staged = staged;
-      w[c0 + i]->control_host[0] = 0;
     }
     pcg_batch_kernel<<<m, kThreads, staged ? kStageSmem : 0, stream>>>(B);
     const cudaError_t e = cudaGetLastError();
@@ -1577,12 +1589,11 @@ int pcg_launch_batch(int count, const DeviceSell *const *A, const double *const 
       msg = std::string("batch launch failed: ") + cudaGetErrorString(e);
       return FFG_CUDA_ERROR;
     }
-    for (int i = 0; i < m; ++i)
-      if (cudaMemcpyAsync(w[c0 + i]->result_host, w[c0 + i]->result,
-                          kResultDoubles * sizeof(double), cudaMemcpyDeviceToHost,
-                          stream) != cudaSuccess)
-        return FFG_CUDA_ERROR;
   }
+  for (int i = 0; i < count; ++i)
+    if (cudaMemcpyAsync(w[i]->result_host, w[i]->result, kResultDoubles * sizeof(double),
+                        cudaMemcpyDeviceToHost, stream) != cudaSuccess)
+      return FFG_CUDA_ERROR;
   return FFG_OK;
 }
 

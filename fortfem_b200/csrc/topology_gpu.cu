@@ -801,6 +801,7 @@ int build_topology_device(Topology &t, int mode, const uint8_t *mask, int grid,
   FFG_TRY(cudaMemcpy(hsoff.data(), soff.p, sizeof(int64_t) * hsoff.size(), cudaMemcpyDeviceToHost));
   std::vector<int> cs, hws, hwo;
   sell_partition(hsoff.data(), S.n_slices, grid, cs, hws, hwo);
+  if (int st = sell_shares(hsoff.data(), cs, S)) return st;
   FFG_ALLOC(cta, cs.size());
   FFG_ALLOC(wsl, std::max<size_t>(hws.size(), 1));
   FFG_ALLOC(wof, hwo.size());

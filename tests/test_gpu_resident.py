@@ -1,0 +1,90 @@
+"""The on-chip PCG kernels (a cluster per system, the whole grid with the
+operator in shared memory) at the edges of their partitions: fewer slices than
+CTAs, partial last slices, rows long enough to be split, int32 columns,
+operators larger than shared memory; FP64 and mixed.
+
+The systems are strictly diagonally dominant, |a_ii| >= 2 sum |a_ij|, so
+the Jacobi-scaled operator has its spectrum in [1/2, 3/2] and the solution's
+relative error (in the scaled norm) is at most 3 times the relative residual;
+the row scales spread over a factor 4, hence 12 tol = 1.2e-9 below.
+"""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+import fortfem_b200 as ff
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-10
+
+
+def dominant(n, per_row, span, seed, long_rows=0):
+    """Symmetric, 2 x diagonally dominant, about per_row entries a row within `span`."""
+    rng = np.random.default_rng(seed)
+    m = n * max(per_row - 1, 0) // 2
+    i = rng.integers(0, n, m)
+    j = np.clip(i + rng.integers(-span, span + 1, m), 0, n - 1)
+    if long_rows:
+        rows = rng.choice(n, long_rows, replace=False)
+        i = np.concatenate([i] + [np.full(min(n, 300), r) for r in rows])
+        j = np.concatenate([j] + [rng.choice(n, min(n, 300), replace=False) for _ in rows])
+    v = rng.standard_normal(len(i))
+    keep = i != j
+    A = sp.coo_matrix((v[keep], (i[keep], j[keep])), shape=(n, n)).tocsr()
+    A = A + A.T
+    d = np.maximum(2.0 * np.asarray(abs(A).sum(axis=1)).ravel(), 1.0) * rng.uniform(1.0, 4.0, n)
+    return (A + sp.diags(d)).tocsc()
+
+
+def solve(A, b, precision):
+    A.sort_indices()
+    M = ff.CscMatrix(*A.shape, A.indptr.astype(np.int64), A.indices.astype(np.int32), A.data)
+    x = np.zeros(len(b))
+    st = ff.solve_sparse(M, b, x, ff.solver_options(
+        method="pcg", preconditioner="jacobi", tolerance=TOL, precision=precision,
+        max_iterations=10000, breakdown_guard="spd"))
+    return x, st
+
+
+CASES = [
+    # rows, entries a row, span, rows of 300 entries
+    (1, 1, 1, 0), (2, 2, 1, 0), (31, 5, 30, 0), (33, 5, 32, 0), (257, 7, 40, 0),
+    (511, 300, 510, 0),       # 16 slices, every one split into parts
+    (513, 7, 512, 3),         # 17 slices over 16 CTAs, a few long rows
+    (4097, 9, 4000, 5),       # two sigma windows
+    (12001, 25, 12000, 4),    # cluster (mixed) or grid (FP64)
+    (30011, 7, 180, 0),       # banded: the cluster exchanges its borders only
+    (40009, 12, 40000, 2),    # grid, int32 columns
+    (70001, 60, 3000, 0),     # grid, part of the operator left in L2
+    (260003, 5, 500, 0),      # grid, many rows a CTA
+]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n,per_row,span,long_rows", CASES)
+def test_resident_solve_matches_direct(n, per_row, span, long_rows, precision):
+    A = dominant(n, per_row, span, n, long_rows)
+    xs = np.random.default_rng(n + 1).standard_normal(n)
+    b = A @ xs
+    x, st = solve(A, b, precision)
+    assert st.converged and st.true_relative_residual <= 1.01 * TOL
+    assert np.linalg.norm(x - xs) <= 12 * TOL * np.linalg.norm(xs)
+    # the same bits again
+    y, _ = solve(A, b, precision)
+    assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_resident_hard_system_falls_back_like_the_staged_kernel(precision):
+    """cond ~ 1e11: the mixed loop leaves FP32 (direct form, FP64 continuation) and
+    both precisions end on the true residual they report."""
+    n = 600
+    A = sp.diags([np.full(n - 1, -1.0), np.full(n, 2.0), np.full(n - 1, -1.0)], [-1, 0, 1])
+    A = (A @ A + 1e-9 * sp.identity(n)).tocsc()
+    b = np.ones(n)
+    x, st = solve(A, b, precision)
+    res = np.linalg.norm(b - A @ x) / np.linalg.norm(b)
+    assert np.isfinite(x).all()
+    # FP64 rounding of one evaluation of b - A x
+    floor = 1e-16 * np.linalg.norm(np.abs(A) @ np.abs(x)) / np.linalg.norm(b)
+    assert abs(res - st.true_relative_residual) <= 1e-3 * res + 20 * floor
