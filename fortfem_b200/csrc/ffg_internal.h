@@ -156,6 +156,7 @@ struct DeviceSell {
   // largest count of slices of a CTA under each
   int *cluster_slice = nullptr;
   int cluster_share[2] = {0, 0};
+  std::vector<int64_t> host_soff;  // soff on the host (set by sell_shares)
 };
 
 // Upload the slice structure (values left zero) and the CTA partition.
@@ -210,10 +211,10 @@ int pcg_launch(const DeviceSell &A, const double *b, double *x, const ffg_solver
 int pcg_launch_batch(int count, const DeviceSell *const *A, const double *const *b,
                      double *const *x, const ffg_solver_options &opts, SolveWork *const *w,
                      cudaStream_t stream, std::string &msg);
-// Independent systems in shared cooperative launches, each on a group of
-// pcg_group_ctas(n) CTAs (16384 rows per CTA, at least 2, at most the grid);
-// consecutive systems share a launch while their groups fit the grid.
-int pcg_group_ctas(int64_t n, int grid);
+// Independent systems in shared cooperative launches, each on a group of CTAs
+// whose size depends on the system alone: a k-th of the grid whose shared
+// memory holds the operator (pcg_group_shape); systems that no group holds run
+// one after another on the whole device.
 int pcg_launch_groups(int count, const DeviceSell *const *A, const double *const *b,
                       double *const *x, const ffg_solver_options &opts, SolveWork *const *w,
                       cudaStream_t stream, std::string &msg);

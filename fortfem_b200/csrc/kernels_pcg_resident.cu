@@ -7,8 +7,8 @@
 // vector (the operand of A) and the partial sums of the dot products between
 // CTAs.  What bounds it is latency: two reductions an iteration.  Per
 // iteration and solve, measured on a B200 against the kernels it replaces:
-// P1, 3,969 rows, 2.6 us (14 us with 148 CTAs and grid barriers); P1, 85,800
-// rows, 8.3 us (13.6); P2, 71,955 rows, 11.5 us (20.0); a batch of 12 systems of
+// P1, 3,969 rows, 2.5 us (14 us with 148 CTAs and grid barriers); P1, 85,800
+// rows, 7.5 us (13.6); P2, 71,955 rows, 10.5 us (20.0); a batch of 12 systems of
 // 961 to 21,025 rows 3.5 ms (41 ms with one CTA a system).
 //
 // * pcg_cluster_kernel: a thread-block cluster per system.  Every CTA holds a
@@ -18,9 +18,9 @@
 //   st.async messages counted by mbarriers.  Clusters wait on nothing outside
 //   themselves, so launches of this kernel may overlap.
 // * pcg_resident_kernel: one cooperative grid per system.  The published vector
-//   is in global memory (L2); a reduction is an all-to-all of 32-byte messages,
-//   one per CTA, polled by every CTA: the message carries the partial sums and
-//   is its own arrival flag.
+//   is in global memory (L2); a reduction is an all-to-all of messages, one per
+//   CTA, polled by every CTA: the message carries the partial sums and is its
+//   own arrival flag.
 //
 // Slices that do not fit stay in global memory and are read from L2.  The
 // recurrences, stopping rules and fallbacks are those of kernels_pcg.cu; the
@@ -44,6 +44,11 @@ constexpr int kMaxCluster = 16;
 constexpr int kVals = 2;           // values of one reduction, at most
 constexpr int kPoll = 5;            // messages a lane polls: up to 160 CTAs
 constexpr int kBatch = 8;          // columns of a row in flight
+// Before the grid's first poll of a sync: the polls of 148 CTAs hit the same few
+// L2 lines and slow the messages and the fences they wait for (P1, 85,800
+// rows: 9.4 us an iteration without naps, 7.8 with these; between polls a nap
+// gained nothing).
+constexpr unsigned kNapSums = 200, kNapData = 700;  // ns
 constexpr int kLimitEvery = 64;    // iterations between looks at the wall limit
 constexpr int kPoolMax = 225 * 1024;
 
@@ -209,10 +214,14 @@ struct ClusterSync {
   }
 };
 
-// A grid message: two doubles, each split in halves that carry the phase, so
-// that every 8-byte element validates itself: element 2 s + h is half h of
-// value s above the 32-bit tag.
-template <int NT>
+// A grid message: 16 bytes per value, [parity][value][CTA], a double split in
+// halves that each carry the phase below them, so that every 8-byte element
+// validates itself.  The polled sectors are what a sync costs beyond latency:
+// with the two values of a CTA side by side, 32 bytes read by two loads, a sync
+// with two sums took 4.7 us where this layout takes 3.4.
+// kGroup: instantiated once per kernel (a function that two kernels share finds
+// the shared memory through an indirection: 15 % of an iteration).
+template <int NT, bool kGroup>
 struct GridSync {
   int rank, n;
   unsigned phase;
@@ -229,6 +238,7 @@ struct GridSync {
   template <int NV, bool kData>
   __device__ __forceinline__ bool go(const double (&v)[kVals], double (&out)[kVals]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int NM = NV > 0 ? NV : 1;  // values a message carries
     ++phase;
     double x = 0.0;
     if (NV > 0) x = block_sums<NV, NT>(v);
@@ -247,11 +257,14 @@ struct GridSync {
           e[2 * s] = (bits << 32) | phase;
           e[2 * s + 1] = (bits & 0xffffffff00000000ull) | phase;
         }
-        asm volatile("st.relaxed.gpu.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(msg + 4 * rank),
-                     "l"(e[0]), "l"(e[1]), "l"(e[2]), "l"(e[3])
-                     : "memory");
+#pragma unroll
+        for (int s = 0; s < NM; ++s)
+          asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(msg + 2 * (s * n + rank)),
+                       "l"(e[2 * s]), "l"(e[2 * s + 1])
+                       : "memory");
       }
       __syncwarp();
+      __nanosleep(kData ? kNapData : kNapSums);
       unsigned long long e[kPoll][4], t0 = 0;
       unsigned spins = 0;
       bool good = true;
@@ -260,16 +273,18 @@ struct GridSync {
 #pragma unroll
         for (int k = 0; k < kPoll; ++k) {
           if (lane + 32 * k < n)
-            asm volatile("ld.relaxed.gpu.global.v4.b64 {%0, %1, %2, %3}, [%4];"
-                         : "=l"(e[k][0]), "=l"(e[k][1]), "=l"(e[k][2]), "=l"(e[k][3])
-                         : "l"(msg + 4 * (lane + 32 * k))
-                         : "memory");
+#pragma unroll
+            for (int s = 0; s < NM; ++s)
+              asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];"
+                           : "=l"(e[k][2 * s]), "=l"(e[k][2 * s + 1])
+                           : "l"(msg + 2 * (s * n + lane + 32 * k))
+                           : "memory");
         }
 #pragma unroll
         for (int k = 0; k < kPoll; ++k)
           if (lane + 32 * k < n)
 #pragma unroll
-            for (int j = 0; j < (NV > 0 ? 2 * NV : 1); ++j) here = here && (unsigned)e[k][j] == phase;
+            for (int j = 0; j < 2 * NM; ++j) here = here && (unsigned)e[k][j] == phase;
         if (__all_sync(0xffffffffu, here)) break;
         if ((++spins & 255u) == 0) {
           if (t0 == 0) t0 = globaltimer();
@@ -391,17 +406,19 @@ struct Solve {
       const SliceEnt t = tab[i];
       if (t.off < 0) continue;
       const int row = row_of(32 * i + lane);
+      with_columns(row, [&](auto col) {
 #pragma unroll 4
-      for (int j = 0; j < t.len; ++j) {
-        const int64_t e = t.goff + (int64_t)j * 32 + lane;
-        const int d = t.off + j * 32 + lane;
-        sv[d] = __ldcs(val + e);
-        if (IDX == kAbs32) reinterpret_cast<int *>(midx)[d] = __ldcs(gP.col + e);
-        else if (IDX == kRel16) reinterpret_cast<int16_t *>(midx)[d] = __ldcs(gP.dcol + e);
-        else
-          reinterpret_cast<uint16_t *>(midx)[d] =
-              (uint16_t)(gP.dcol ? row + (int)__ldcs(gP.dcol + e) : __ldcs(gP.col + e));
-      }
+        for (int j = 0; j < t.len; ++j) {
+          const int64_t e = t.goff + (int64_t)j * 32 + lane;
+          const int d = t.off + j * 32 + lane;
+          const V a = __ldcs(val + e);
+          const int c = col(e);
+          sv[d] = a;
+          if (IDX == kAbs32) reinterpret_cast<int *>(midx)[d] = c;
+          else if (IDX == kRel16) reinterpret_cast<int16_t *>(midx)[d] = (int16_t)(c - row);
+          else reinterpret_cast<uint16_t *>(midx)[d] = (uint16_t)c;
+        }
+      });
     }
     __syncthreads();
     if constexpr (IDX == kAbs16) exchange_plan(need);
@@ -419,13 +436,14 @@ struct Solve {
     for (int i = warp; i < nsl; i += NT / 32) {
       const SliceEnt t = tab[i];
       const int row = row_of(32 * i + lane);
+      if (t.off >= 0) {
 #pragma unroll 4
-      for (int j = 0; j < t.len; ++j) {
-        const int64_t e = t.goff + (int64_t)j * 32 + lane;
-        const int c = t.off >= 0 ? column(row, t.off + j * 32 + lane)
-                      : gP.dcol  ? row + (int)gP.dcol[e]
-                                 : gP.col[e];
-        need[c >> 5] = 1;
+        for (int j = 0; j < t.len; ++j) need[column(row, t.off + j * 32 + lane) >> 5] = 1;
+      } else {
+        with_columns(row, [&](auto col) {
+#pragma unroll 4
+          for (int j = 0; j < t.len; ++j) need[col(t.goff + (int64_t)j * 32 + lane) >> 5] = 1;
+        });
       }
     }
     __syncthreads();
@@ -475,6 +493,20 @@ struct Solve {
     return reinterpret_cast<const uint16_t *>(midx)[d];
   }
 
+  // Calls f with what reads the column of an operator entry from global memory
+  // (one instance of f's loop per index width: a branch in the loop would end
+  // the overlap of its loads).
+  template <class F> __device__ __forceinline__ void with_columns(int row, F f) {
+    if (IDX == kRel16 || (IDX == kAbs16 && gP.dcol)) {
+      const int16_t *dcol = gP.dcol;
+      f([=](int64_t e) { return row + (int)dcol[e]; });
+    }
+    if (IDX == kAbs32 || (IDX == kAbs16 && !gP.dcol)) {
+      const int *col = gP.col;
+      f([=](int64_t e) { return col[e]; });
+    }
+  }
+
   // f(j, true) for the columns j in [j0, j1), kBatch at a time so that their
   // loads are in flight together; the last batch is filled up with f(j1 - 1, false).
   template <class F> __device__ __forceinline__ void batches(int j0, int j1, F f) {
@@ -516,11 +548,12 @@ struct Solve {
           acc += a * z[column(row, d)];
         });
       } else {
-        batches(j0, j1, [&](int j, bool in) {
-          const int64_t e = t.goff + (int64_t)j * 32 + lane;
-          const int c = gP.dcol ? row + (int)gP.dcol[e] : gP.col[e];
-          const V a = in ? val[e] : V(0);
-          acc += a * z[c];
+        with_columns(row, [&](auto col) {
+          batches(j0, j1, [&](int j, bool in) {
+            const int64_t e = t.goff + (int64_t)j * 32 + lane;
+            const V a = in ? val[e] : V(0);  // again next iteration: kept in L2
+            acc += a * z[col(e)];
+          });
         });
       }
       if (t.parts > 1) part[(t.part0 + k) * 32 + lane] = acc;
@@ -540,30 +573,40 @@ struct Solve {
     return dot;
   }
 
-  // r64 = b - A x with the FP64 operator (x in global memory); with with_p also
+  // r64 = b - A x with the FP64 operator (x in global memory); with kP also
   // q = A p from the published p, in FP64.  Returns the thread's share of (r64, r64).
-  __device__ __forceinline__ double residual(bool with_p, float *q) {
+  template <bool kP>
+  __device__ __forceinline__ double residual(float *q) {
     const float *p = published<float>();
+    const double *x = gP.x, *v64 = gP.v64;
     double2 *part = reinterpret_cast<double2 *>(scratch);
     double dot = 0.0;
     auto fin = [&](int li, int row, double ax, double ap) {
       const double r = gP.b[row] - ax;
       gP.r64[row] = r;
-      if (with_p) q[li] = (float)ap;
+      if (kP) q[li] = (float)ap;
       dot += r * r;
     };
     for_items([&](int i, const SliceEnt &t, int k, int j0, int j1) {
       const int li = 32 * i + lane, row = row_of(li);
       double ax = 0.0, ap = 0.0;
-      batches(j0, j1, [&](int j, bool in) {
-        const int64_t e = t.goff + (int64_t)j * 32 + lane;
-        const int c = t.off >= 0 ? column(row, t.off + j * 32 + lane)
-                      : gP.dcol  ? row + (int)__ldcs(gP.dcol + e)
-                                 : __ldcs(gP.col + e);
-        const double v = in ? __ldcs(gP.v64 + e) : 0.0;
-        ax += v * gP.x[c];
-        if (with_p) ap += v * (double)p[c];
-      });
+      auto add = [&](int64_t e, int c, bool in) {
+        const double v = in ? __ldcs(v64 + e) : 0.0;
+        ax += v * x[c];
+        if (kP) ap += v * (double)p[c];
+      };
+      if (t.off >= 0) {
+        batches(j0, j1, [&](int j, bool in) {
+          add(t.goff + (int64_t)j * 32 + lane, column(row, t.off + j * 32 + lane), in);
+        });
+      } else {
+        with_columns(row, [&](auto col) {
+          batches(j0, j1, [&](int j, bool in) {
+            const int64_t e = t.goff + (int64_t)j * 32 + lane;
+            add(e, col(e), in);
+          });
+        });
+      }
       if (t.parts > 1) part[(t.part0 + k) * 32 + lane] = make_double2(ax, ap);
       else if (row < gP.n) fin(li, row, ax, ap);
     });
@@ -586,7 +629,7 @@ struct Solve {
   }
 
   __device__ __forceinline__ bool residual_norms(double (&red)[kVals]) {
-    double part[kVals] = {residual(false, nullptr), 0.0};
+    double part[kVals] = {residual<false>(nullptr), 0.0};
     for_rows([&](int, int row) {
       const double bb = gP.b[row];
       part[1] += bb * bb;
@@ -705,7 +748,7 @@ struct Solve {
         restart = true;
         for_rows([&](int li, int row) { gP.x[row] = x[li]; });
         if (!barrier()) { o.aborted = 1; return; }
-        part[0] = residual(false, nullptr);
+        part[0] = residual<false>(nullptr);
         if (!S.template sums<1>(part, red)) { o.aborted = 1; return; }
         true_res = sqrt(red[0]);
         est2 = red[0];
@@ -733,7 +776,7 @@ struct Solve {
     t0 = stamp();
     if (rnorm > target) for_rows([&](int li, int row) { gP.x[row] = x[li]; });
     if (!barrier()) { o.aborted = 1; return; }
-    part[0] = residual(false, nullptr);
+    part[0] = residual<false>(nullptr);
     if (!S.template sums<1>(part, red)) { o.aborted = 1; return; }
     tm.u += stamp() - t0;
     o.true_res = sqrt(red[0]);
@@ -874,7 +917,7 @@ struct Solve {
       }
       if (!barrier()) { o.aborted = 1; return; }
       unfolded = false;
-      part[0] = residual(!direct, q);
+      part[0] = direct ? residual<false>(nullptr) : residual<true>(q);
       if (!S.template sums<1>(part, red)) { o.aborted = 1; return; }
       true_res = sqrt(red[0]);
       if (true_res <= target) { converged = 1; tm.u += stamp() - t0; break; }
@@ -914,7 +957,7 @@ struct Solve {
     }
     if (o.stagnated) return;  // the FP64 continuation measures its own residual
     t0 = stamp();
-    part[0] = residual(false, nullptr);
+    part[0] = residual<false>(nullptr);
     if (!S.template sums<1>(part, red)) { o.aborted = 1; return; }
     tm.u += stamp() - t0;
     o.true_res = sqrt(red[0]);
@@ -934,21 +977,24 @@ struct Solve {
     lane = threadIdx.x & 31;
     warp = threadIdx.x >> 5;
     // Columns of a part: small enough that the slices spread over the warps,
-    // whole slices where there are many of them a warp.
-    const int chunk = nsl >= 2 * (NT / 32) ? 32 : 16;
+    // whole slices where there are many of them a warp, and more where the
+    // items and their scratch would not fit (P4, 132,651 rows: whole slices
+    // there cost one CTA 37 us where the others took 12).  Items in slice
+    // order, at the pool's end (its start holds the published vector's replica).
     for (int i = tid; i < nsl; i += NT) {
       const int s = s0 + i;
       const int64_t g = gP.soff[s];
-      const int len = (int)((gP.soff[s + 1] - g) / kSliceRows);
-      const int parts = len <= chunk + chunk / 4 ? 1 : (len + chunk - 1) / chunk;
-      const int cols = ((len + parts - 1) / parts + kBatch - 1) / kBatch * kBatch;
-      tab[i] = SliceEnt{g, -1, len, 0, parts, cols};
+      tab[i] = SliceEnt{g, -1, (int)((gP.soff[s + 1] - g) / kSliceRows), 0, 1, 0};
     }
-    // items in slice order, at the pool's end (its start holds the published
-    // vector's replica); without room for them and their scratch the slices
-    // stay whole
-    __syncthreads();
-    for (int pass = 0; pass < 2; ++pass) {
+    for (int chunk = nsl >= 2 * (NT / 32) ? 32 : 16;; chunk *= 2) {
+      const bool last = chunk > kMaxColumnLength;
+      for (int i = tid; i < nsl; i += NT) {
+        const int len = tab[i].len;
+        const int parts = last || len <= chunk + chunk / 4 ? 1 : (len + chunk - 1) / chunk;
+        tab[i].parts = parts;
+        tab[i].cols = parts == 1 ? len : ((len + parts - 1) / parts + kBatch - 1) / kBatch * kBatch;
+      }
+      __syncthreads();
       if (warp == 0) {
         int sum = 0, rows = 0;
         for (int i0 = 0; i0 < nsl; i0 += 32) {
@@ -979,12 +1025,7 @@ struct Solve {
       scratch_rows = gSh.rows;
       const size_t extra = (size_t)(items - nsl) * sizeof(unsigned) +
                            (size_t)scratch_rows * 32 * sizeof(double2);
-      if (pass > 0 || extra <= h.part_bytes) break;
-      __syncthreads();
-      for (int i = tid; i < nsl; i += NT) {
-        tab[i].parts = 1;
-        tab[i].cols = tab[i].len;
-      }
+      if (last || extra <= h.part_bytes) break;
       __syncthreads();
     }
     const unsigned bytes = (unsigned)((items * sizeof(unsigned) + 127) & ~(size_t)127);
@@ -1135,7 +1176,48 @@ __global__ void __launch_bounds__(kGridThreads, 1)
   const int c = (int)blockIdx.x, s0 = gP.cta_slice[c];
   const int nsl = gP.cta_slice[c + 1] - s0;
   const Share h{s0, nsl, nsl, pool_bytes, (unsigned)gP.part_bytes};
-  run_solve<GridSync<kGridThreads>, false, kGridThreads>(h, GridSync<kGridThreads>{c, gP.ncta, 0u});
+  using Sync = GridSync<kGridThreads, false>;
+  run_solve<Sync, false, kGridThreads>(h, Sync{c, gP.ncta, 0u});
+}
+
+// Slice where CTA r of a group of G starts: equal cost, a slice costing its
+// entries and kGroupSliceCost for its rows.
+constexpr int kGroupSliceCost = 256;
+__host__ __device__ inline int group_cut(const int64_t *soff, int64_t n_slices, int r, int G) {
+  const int64_t target =
+      (soff[n_slices] + (int64_t)kGroupSliceCost * n_slices) * (int64_t)r / G;
+  int64_t lo = 0, hi = n_slices;  // first slice whose cost before it reaches the target
+  while (lo < hi) {
+    const int64_t m = (lo + hi) / 2;
+    if (soff[m] + (int64_t)kGroupSliceCost * m < target) lo = m + 1;
+    else hi = m;
+  }
+  return r >= G ? (int)n_slices : (int)lo;
+}
+
+// Several systems in one cooperative launch, system i on CTAs first[i] ..
+// first[i + 1] - 1.  A group's sync waits only on its own CTAs, which the launch
+// makes resident together.
+struct GroupBatch {
+  PcgParams sys[kMaxResidentGroups];
+  int first[kMaxResidentGroups + 1];
+  int count;
+};
+__global__ void __launch_bounds__(kGridThreads, 1)
+    pcg_resident_group_kernel(const __grid_constant__ GroupBatch B) {
+  int i = 0;
+  while (i + 1 < B.count && B.first[i + 1] <= (int)blockIdx.x) ++i;
+  if (threadIdx.x == 0) {
+    gP = B.sys[i];
+    gSh.ok = 1;
+  }
+  __syncthreads();
+  const int c = (int)blockIdx.x - B.first[i];
+  const int s0 = group_cut(gP.soff, gP.n_slices, c, gP.ncta);
+  const int nsl = group_cut(gP.soff, gP.n_slices, c + 1, gP.ncta) - s0;
+  const Share h{s0, nsl, nsl, kPoolMax, (unsigned)gP.part_bytes};
+  using Sync = GridSync<kGridThreads, true>;
+  run_solve<Sync, false, kGridThreads>(h, Sync{c, gP.ncta, 0u});
 }
 
 // Shared memory beside the operator: the slice and item tables, five vectors
@@ -1161,9 +1243,10 @@ int resident_ready() {
   std::lock_guard<std::mutex> lock(mu);
   if (state[dev] == 0) {
     state[dev] = -1;
-    bool ok = cudaFuncSetAttribute((const void *)pcg_resident_kernel,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   kPoolMax) == cudaSuccess;
+    bool ok = true;
+    for (const void *f : {(const void *)pcg_resident_kernel, (const void *)pcg_resident_group_kernel})
+      ok = ok && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kPoolMax) ==
+                     cudaSuccess;
     int top = kMaxCluster;
     auto cluster_kernel = [&](auto kern, int threads) {
       ok = ok &&
@@ -1235,13 +1318,14 @@ int pcg_cluster_size(const DeviceSell &A, int precision, bool batched) {
   return A.padded <= (fp64 ? 280000 : 450000) ? c : 0;
 }
 
-// The grid kernel where the operator fits the chip, and beyond that while a CTA
-// has at most kGridSlices slices: there the staged kernel, which gives a slice
-// to one warp, leaves warps idle (P3, 73,964 rows, 3.3 M entries, FP64: 20.2
-// against 10.1 ms; P4, 103,823 rows, 7.1 M entries, mixed: 35.2 against 16.3
-// ms), and past it the staged copies win (P2, 357,911 rows, mixed: 16.0
-// against 19.9 ms).
-constexpr int kGridSlices = 40;
+// The grid kernel where the operator fits the chip, and beyond that while it
+// stays in L2 between iterations (resident part + L2, solve time against the
+// staged kernel): P2, 250,047 rows, FP64 (69 MB) 14.3 / 16.5 ms, 357,911 rows
+// mixed (59 MB) 14.4 / 16.0, FP64 (98 MB) 35 / 23; 493,039 rows mixed (82 MB)
+// 21.1 / 19.9.  The staged kernel gives a slice to one warp of 32, so with
+// fewer slices a CTA than that the line lies higher: P4, 132,651 rows, mixed
+// (55 MB) 20.0 / 37.5 ms, FP64 (91 MB) 39 / 64.
+constexpr size_t kGridL2Bytes = 75000000, kGridL2BytesFew = 95000000;
 
 size_t pcg_grid_resident(const DeviceSell &A, int precision) {
   if (precision == FFG_PRECISION_MIXED16 || A.n < 1 || A.grid > 32 * kPoll) return 0;
@@ -1249,11 +1333,63 @@ size_t pcg_grid_resident(const DeviceSell &A, int precision) {
   const bool fp64 = precision == FFG_PRECISION_FP64;
   const size_t fixed = loops_bytes(A.share_slices, A.n_slices, fp64, false);
   if (fixed > (size_t)kPoolMax) return 0;
-  // the operator and about a quarter more for the parts of long slices
-  const size_t need =
-      fixed + (size_t)A.share_entries * ((fp64 ? 8 : 4) + (A.dcol ? 2 : 4)) * 5 / 4;
-  if (need > (size_t)kPoolMax && A.share_slices > kGridSlices) return 0;
+  // the operator as this precision's loop keeps it, and, where rows are long
+  // enough to be split, about a quarter more for their parts
+  size_t need = (size_t)A.share_entries * ((fp64 ? 8 : 4) + (A.dcol ? 2 : 4));
+  if (A.padded > 16 * A.n) need += need / 4;
+  need = std::max(fixed, need + fixed_bytes(A.share_slices, A.n_slices, fp64 ? 8 : 4, false));
+  const size_t bytes = (size_t)A.padded * ((fp64 ? 8 : 4) + (A.dcol ? 2 : 4));
+  if (need > (size_t)kPoolMax &&
+      bytes > (A.n_slices > (int64_t)32 * A.grid ? kGridL2Bytes : kGridL2BytesFew))
+    return 0;
   return std::min<size_t>((need + 1023) & ~(size_t)1023, kPoolMax);
+}
+
+int pcg_group_shape(const DeviceSell &A, int precision, int grid, int *max_slices) {
+  if (precision == FFG_PRECISION_MIXED16 || A.n < 1 || grid > 32 * kPoll ||
+      (int64_t)A.host_soff.size() != A.n_slices + 1 || !resident_ready())
+    return 0;
+  const bool fp64 = precision == FFG_PRECISION_FP64;
+  const size_t entry = (fp64 ? 8 : 4) + (A.dcol ? 2 : 4);
+  const int64_t *soff = A.host_soff.data();
+  // a k-th of the grid each, so that groups fill it: the largest k (of at most
+  // kMaxResidentGroups) whose CTAs hold the operator but for a twelfth
+  for (int k = std::min(kMaxResidentGroups, grid / 2); k >= 1; --k) {
+    const int G = grid / k;
+    int64_t entries = 0;
+    int slices = 0;
+    for (int r = 0, s0 = 0; r < G; ++r) {
+      const int s1 = group_cut(soff, A.n_slices, r + 1, G);
+      slices = std::max(slices, s1 - s0);
+      entries = std::max(entries, soff[s1] - soff[s0]);
+      s0 = s1;
+    }
+    const size_t fixed = loops_bytes(slices, A.n_slices, fp64, false);
+    if (fixed <= (size_t)kPoolMax &&
+        fixed + (size_t)entries * entry <= (size_t)kPoolMax + kPoolMax / 12) {
+      *max_slices = slices;
+      return G;
+    }
+  }
+  return 0;
+}
+
+cudaError_t pcg_launch_resident_groups(int count, const PcgParams *sys, cudaStream_t s) {
+  static_assert(sizeof(GroupBatch) <= 32000, "kernel parameter block too large");
+  GroupBatch B;
+  B.count = count;
+  B.first[0] = 0;
+  for (int i = 0; i < count; ++i) {
+    PcgParams &P = B.sys[i];
+    P = sys[i];
+    const size_t fixed =
+        loops_bytes(P.share_slices, P.n_slices, P.precision == FFG_PRECISION_FP64, false);
+    P.part_bytes = (int)std::min<size_t>(kPoolMax / 8, kPoolMax - fixed);
+    B.first[i + 1] = B.first[i] + P.ncta;
+  }
+  void *args[] = {&B};
+  return cudaLaunchCooperativeKernel((const void *)pcg_resident_group_kernel,
+                                     dim3(B.first[count]), dim3(kGridThreads), args, kPoolMax, s);
 }
 
 cudaError_t pcg_launch_cluster(int count, const PcgParams *sys, int cluster, bool batched,

@@ -94,6 +94,14 @@ size_t pcg_resident_message_bytes(int ctas);
 // kernel enqueued just before, on which it does not depend.
 cudaError_t pcg_launch_cluster(int count, const PcgParams *sys, int cluster, bool batched,
                                bool overlap, cudaStream_t s);
+// CTAs of the group that holds the operator in shared memory within a launch of
+// several systems, or 0 when no group of up to `grid` does; max_slices: the most
+// slices of one of them.
+int pcg_group_shape(const DeviceSell &A, int precision, int grid, int *max_slices);
+// Systems on consecutive groups of sys[i].ncta CTAs (share_slices set), at most
+// kMaxResidentGroups of them, in one cooperative launch.
+constexpr int kMaxResidentGroups = 16;
+cudaError_t pcg_launch_resident_groups(int count, const PcgParams *sys, cudaStream_t s);
 // P.ncta CTAs, cooperative.
 cudaError_t pcg_launch_resident(const PcgParams &P, size_t pool_bytes, cudaStream_t s);
 

@@ -123,7 +123,7 @@ class Scheduler:
     # another on the whole device
     groups: bool = False
     grid: int = 148
-    group_rows: int = 16384
+    group_rows: int = 2048
     max_groups: int = 16
     queue: deque = field(default_factory=deque)
     inflight: List[Batch] = field(default_factory=list)

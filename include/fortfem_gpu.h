@@ -465,15 +465,16 @@ void ffg_problem_phase_times(int handle, double *seconds, int *status);
  * `count` values, the other per-problem arrays hold `count` pointers (the
  * arrays cell_a, cell_b, source_samples, constrained_values may be null, as
  * may their entries).  mode FFG_BATCH_CTA_PER_SYSTEM solves every system on
- * one thread block of its own in a single launch (for many small systems;
- * a system's result does not depend on the rest of the batch);
+ * a thread-block cluster of its own (8 or 16 blocks by its size; one block
+ * where its vectors do not fit a cluster's shared memory), for many small
+ * systems; a system's result does not depend on the rest of the batch;
  * FFG_BATCH_WHOLE_DEVICE solves them one after another on the whole GPU (for
  * large systems); FFG_BATCH_CTA_GROUPS solves them side by side in shared
- * cooperative launches, each system on a group of thread blocks sized by its
- * row count alone (16384 rows per block, at least 2, at most one per SM), so
- * that mid-size systems, whose iterations are bound by the grid barrier
- * rather than by bandwidth, share the GPU while a system's result still does
- * not depend on the rest of the batch.  A problem may belong to one
+ * cooperative launches, each system on the fraction of the SMs (at least a
+ * 16th) whose shared memory holds its operator, so that mid-size systems,
+ * whose iterations are bound by synchronisation rather than by bandwidth,
+ * share the GPU while a system's result still does not depend on the rest of
+ * the batch (a system too large for that takes the whole GPU).  A problem may belong to one
  * unfinished batch at a time. */
 #define FFG_BATCH_CTA_PER_SYSTEM 0
 #define FFG_BATCH_WHOLE_DEVICE 1
