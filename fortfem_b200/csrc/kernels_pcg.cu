@@ -51,7 +51,7 @@ namespace {
 
 constexpr int kThreads = 1024;
 constexpr int kWarps = kThreads / 32;
-constexpr int kSlots = 4;
+constexpr int kSlots = kVals;
 constexpr int kPartialBatch = 8;   // partial loads in flight per lane
 // Staged SpMV: every warp streams its slices through kStages shared-memory
 // buffers of kStageBytes (32 rows by as many columns as fit: values, then
@@ -158,6 +158,30 @@ __device__ void read_partials(const PcgParams &P, unsigned int phase, double *ou
   __syncthreads();
   for (int s = 0; s < nslot; ++s) out[s] = res[s];
   __syncthreads();
+}
+
+// The sums of the threads' v[0..NV) over the system's CTAs, the same bits in
+// every thread, with release / acquire of all earlier writes (NV = 0: the
+// barrier alone).  False: give up.
+template <int NV>
+__device__ __forceinline__ bool sync_sums(const PcgParams &P, unsigned int &phase,
+                                          const double (&v)[kVals], double (&out)[kVals]) {
+  if (NV > 0) write_partials(P, phase, v, NV);
+  if (!grid_barrier(P, phase)) return false;
+  if (NV > 0) read_partials(P, phase, out, NV);
+  return true;
+}
+
+// Whether the wall limit has passed, judged by the first CTA every kLimitEvery
+// iterations; `ok` is false when the sync gave up.
+__device__ __forceinline__ bool past_limit(const PcgParams &P, unsigned int &phase, int iteration,
+                                           unsigned long long t_start, bool &ok) {
+  ok = true;
+  if (iteration % kLimitEvery != 0) return false;
+  double v[kVals] = {0.0, 0.0}, out[kVals];
+  if (cta_of(P) == 0 && threadIdx.x == 0 && globaltimer() - t_start > P.limit_ns) v[0] = 1.0;
+  ok = sync_sums<1>(P, phase, v, out);
+  return ok && out[0] != 0.0;
 }
 
 // Slices [s0, s1) of the calling CTA.
@@ -497,7 +521,7 @@ __device__ __forceinline__ void for_rows_even_batched(const PcgParams &P, L load
 }
 
 __device__ __forceinline__ unsigned long long stamp(const PcgParams &P) {
-  return (cta_of(P) == 0 && threadIdx.x == 0) ? globaltimer() : 0ull;
+  return (cta_of(P) == 0 && threadIdx.x == 0) ? clock_now() : 0ull;
 }
 
 // Gather policies of the SpMV: accumulate(acc, a, c) adds the stored entry a
@@ -612,18 +636,15 @@ __device__ __forceinline__ double residual(const PcgParams &P, const float *p = 
 }
 
 // r64 = b - A x and the partial sums of (r64, r64) and (b, b), reduced.
-__device__ bool residual_norms(const PcgParams &P, unsigned int &phase, double *red) {
-  double part[kSlots];
+__device__ bool residual_norms(const PcgParams &P, unsigned int &phase, double (&red)[kVals]) {
+  double part[kVals];
   part[0] = residual(P);
   part[1] = 0.0;
   for_rows(P, [&](int row) {
     const double bb = P.b[row];
     part[1] += bb * bb;
   });
-  write_partials(P, phase, part, 2);
-  if (!grid_barrier(P, phase)) return false;
-  read_partials(P, phase, red, 2);
-  return true;
+  return sync_sums<2>(P, phase, part, red);
 }
 
 // FP64 Jacobi-PCG, the reference's recurrences.  `continuation` runs it after
@@ -637,7 +658,7 @@ __device__ __noinline__ void cg64(const PcgParams &P, unsigned int &phase,
   double *r = P.rd;
   double *q = P.qd;
   double2 *zp[2] = {P.zpd0, P.zpd1};
-  double part[kSlots], red[kSlots];
+  double part[kVals] = {0.0, 0.0}, red[kVals];
   unsigned long long t0, t1, t2;
 
   t0 = stamp(P);
@@ -662,13 +683,13 @@ __device__ __noinline__ void cg64(const PcgParams &P, unsigned int &phase,
       zp[0][row] = double2{z, 0.0};
       part[0] += rr * z;
     });
-    write_partials(P, phase, part, 1);
-    if (!grid_barrier(P, phase)) { o.aborted = 1; return; }
-    read_partials(P, phase, red, 1);
+    if (!sync_sums<1>(P, phase, part, red)) { o.aborted = 1; return; }
     rz = red[0];
   }
   tm.u += stamp(P) - t0;
-  double beta = 0.0;
+  // the residual estimate, squared, against the target, squared
+  double beta = 0.0, est2 = rnorm * rnorm;
+  const double target2 = target * target;
   int cur = 0;
   const int budget = P.max_it - o.iterations;
   for (int it = 1; !converged && it <= budget; ++it) {
@@ -677,10 +698,8 @@ __device__ __noinline__ void cg64(const PcgParams &P, unsigned int &phase,
     // A: p = z + beta p_old, q = A p, (p, q)
     t0 = stamp(P);
     part[0] = spmv(P, A, PairGather<double, double2>{zc, zn, q, beta});
-    write_partials(P, phase, part, 1);
     t1 = stamp(P);
-    if (!grid_barrier(P, phase)) { o.aborted = 1; return; }
-    read_partials(P, phase, red, 1);
+    if (!sync_sums<1>(P, phase, part, red)) { o.aborted = 1; return; }
     t2 = stamp(P);
     tm.a += t1 - t0;
     tm.aw += t2 - t1;
@@ -692,7 +711,6 @@ __device__ __noinline__ void cg64(const PcgParams &P, unsigned int &phase,
     // B: x += alpha p, r -= alpha q, z = D^-1 r
     t0 = stamp(P);
     part[0] = part[1] = 0.0;
-    part[2] = (cta_of(P) == 0 && threadIdx.x == 0 && globaltimer() - t_start > P.limit_ns) ? 1.0 : 0.0;
     {
       double2 a[kRowBatch] = {};
       double xv[kRowBatch] = {}, rv[kRowBatch] = {}, qv[kRowBatch] = {}, dv[kRowBatch] = {};
@@ -715,23 +733,23 @@ __device__ __noinline__ void cg64(const PcgParams &P, unsigned int &phase,
             part[1] += rr * z;
           });
     }
-    write_partials(P, phase, part, 3);
     t1 = stamp(P);
-    if (!grid_barrier(P, phase)) { o.aborted = 1; return; }
-    read_partials(P, phase, red, 3);
+    if (!sync_sums<2>(P, phase, part, red)) { o.aborted = 1; return; }
     t2 = stamp(P);
     tm.b += t1 - t0;
     tm.bw += t2 - t1;
     ++o.iterations;
     double rz_new = red[1];
-    const double est = sqrt(red[0]);
-    true_res = est;
-    if (red[2] != 0.0) { o.status = FFG_TIMEOUT; break; }
-    if (est <= target && !continuation) { converged = 1; break; }
+    est2 = red[0];
+    const bool reached = est2 <= target2;
+    bool ok;
+    if (past_limit(P, phase, o.iterations, t_start, ok)) { o.status = FFG_TIMEOUT; break; }
+    if (!ok) { o.aborted = 1; return; }
+    if (reached && !continuation) { converged = 1; break; }
     ++cycle_its;
     bool restart = false;
     if (continuation &&
-        (est <= target || (first_cycle > 0 && cycle_its >= 2 * first_cycle))) {
+        (reached || (first_cycle > 0 && cycle_its >= 2 * first_cycle))) {
       // the continuation's target is the true residual: check b - A x and,
       // while it still falls, start a new CG cycle from it (the recursive
       // residual of a long FP64 run drifts from the true one, and a cycle
@@ -741,10 +759,9 @@ __device__ __noinline__ void cg64(const PcgParams &P, unsigned int &phase,
       cycle_its = 0;
       restart = true;
       part[0] = residual(P);
-      write_partials(P, phase, part, 1);
-      if (!grid_barrier(P, phase)) { o.aborted = 1; return; }
-      read_partials(P, phase, red, 1);
+      if (!sync_sums<1>(P, phase, part, red)) { o.aborted = 1; return; }
       true_res = sqrt(red[0]);
+      est2 = red[0];
       if (true_res <= target) { converged = 1; tm.u += stamp(P) - t0; break; }
       stall = (true_res > 0.5 * last_true) ? stall + 1 : 0;
       last_true = true_res;
@@ -760,9 +777,7 @@ __device__ __noinline__ void cg64(const PcgParams &P, unsigned int &phase,
         zn[row] = a;
         part[0] += rr2 * z;
       });
-      write_partials(P, phase, part, 1);
-      if (!grid_barrier(P, phase)) { o.aborted = 1; return; }
-      read_partials(P, phase, red, 1);
+      if (!sync_sums<1>(P, phase, part, red)) { o.aborted = 1; return; }
       tm.u += stamp(P) - t0;
       rz_new = red[0];
     }
@@ -771,13 +786,11 @@ __device__ __noinline__ void cg64(const PcgParams &P, unsigned int &phase,
     cur ^= 1;
   }
   o.converged = converged;
-  o.final_res = true_res;
+  o.final_res = sqrt(est2);
   // true FP64 residual of the returned x
   t0 = stamp(P);
   part[0] = residual(P);
-  write_partials(P, phase, part, 1);
-  if (!grid_barrier(P, phase)) { o.aborted = 1; return; }
-  read_partials(P, phase, red, 1);
+  if (!sync_sums<1>(P, phase, part, red)) { o.aborted = 1; return; }
   tm.u += stamp(P) - t0;
   o.true_res = sqrt(red[0]);
 }
@@ -789,7 +802,8 @@ __device__ bool fold_x(const PcgParams &P, unsigned int &phase) {
     P.x[row] += (double)P.xf[row];
     P.xf[row] = 0.f;
   });
-  return grid_barrier(P, phase);
+  double none[kVals], out[kVals];
+  return sync_sums<0>(P, phase, none, out);
 }
 
 // Mixed mode: the PCG recurrences in FP32 on a scaled residual, the solution
@@ -811,7 +825,7 @@ __device__ __noinline__ void cg_mixed(const PcgParams &P, unsigned int &phase,
   const float *dinv = P.d32;
   float *r = P.rf, *z = P.zf, *p = P.pf, *q = P.qf;
   float2 *zp[2] = {P.zpf0, P.zpf1};
-  double part[kSlots], red[kSlots];
+  double part[kVals] = {0.0, 0.0}, red[kVals];
   unsigned long long t0, t1, t2;
 
   t0 = stamp(P);
@@ -840,12 +854,15 @@ __device__ __noinline__ void cg_mixed(const PcgParams &P, unsigned int &phase,
       P.xf[row] = 0.f;
       part[0] += (double)rr * (double)zz;
     });
-    write_partials(P, phase, part, 1);
-    if (!grid_barrier(P, phase)) { o.aborted = 1; return; }
-    read_partials(P, phase, red, 1);
+    if (!sync_sums<1>(P, phase, part, red)) { o.aborted = 1; return; }
     rz = red[0];
   }
   tm.u += stamp(P) - t0;
+  auto stop = [&]() {
+    const double t = target / scale;
+    return fmax(t * t, P.delta * P.delta);
+  };
+  double stop_rr = stop();
   double beta = 0.0;
   bool unfolded = false;  // xf holds a step not yet added to x
   const int budget = P.max_it - o.iterations;
@@ -861,10 +878,8 @@ __device__ __noinline__ void cg_mixed(const PcgParams &P, unsigned int &phase,
     else
       part[0] = direct ? spmv(P, P.v32, PairGather<float, float2>{zp[cur], zn, q, bt})
                        : spmv(P, P.v32, ZGather{z, p, q, bt});
-    write_partials(P, phase, part, 1);
     t1 = stamp(P);
-    if (!grid_barrier(P, phase)) { o.aborted = 1; return; }
-    read_partials(P, phase, red, 1);
+    if (!sync_sums<1>(P, phase, part, red)) { o.aborted = 1; return; }
     t2 = stamp(P);
     tm.a += t1 - t0;
     tm.aw += t2 - t1;
@@ -885,7 +900,6 @@ __device__ __noinline__ void cg_mixed(const PcgParams &P, unsigned int &phase,
     // B: dx += alpha p, r -= alpha q, z = D^-1 r
     t0 = stamp(P);
     part[0] = part[1] = 0.0;
-    part[2] = (cta_of(P) == 0 && threadIdx.x == 0 && globaltimer() - t_start > P.limit_ns) ? 1.0 : 0.0;
     {
       float xv[kRowBatch] = {}, pv[kRowBatch] = {}, rv[kRowBatch] = {}, qv[kRowBatch] = {},
             dv[kRowBatch] = {};
@@ -910,10 +924,8 @@ __device__ __noinline__ void cg_mixed(const PcgParams &P, unsigned int &phase,
       else
         for_rows_even_batched(P, [&](int row, int u) { load(row, u); pv[u] = p[row]; }, step);
     }
-    write_partials(P, phase, part, 3);
     t1 = stamp(P);
-    if (!grid_barrier(P, phase)) { o.aborted = 1; return; }
-    read_partials(P, phase, red, 3);
+    if (!sync_sums<2>(P, phase, part, red)) { o.aborted = 1; return; }
     t2 = stamp(P);
     tm.b += t1 - t0;
     tm.bw += t2 - t1;
@@ -921,16 +933,22 @@ __device__ __noinline__ void cg_mixed(const PcgParams &P, unsigned int &phase,
     unfolded = true;
     if (direct) cur ^= 1;
     const double rr = red[0], rz_new = red[1];
-    const double est = sqrt(rr) * scale;
-    if (red[2] != 0.0) { o.status = FFG_TIMEOUT; true_res = est; break; }
+    bool ok;
+    if (past_limit(P, phase, o.iterations, t_start, ok)) {
+      o.status = FFG_TIMEOUT;
+      true_res = sqrt(rr) * scale;
+      break;
+    }
+    if (!ok) { o.aborted = 1; return; }
     // reliable update: replace the recursive residual with b - A x in FP64
     // when it has fallen by delta, claims convergence, has grown tenfold
     // past the last true residual (the FP32 recurrence is diverging; the
     // search then restarts), or has not triggered within `window`
     // iterations (an FP32 plateau, judged by the stall test below)
-    const bool grew = !(est < 10.0 * scale);
+    // (the estimate sqrt(rr) * scale against the three, squared)
+    const bool grew = !(rr < 100.0);
     const bool slow = o.iterations - since > window;
-    if (!(est <= target || rr <= P.delta * P.delta || grew || slow)) {
+    if (!(rr <= stop_rr || grew || slow)) {
       beta = rz_new / rz;
       rz = rz_new;
       continue;
@@ -943,9 +961,7 @@ __device__ __noinline__ void cg_mixed(const PcgParams &P, unsigned int &phase,
     // q = A p comes with the residual (used if the update goes on in the
     // recurrence form)
     part[0] = direct ? residual(P) : residual(P, p, q);
-    write_partials(P, phase, part, 1);
-    if (!grid_barrier(P, phase)) { o.aborted = 1; return; }
-    read_partials(P, phase, red, 1);
+    if (!sync_sums<1>(P, phase, part, red)) { o.aborted = 1; return; }
     true_res = sqrt(red[0]);
     if (true_res <= target) { converged = 1; tm.u += stamp(P) - t0; break; }
     if (!(true_res > 0.0) || !is_finite_d(true_res)) break;
@@ -988,14 +1004,13 @@ __device__ __noinline__ void cg_mixed(const PcgParams &P, unsigned int &phase,
         part[0] += (double)rr2 * (double)zz;
       });
     }
-    write_partials(P, phase, part, 1);
-    if (!grid_barrier(P, phase)) { o.aborted = 1; return; }
-    read_partials(P, phase, red, 1);
+    if (!sync_sums<1>(P, phase, part, red)) { o.aborted = 1; return; }
     tm.u += stamp(P) - t0;
     // p_new = z + beta' (ratio p): beta' against the old (r, z) in new units
     beta = grew ? 0.0 : red[0] / (rz * ratio);
     rz = red[0];
     scale = true_res;
+    stop_rr = stop();
     window = max(kMinWindow, 4 * (o.iterations - since));
     since = o.iterations;
   }
@@ -1010,9 +1025,7 @@ __device__ __noinline__ void cg_mixed(const PcgParams &P, unsigned int &phase,
   // true FP64 residual of the returned x
   t0 = stamp(P);
   part[0] = residual(P);
-  write_partials(P, phase, part, 1);
-  if (!grid_barrier(P, phase)) { o.aborted = 1; return; }
-  read_partials(P, phase, red, 1);
+  if (!sync_sums<1>(P, phase, part, red)) { o.aborted = 1; return; }
   tm.u += stamp(P) - t0;
   o.true_res = sqrt(red[0]);
   o.final_res = o.true_res;
@@ -1027,8 +1040,7 @@ __device__ __forceinline__ void pcg_body(const PcgParams &P) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  // only block 0 judges the wall limit; its verdict travels through a partial slot
-  const unsigned long long t_start = globaltimer();
+  const unsigned long long t_start = globaltimer(), c_start = clock_now();
   Outcome o;
   Timing tm;
   int continued = 0;
@@ -1040,13 +1052,16 @@ __device__ __forceinline__ void pcg_body(const PcgParams &P) {
       continued = o.restart ? 2 : 1;
       if (o.restart) {
         for_rows_even(P, [&](int row) { P.x[row] = 0.0; });
-        if (!grid_barrier(P, phase)) return;
+        double none[kVals], out[kVals];
+        if (!sync_sums<0>(P, phase, none, out)) return;
       }
       cg64(P, phase, t_start, true, o, tm);
     }
   }
   if (o.aborted) return;
   if (cta_of(P) == 0 && threadIdx.x == 0) {
+    const double c = (double)(clock_now() - c_start);
+    const double sec = c > 0.0 ? 1e-9 * (double)(globaltimer() - t_start) / c : 0.0;
     P.result[0] = o.converged;
     P.result[1] = o.iterations;
     P.result[2] = o.updates;
@@ -1055,11 +1070,11 @@ __device__ __forceinline__ void pcg_body(const PcgParams &P) {
     P.result[5] = o.status;
     P.result[6] = o.bnorm;
     P.result[7] = continued;
-    P.result[8] = 1e-9 * (double)tm.a;
-    P.result[9] = 1e-9 * (double)tm.aw;
-    P.result[10] = 1e-9 * (double)tm.b;
-    P.result[11] = 1e-9 * (double)tm.bw;
-    P.result[12] = 1e-9 * (double)tm.u;
+    P.result[8] = sec * (double)tm.a;
+    P.result[9] = sec * (double)tm.aw;
+    P.result[10] = sec * (double)tm.b;
+    P.result[11] = sec * (double)tm.bw;
+    P.result[12] = sec * (double)tm.u;
   }
 }
 
@@ -1363,7 +1378,7 @@ void free_sell(DeviceSell &d) {
 // Partial sums of pcg_kernel ([2][kSlots][grid] doubles) or messages of the
 // resident kernel.
 static size_t partial_bytes(int grid) {
-  return std::max(2 * kSlots * (size_t)grid * sizeof(double), pcg_resident_message_bytes(grid));
+  return std::max(2 * kSlots * (size_t)grid * sizeof(double), pcg_message_bytes(grid));
 }
 
 int solve_work_alloc(SolveWork &w, int64_t n, int grid) {
@@ -1397,7 +1412,7 @@ int solve_work_alloc(SolveWork &w, int64_t n, int grid) {
   if (!bad) {
     std::memset(w.result_host, 0, kResultDoubles * sizeof(double));
     w.control_host[0] = w.control_host[1] = 0;
-    if (cudaMemset(w.control, 0, 64) != cudaSuccess || cudaMemset(w.barrier, 0, 64) != cudaSuccess)
+    if (cudaMemset(w.control, 0, 64) != cudaSuccess)
       bad = true;
   }
   if (bad) {
@@ -1410,8 +1425,7 @@ int solve_work_alloc(SolveWork &w, int64_t n, int grid) {
 
 void solve_work_free(SolveWork &w) {
   void *ptrs[] = {w.r64, w.rd, w.qd, w.zpd0, w.zpd1, w.rf, w.zf, w.pf, w.qf, w.xf, w.zpf0, w.zpf1,
-                  w.partial,
-                  w.barrier, w.control, w.result};
+                  w.partial, w.barrier, w.control, w.result};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (w.result_host) cudaFreeHost(w.result_host);
@@ -1484,7 +1498,7 @@ int pcg_launch(const DeviceSell &A, const double *b, double *x, const ffg_solver
   if (cluster) {
     e = pcg_launch_cluster(1, &P, cluster, false, false, stream);
   } else if (const size_t pool = pcg_grid_resident(A, opts.precision)) {
-    if (cudaMemsetAsync(w.partial, 0, pcg_resident_message_bytes(w.grid), stream) != cudaSuccess)
+    if (cudaMemsetAsync(w.partial, 0, pcg_message_bytes(w.grid), stream) != cudaSuccess)
       return FFG_CUDA_ERROR;
     e = pcg_launch_resident(P, pool, stream);
   } else {
@@ -1597,7 +1611,7 @@ int pcg_launch_groups(int count, const DeviceSell *const *A, const double *const
     } else if (cudaMemsetAsync(w[i]->control, 0, 64, stream) != cudaSuccess ||
                cudaMemsetAsync(w[i]->result, 0, kResultDoubles * sizeof(double), stream) !=
                    cudaSuccess ||
-               cudaMemsetAsync(w[i]->partial, 0, pcg_resident_message_bytes(ctas[i]), stream) !=
+               cudaMemsetAsync(w[i]->partial, 0, pcg_message_bytes(ctas[i]), stream) !=
                    cudaSuccess) {
       return FFG_CUDA_ERROR;
     }

@@ -41,16 +41,15 @@ namespace {
 
 constexpr int kGridThreads = 512;
 constexpr int kMaxCluster = 16;
-constexpr int kVals = 2;           // values of one reduction, at most
-constexpr int kPoll = 5;            // messages a lane polls: up to 160 CTAs
 constexpr int kBatch = 8;          // columns of a row in flight
+constexpr int kPoolMax = 225 * 1024;
+
 // Before the grid's first poll of a sync: the polls of 148 CTAs hit the same few
 // L2 lines and slow the messages and the fences they wait for (P1, 85,800
 // rows: 9.4 us an iteration without naps, 7.8 with these; between polls a nap
 // gained nothing).
 constexpr unsigned kNapSums = 200, kNapData = 700;  // ns
-constexpr int kLimitEvery = 64;    // iterations between looks at the wall limit
-constexpr int kPoolMax = 225 * 1024;
+
 
 // A slice of this CTA: where it starts in the operator, in the CTA's
 // shared-memory copy (-1: not copied), and its length in columns.
@@ -62,9 +61,8 @@ struct SliceEnt {
 };
 
 struct ResShared {
-  double red[kVals][16];
+  double red[kVals][16], res[kVals];
   double slot[2][kVals][kMaxCluster];
-  double res[kVals];
   unsigned long long mbar[2];
   int ok, items, rows;
   int need;               // slices that arrive in an exchange
@@ -77,12 +75,6 @@ __device__ __forceinline__ double warp_sum(double x) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
   return x;
-}
-
-__device__ __forceinline__ unsigned long long clock_now() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %clock64;" : "=l"(t));
-  return t;
 }
 
 __device__ __forceinline__ unsigned mapa(unsigned addr, int rank) {
@@ -219,8 +211,8 @@ struct ClusterSync {
 // validates itself.  The polled sectors are what a sync costs beyond latency:
 // with the two values of a CTA side by side, 32 bytes read by two loads, a sync
 // with two sums took 4.7 us where this layout takes 3.4.
-// kGroup: instantiated once per kernel (a function that two kernels share finds
-// the shared memory through an indirection: 15 % of an iteration).
+// Every CTA calls the same syncs in the same order; msg is zero before the launch.
+// kGroup: instantiated once per kernel.
 template <int NT, bool kGroup>
 struct GridSync {
   int rank, n;
@@ -244,7 +236,7 @@ struct GridSync {
     if (NV > 0) x = block_sums<NV, NT>(v);
     else __syncthreads();
     if (warp == 0) {
-      unsigned long long *msg =
+      unsigned long long *slots =
           reinterpret_cast<unsigned long long *>(gP.partial) + (size_t)(phase & 1u) * 4 * n;
       const double x1 = __shfl_sync(0xffffffffu, x, 16);
       if (lane == 0) {
@@ -259,7 +251,7 @@ struct GridSync {
         }
 #pragma unroll
         for (int s = 0; s < NM; ++s)
-          asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(msg + 2 * (s * n + rank)),
+          asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(slots + 2 * (s * n + rank)),
                        "l"(e[2 * s]), "l"(e[2 * s + 1])
                        : "memory");
       }
@@ -277,7 +269,7 @@ struct GridSync {
             for (int s = 0; s < NM; ++s)
               asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];"
                            : "=l"(e[k][2 * s]), "=l"(e[k][2 * s + 1])
-                           : "l"(msg + 2 * (s * n + lane + 32 * k))
+                           : "l"(slots + 2 * (s * n + lane + 32 * k))
                            : "memory");
         }
 #pragma unroll
@@ -1289,7 +1281,7 @@ size_t loops_bytes(int64_t slices, int64_t n_slices, bool fp64, bool replica) {
 }
 }  // namespace
 
-size_t pcg_resident_message_bytes(int ctas) { return 2 * (size_t)ctas * 32; }
+size_t pcg_message_bytes(int ctas) { return 2 * (size_t)ctas * 32; }
 
 // Lines between the kernels, measured on a B200 (solve time of P1, P2 and
 // order-1 Nedelec systems, clusters of 16 against the whole grid):

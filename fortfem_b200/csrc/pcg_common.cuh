@@ -34,7 +34,7 @@ struct PcgParams {
   float2 *zpf0, *zpf1;       // mixed mode after a switch to direct A p: (z, p) pairs
   double *rd, *qd;
   double2 *zpd0, *zpd1;
-  double *partial;  // [2][kSlots][grid]
+  double *partial;  // partial sums [2][2][grid], or messages (pcg_message_bytes)
   unsigned int *bar;
   int *control;     // [0] error status
   double *result;   // kResultDoubles
@@ -58,6 +58,12 @@ __device__ __forceinline__ unsigned long long globaltimer() {
   return t;
 }
 
+__device__ __forceinline__ unsigned long long clock_now() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %clock64;" : "=l"(t));
+  return t;
+}
+
 __device__ __forceinline__ int ld_volatile_int(const int *p) {
   return *reinterpret_cast<const volatile int *>(p);
 }
@@ -67,6 +73,10 @@ __device__ __forceinline__ unsigned smem_addr(const void *p) {
 }
 
 __device__ __forceinline__ bool is_finite_d(double x) { return isfinite(x); }
+
+constexpr int kVals = 2;  // values of one reduction, at most
+constexpr int kPoll = 5;            // messages a lane polls: up to 160 CTAs
+constexpr int kLimitEvery = 64;    // iterations between looks at the wall limit
 
 struct Outcome {
   int iterations = 0, updates = 0, converged = 0, status = FFG_OK, stagnated = 0, aborted = 0;
@@ -88,8 +98,8 @@ int pcg_cluster_size(const DeviceSell &A, int precision, bool batched);
 // Shared memory per CTA with which the cooperative grid holds the operator on
 // chip, or 0 when it does not.
 size_t pcg_grid_resident(const DeviceSell &A, int precision);
-// Bytes at PcgParams::partial (zero before a launch) for the grid's messages.
-size_t pcg_resident_message_bytes(int ctas);
+// Bytes at PcgParams::partial (zero before a launch) for the messages of `ctas` CTAs.
+size_t pcg_message_bytes(int ctas);
 // One cluster of `cluster` CTAs per system; overlap: beside the launch of this
 // kernel enqueued just before, on which it does not depend.
 cudaError_t pcg_launch_cluster(int count, const PcgParams *sys, int cluster, bool batched,
