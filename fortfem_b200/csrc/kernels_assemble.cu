@@ -352,26 +352,28 @@ __global__ void csc_column_warp_kernel(int64_t n_free, int max_len,
   if (lane == 0) rhs[j] = b - lift;
 }
 
-// SELL rows of Nedelec elements (16 <= n_b <= 128), one 256-thread CTA per
-// half slice (16 rows, so that four CTAs share an SM and one's write-out
-// overlaps the others' gathers): warp w gathers rows w and w + 8 of the half
-// (free column j = perm[row]) with its lanes over the element's local rows
-// i, as csc_column_warp_kernel does for a CSC column, into the half's image
-// in shared memory (slot s of row r at s * 17 + r), every entry receiving
-// its terms in ascending incidence order as in column_kernel; then the CTA
-// writes the half's FP64 and FP32 values (128 contiguous bytes of FP64 per
-// slot step) and each row's Jacobi diagonal and right-hand side.  Both rows'
-// columns, incidence ranges and first 32 incidences are loaded before either
-// is gathered; U incidences' element columns and slot rows (NI values per
-// lane each) are loaded before any of them is added.
+// SELL rows of Nedelec elements (n_b >= 16), one part of a slice (R rows) at a
+// time in 256-thread CTAs that stay on their SM: LR lanes gather one row (free
+// column j = perm[row]) over the element's local rows i, as
+// csc_column_warp_kernel does for a CSC column, into the part's image in shared
+// memory (slot s of row r at s * (R + 1) + r), every entry receiving its terms
+// in ascending incidence order as in column_kernel; then the CTA writes the
+// part's FP64 and FP32 values (R * 8 contiguous bytes of FP64 per slot step)
+// and clears the image behind it.  Bound: it moves the element matrices, the
+// slots and the rows once (3.2 GB at order 3 on a 24^3 box, 0.5 ms of copy
+// bandwidth), and came to issue slots and load latency first, so there is one
+// instruction stream for 32 / LR rows, no branch per entry, and what the next
+// part needs is loaded a part ahead.  Measured, a warp per row with a branch
+// per entry and CTAs of one part against this: order 3 on 24^3 1096 against
+// 693 us, order 4 (FP32 element matrices) on 17 x 16 x 17 940 against 693 us;
+// order 6 on 12^3, which went a thread per column, 5406 against 2212 us.
 struct SliceArgs {
   const int2 *range;  // per SELL row: [p0, p1) of its column's incidences
-  int nb, ld32;
+  int nb, ld32, max_width;
   int64_t cs32;  // FP32 element matrices: elements per cell
-  int64_t n;  // rows (free DoFs)
-  const int *perm;
-  const int64_t *soff, *col_ptr, *inc_ptr;
-  const int *row_idx, *inc_cell, *gd;
+  int64_t n, n_parts;  // rows (free DoFs), parts of all slices
+  const int64_t *soff;
+  const int *inc_cell, *gd;
   const uint8_t *inc_local;
   const uint16_t *slot;
   const double *elem, *cell_rhs, *g;
@@ -379,33 +381,26 @@ struct SliceArgs {
   double *val64, *dinv64, *rhs;
   float *val32, *dinv32;
 };
-constexpr int kSliceHalf = kSliceRows / 2;      // rows of a CTA
-constexpr int kSliceStride = kSliceHalf + 1;    // shared-memory row pitch of a half-slice image
 constexpr int kSliceThreads = 256;
-constexpr int kSliceRowsPerWarp = kSliceHalf / (kSliceThreads / 32);
-static_assert(kSliceRowsPerWarp == 2, "two rows per warp");
+constexpr int kSliceWarps = kSliceThreads / 32;
 
-// The incidences of one row: whether the row exists (j = 0, or -1 past the
-// last row), its incidence range [p0, p1) and the first 32 incidences' cells
-// and local indices, one per lane.
+// One row: its incidence range [p0, p1) (empty past the last row) and its
+// first LR incidences' cells and local indices, one per lane of its group.
 struct SliceRowHead {
-  int j;
-  int64_t p0, p1;
-  int e, l;
+  int p0, p1, e, l;
 };
 
-__device__ __forceinline__ void slice_head(const SliceArgs &A, int64_t row, int lane,
-                                           SliceRowHead &h) {
-  h.j = row < A.n ? 0 : -1;
-  const int2 rg = h.j >= 0 ? A.range[row] : make_int2(0, 0);
-  h.p0 = rg.x;
-  h.p1 = rg.y;
-  h.e = 0;
-  h.l = 0;
-  if (h.p0 + lane < h.p1) {
-    h.e = A.inc_cell[h.p0 + lane];
-    h.l = A.inc_local[h.p0 + lane];
+__device__ __forceinline__ int2 slice_range(const SliceArgs &A, int64_t row) {
+  return row < A.n ? A.range[row] : make_int2(0, 0);
+}
+
+__device__ __forceinline__ SliceRowHead slice_head(const SliceArgs &A, int2 rg, int i0) {
+  SliceRowHead h{rg.x, rg.y, 0, 0};
+  if (i0 < rg.y - rg.x) {
+    h.e = A.inc_cell[(int64_t)rg.x + i0];
+    h.l = A.inc_local[(int64_t)rg.x + i0];
   }
+  return h;
 }
 
 // Incidence range of every SELL row's column (the slice gather's heads).
@@ -417,70 +412,86 @@ __global__ void inc_range_kernel(int64_t n, const int *perm, const int64_t *inc_
   range[r] = make_int2((int)inc_ptr[j], (int)inc_ptr[j + 1]);
 }
 
-template <int NI, int U, bool F32>
+// Row r of the part by the calling group of LR lanes (32 / LR rows per warp
+// side by side); the lane's local rows are i0, i0 + LR, ..., of which only the
+// last can be past nb.  Loads of U incidences are issued before any is added.
+// Constrained local rows are added to a slot behind the image that nothing
+// reads, so that the adds have no branches.
+template <int NI, int U, bool F32, int LR>
 __device__ __forceinline__ void slice_row(const SliceArgs &A, double *img, int r, int64_t row,
-                                          int lane, SliceRowHead h) {
+                                          int i0, const SliceRowHead &h) {
+  constexpr int kPitch = kSliceWarps * (32 / LR) + 1;
+  constexpr unsigned kAll = 0xffffffffu;
   const int nb = A.nb;
+  const bool tail = i0 + LR * (NI - 1) < nb;
   double b = 0.0, lift = 0.0;
-  const int64_t p0 = h.p0, p1 = h.p1;
-  // local rows of this lane and whether they exist (nb <= 32 NI)
-  bool has[NI];
-#pragma unroll
-  for (int c = 0; c < NI; ++c) has[c] = lane + 32 * c < nb;
-  // element columns: FP64 nb x nb or FP32 with leading dimension ld32, per cell
-  const int ld = F32 ? A.ld32 : nb;
-  const size_t cell_stride = F32 ? (size_t)A.cs32 : (size_t)nb * nb;
-  for (int64_t pb = p0; pb < p1; pb += 32) {
-    const int cnt = (int)min((int64_t)32, p1 - pb);
-    int my_e = h.e, my_l = h.l;
-    if (pb != p0) {
-      my_e = lane < cnt ? A.inc_cell[pb + lane] : 0;
-      my_l = lane < cnt ? A.inc_local[pb + lane] : 0;
+  const int cnt = h.p1 - h.p0;
+  const int all = LR == 32 ? cnt : __reduce_max_sync(kAll, cnt);
+  int dslot = A.max_width;
+  for (int base = 0; base < all; base += LR) {
+    int e = h.e, l = h.l;
+    if (base > 0) {
+      const int64_t p = (int64_t)h.p0 + base + i0;
+      e = base + i0 < cnt ? A.inc_cell[p] : 0;
+      l = base + i0 < cnt ? A.inc_local[p] : 0;
     }
-    const double my_f = lane < cnt ? A.cell_rhs[(size_t)nb * my_e + my_l] : 0.0;
-    // per lane: the offset of its incidence's element column
-    const size_t my_col = (size_t)my_e * cell_stride + (size_t)ld * my_l;
-    for (int u0 = 0; u0 < cnt; u0 += U) {
+    // the lane's incidence: the offset of its element column and its load
+    const size_t my_col = F32 ? (size_t)e * (size_t)A.cs32 + (size_t)(A.ld32 * l)
+                              : ((size_t)e * nb + l) * (size_t)nb;
+    const double my_f = base + i0 < cnt ? A.cell_rhs[(size_t)nb * e + l] : 0.0;
+    const uint16_t *slp = A.slot + ((size_t)h.p0 + base) * nb + i0;
+    const int n = min(LR, all - base);
+    for (int u0 = 0; u0 < n; u0 += U) {
       double kil[U][NI];
-      uint16_t sl[U][NI];
-      int ev[U];
+      int sl[U][NI];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const bool live = u0 + u < cnt;
-        const int uu = live ? u0 + u : u0;
-        const size_t col = __shfl_sync(0xffffffffu, my_col, uu) + lane;
-        ev[u] = __shfl_sync(0xffffffffu, my_e, uu);
-        const uint16_t *slp = A.slot + (size_t)(pb + uu) * nb + lane;
+        const bool live = base + u0 + u < cnt;
+        const size_t col = __shfl_sync(kAll, my_col, (u0 + u) & (LR - 1), LR) + i0;
 #pragma unroll
         for (int c = 0; c < NI; ++c) {
-          const bool in = has[c] && live;
-          if (F32) kil[u][c] = in ? (double)A.elem32[col + 32 * c] : 0.0;
-          else kil[u][c] = in ? A.elem[col + 32 * c] : 0.0;
-          sl[u][c] = in ? slp[32 * c] : kConstrainedSlot;
+          const bool in = live && (c < NI - 1 || tail);
+          if (F32) kil[u][c] = in ? (double)__ldg(A.elem32 + col + LR * c) : 0.0;
+          else kil[u][c] = in ? __ldg(A.elem + col + LR * c) : 0.0;
+          sl[u][c] = in ? (int)__ldg(slp + LR * c) : (int)kConstrainedSlot;
+        }
+        slp += nb;
+      }
+      // the diagonal's slot: local row l of any incidence (e, l) of column j
+      // has global DoF j, so its slot entry is the diagonal
+      if (u0 == 0 && base == 0) {
+        const int l0 = __shfl_sync(kAll, l, 0, LR);
+#pragma unroll
+        for (int c = 0; c < NI; ++c)
+          if (i0 + LR * c == l0) dslot = sl[0][c];
+        dslot = min(__shfl_sync(kAll, dslot, l0 & (LR - 1), LR), A.max_width);
+      }
+      if (A.g) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int *ge = A.gd + (size_t)nb * __shfl_sync(kAll, e, (u0 + u) & (LR - 1), LR) + i0;
+#pragma unroll
+          for (int c = 0; c < NI; ++c)
+            if (sl[u][c] == kConstrainedSlot && base + u0 + u < cnt && (c < NI - 1 || tail))
+              lift += kil[u][c] * A.g[ge[LR * c]];
         }
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
 #pragma unroll
-        for (int c = 0; c < NI; ++c) {
-          if (sl[u][c] != kConstrainedSlot) {
-            img[sl[u][c] * kSliceStride + r] += kil[u][c];
-          } else if (A.g && has[c] && u0 + u < cnt) {
-            lift += kil[u][c] * A.g[A.gd[(size_t)nb * ev[u] + lane + 32 * c]];
-          }
-        }
+        for (int c = 0; c < NI; ++c)
+          img[min(sl[u][c], A.max_width) * kPitch + r] += kil[u][c];
+        b += __shfl_sync(kAll, my_f, (u0 + u) & (LR - 1), LR);
         __syncwarp();
       }
     }
-    for (int u = 0; u < cnt; ++u) b += __shfl_sync(0xffffffffu, my_f, u);
   }
+  if (A.g) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) lift += __shfl_xor_sync(0xffffffffu, lift, o);
-  if (lane == 0) {
-    // the diagonal's slot: local row l of any incidence (e, l) of column j
-    // has global DoF j, so its slot entry is the diagonal
-    const int dslot = p1 > p0 ? A.slot[(size_t)p0 * nb + h.l] : kConstrainedSlot;
-    const double d = dslot != kConstrainedSlot ? img[dslot * kSliceStride + r] : 0.0;
+    for (int o = LR / 2; o > 0; o >>= 1) lift += __shfl_xor_sync(kAll, lift, o);
+  }
+  if (i0 == 0 && row < A.n) {
+    const double d = dslot < A.max_width ? img[dslot * kPitch + r] : 0.0;
     const double di = (fabs(d) > 1.0e-14) ? 1.0 / d : 1.0;
     A.dinv64[row] = di;
     A.dinv32[row] = (float)di;
@@ -488,118 +499,41 @@ __device__ __forceinline__ void slice_row(const SliceArgs &A, double *img, int r
   }
 }
 
-// Two rows of a warp gathered in lockstep (both with at most 32 incidences):
-// batch u0 loads U incidences of each row before either is added, so both
-// rows' element columns are in flight together; each row still receives its
-// terms in ascending incidence order, into its own column of the image.
-template <int NI, int U, bool F32>
-__device__ __forceinline__ void slice_pair(const SliceArgs &A, double *img, const int (&r)[2],
-                                           const int64_t (&row)[2], int lane,
-                                           const SliceRowHead (&h)[2]) {
-  const int nb = A.nb;
-  const int ld = F32 ? A.ld32 : nb;
-  const size_t cell_stride = F32 ? (size_t)A.cs32 : (size_t)nb * nb;
-  bool has[NI];
-#pragma unroll
-  for (int c = 0; c < NI; ++c) has[c] = lane + 32 * c < nb;
-  int cnt[2];
-  size_t my_col[2];
-  double my_f[2], b[2] = {0.0, 0.0}, lift[2] = {0.0, 0.0};
-#pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    cnt[q] = h[q].j >= 0 ? (int)(h[q].p1 - h[q].p0) : 0;
-    my_col[q] = (size_t)h[q].e * cell_stride + (size_t)ld * h[q].l;
-    my_f[q] = lane < cnt[q] ? A.cell_rhs[(size_t)nb * h[q].e + h[q].l] : 0.0;
-  }
-  const int n_max = max(cnt[0], cnt[1]);
-  for (int u0 = 0; u0 < n_max; u0 += U) {
-    double kil[2][U][NI];
-    uint16_t sl[2][U][NI];
-    int ev[2][U];
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const bool live = u0 + u < cnt[q];
-        const int uu = live ? u0 + u : 0;
-        const size_t col = __shfl_sync(0xffffffffu, my_col[q], uu) + lane;
-        ev[q][u] = __shfl_sync(0xffffffffu, h[q].e, uu);
-        const uint16_t *slp = A.slot + (size_t)(h[q].p0 + uu) * nb + lane;
-#pragma unroll
-        for (int c = 0; c < NI; ++c) {
-          const bool in = has[c] && live;
-          if (F32) kil[q][u][c] = in ? (double)A.elem32[col + 32 * c] : 0.0;
-          else kil[q][u][c] = in ? A.elem[col + 32 * c] : 0.0;
-          sl[q][u][c] = in ? slp[32 * c] : kConstrainedSlot;
-        }
-      }
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-#pragma unroll
-        for (int c = 0; c < NI; ++c) {
-          if (sl[q][u][c] != kConstrainedSlot) {
-            img[sl[q][u][c] * kSliceStride + r[q]] += kil[q][u][c];
-          } else if (A.g && has[c] && u0 + u < cnt[q]) {
-            lift[q] += kil[q][u][c] * A.g[A.gd[(size_t)nb * ev[q][u] + lane + 32 * c]];
-          }
-        }
-      }
-    __syncwarp();
-  }
-#pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    if (h[q].j < 0) continue;
-    for (int u = 0; u < cnt[q]; ++u) b[q] += __shfl_sync(0xffffffffu, my_f[q], u);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) lift[q] += __shfl_xor_sync(0xffffffffu, lift[q], o);
-    if (lane == 0) {
-      // the diagonal's slot: local row l of any incidence (e, l) of column j
-      // has global DoF j, so its slot entry is the diagonal
-      const int dslot = cnt[q] > 0 ? A.slot[(size_t)h[q].p0 * nb + h[q].l] : kConstrainedSlot;
-      const double d = dslot != kConstrainedSlot ? img[dslot * kSliceStride + r[q]] : 0.0;
-      const double di = (fabs(d) > 1.0e-14) ? 1.0 / d : 1.0;
-      A.dinv64[row[q]] = di;
-      A.dinv32[row[q]] = (float)di;
-      A.rhs[row[q]] = b[q] - lift[q];
-    }
-  }
-}
-
-template <int NI, int U, bool F32>
-__global__ void __launch_bounds__(kSliceThreads, 4) sell_slice_kernel(const __grid_constant__ SliceArgs A) {
+// The next part's incidences and the ranges of the one after it are loaded
+// while a part is gathered, so that the chain range -> incidence -> element
+// column costs one memory latency per part.
+template <int NI, int U, bool F32, int LR, int CTAS>
+__global__ void __launch_bounds__(kSliceThreads, CTAS)
+sell_slice_kernel(const __grid_constant__ SliceArgs A) {
   extern __shared__ double img[];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr int kW = kSliceThreads / 32;
-  const int64_t hs = blockIdx.x;
-  const int64_t k = hs >> 1;
-  const int half = (int)(hs & 1);
-  const int64_t s0 = A.soff[k];
-  const int width = (int)((A.soff[k + 1] - s0) / kSliceRows);
-  const int64_t row0 = hs * kSliceHalf;
-  // both rows' heads before the image is cleared, so their loads overlap it
-  SliceRowHead h0, h1;
-  slice_head(A, row0 + w, lane, h0);
-  slice_head(A, row0 + w + kW, lane, h1);
-  for (int q = threadIdx.x; q < width * kSliceStride; q += blockDim.x) img[q] = 0.0;
+  constexpr int R = kSliceWarps * (32 / LR), kPitch = R + 1, kParts = kSliceRows / R;
+  const int r = threadIdx.x / LR, i0 = threadIdx.x % LR;
+  const int64_t step = gridDim.x;
+  SliceRowHead h = slice_head(A, slice_range(A, blockIdx.x * (int64_t)R + r), i0);
+  int2 rg = slice_range(A, (blockIdx.x + step) * R + r);
+  for (int q = threadIdx.x; q < (A.max_width + 1) * kPitch; q += kSliceThreads) img[q] = 0.0;
   __syncthreads();
-  if (h0.p1 - h0.p0 <= 32 && h1.p1 - h1.p0 <= 32) {
-    const SliceRowHead hh[2] = {h0, h1};
-    const int rr[2] = {w, w + kW};
-    const int64_t rows[2] = {row0 + w, row0 + w + kW};
-    slice_pair<NI, U, F32>(A, img, rr, rows, lane, hh);
-  } else {
-    if (h0.j >= 0) slice_row<NI, U, F32>(A, img, w, row0 + w, lane, h0);
-    if (h1.j >= 0) slice_row<NI, U, F32>(A, img, w + kW, row0 + w + kW, lane, h1);
-  }
-  __syncthreads();
-  for (int q = threadIdx.x; q < width * kSliceHalf; q += blockDim.x) {
-    const int sl = q / kSliceHalf, r = q % kSliceHalf;
-    const double v = img[sl * kSliceStride + r];
-    const int64_t at = s0 + (int64_t)sl * kSliceRows + half * kSliceHalf + r;
-    A.val64[at] = v;
-    A.val32[at] = (float)v;
+  for (int64_t part = blockIdx.x; part < A.n_parts; part += step) {
+    const int64_t row = part * R + r;
+    const int64_t s0 = A.soff[part / kParts], s1 = A.soff[part / kParts + 1];
+    const SliceRowHead hn = slice_head(A, rg, i0);
+    rg = slice_range(A, row + 2 * step * R);
+    slice_row<NI, U, F32, LR>(A, img, r, row, i0, h);
+    __syncthreads();
+    const int width = (int)((s1 - s0) / kSliceRows);
+    const int64_t at = s0 + (part % kParts) * R;
+    for (int t = threadIdx.x; t < width * (R / 2); t += kSliceThreads) {
+      const int sl = t / (R / 2), rr = 2 * (t % (R / 2));
+      double *p = img + sl * kPitch + rr;
+      const double2 v = {p[0], p[1]};
+      p[0] = 0.0;
+      p[1] = 0.0;
+      const int64_t o = at + sl * kSliceRows + rr;
+      *reinterpret_cast<double2 *>(A.val64 + o) = v;
+      *reinterpret_cast<float2 *>(A.val32 + o) = make_float2((float)v.x, (float)v.y);
+    }
+    __syncthreads();
+    h = hn;
   }
 }
 
@@ -740,6 +674,46 @@ int launch_nedelec(const Topology &t, const ElementTables &tab, const DeviceTopo
   return launch_nedelec_oriented(t, *dt.ort, dt, in, elem, cell_rhs, err, s, load_only);
 }
 
+namespace {
+
+constexpr size_t kSliceImage = 224 * 1024;  // image bytes of an SM's CTAs
+
+template <bool F32>
+int launch_slices(const SliceArgs &A, int lanes, size_t smem, cudaStream_t s) {
+  auto go = [&](auto kern) -> int {
+    int dev = 0, sms = 0, ctas = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+            cudaSuccess ||
+        cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, kern, kSliceThreads, smem) !=
+            cudaSuccess ||
+        ctas < 1)
+      return FFG_CUDA_ERROR;
+    const int64_t grid = std::min<int64_t>(A.n_parts, (int64_t)sms * ctas);
+    kern<<<(unsigned)grid, kSliceThreads, smem, s>>>(A);
+    return cudaGetLastError() == cudaSuccess ? FFG_OK : FFG_CUDA_ERROR;
+  };
+  const int ni = (A.nb + lanes - 1) / lanes;
+  // U and the CTAs per SM (the registers) by timing orders 3, 4 and 6: more
+  // loads in flight per warp at fewer warps, or fewer at spilled registers,
+  // both measured 5 % to 40 % slower
+  if (lanes == 16) {
+    if (ni == 2) return go(sell_slice_kernel<2, 2, F32, 16, 4>);
+    if (ni == 3) return go(sell_slice_kernel<3, 1, F32, 16, 5>);
+    if (ni == 6) return go(sell_slice_kernel<6, 1, F32, 16, 4>);
+  } else {
+    if (ni == 1) return go(sell_slice_kernel<1, 1, F32, 32, 4>);
+    if (ni == 2) return go(sell_slice_kernel<2, 1, F32, 32, 4>);
+    if (ni == 3) return go(sell_slice_kernel<3, 1, F32, 32, 4>);
+    if (ni == 5) return go(sell_slice_kernel<5, 1, F32, 32, 4>);
+    if (ni == 7) return go(sell_slice_kernel<7, 1, F32, 32, 3>);
+  }
+  return FFG_INVALID_INPUT;
+}
+
+}  // namespace
+
 int launch_columns(const Topology &t, const ElementTables &tab, const DeviceTopology &dt,
                    const AssemblyInputs &in, const double *geo, int stride,
                    const double *cell_rhs, const double *elem, const int64_t *col_ptr,
@@ -765,12 +739,17 @@ int launch_columns(const Topology &t, const ElementTables &tab, const DeviceTopo
   const bool by_warp = !sell && t.nb >= 16 && t.family != FFG_TRIANGLE_P1 && t.max_column > 0 &&
                        col_bytes <= kColSmem;
   const int wpb = by_warp ? std::max(1, std::min(8, kColSmem / col_bytes)) : 0;
-  // Nedelec SELL rows: one CTA per slice while the slice image fits
-  const size_t slice_smem = (size_t)t.max_column * kSliceStride * sizeof(double);
+  // Nedelec SELL rows: 16 lanes per row up to order 4 (their last step is
+  // fuller than a warp's), a warp per row above or where fewer than three
+  // images of 16 rows fit on an SM
+  const size_t row_smem = ((size_t)t.max_column + 1) * sizeof(double);
+  const int lanes = t.nb <= 96 && row_smem * 17 <= kSliceImage / 3 ? 16 : 32;
+  const int part_rows = kSliceThreads / lanes;
+  const size_t slice_smem = row_smem * (part_rows + 1);
   // incidence ranges stored as int32 (every incidence index below 2^31)
   const int64_t n_inc = t.n_free() > 0 ? (int64_t)t.nb * t.n_cells : 0;
-  if (sell && t.family == FFG_TETRA_NEDELEC && t.nb >= 16 && t.nb <= 128 && t.max_column > 0 &&
-      slice_smem <= 200 * 1024 && sell->perm && n_inc < (int64_t)INT32_MAX) {
+  if (sell && t.family == FFG_TETRA_NEDELEC && t.nb >= 16 && t.max_column > 0 &&
+      slice_smem <= kSliceImage && sell->perm && n_inc < (int64_t)INT32_MAX) {
     if (!sell->inc_range) {
       if (cudaMalloc((void **)&sell->inc_range, sizeof(int2) * (size_t)F) != cudaSuccess)
         return FFG_OUT_OF_MEMORY;
@@ -781,13 +760,11 @@ int launch_columns(const Topology &t, const ElementTables &tab, const DeviceTopo
     A.range = sell->inc_range;
     A.nb = t.nb;
     A.ld32 = ld32;
+    A.max_width = t.max_column;
     A.cs32 = cs32;
     A.n = F;
-    A.perm = sell->perm;
+    A.n_parts = sell->n_slices * (kSliceRows / part_rows);
     A.soff = sell->soff;
-    A.col_ptr = col_ptr;
-    A.inc_ptr = dt.inc_ptr;
-    A.row_idx = row_idx;
     A.inc_cell = dt.inc_cell;
     A.gd = dt.gd;
     A.inc_local = dt.inc_local;
@@ -801,26 +778,8 @@ int launch_columns(const Topology &t, const ElementTables &tab, const DeviceTopo
     A.rhs = rhs;
     A.val32 = sell->val32;
     A.dinv32 = sell->dinv32;
-    const int ni = (t.nb + 31) / 32;
-    auto go = [&](auto kern) -> int {
-      if (slice_smem > 48 * 1024 &&
-          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)slice_smem) != cudaSuccess)
-        return FFG_CUDA_ERROR;
-      kern<<<(unsigned)(2 * sell->n_slices), kSliceThreads, slice_smem, s>>>(A);
-      return cudaGetLastError() == cudaSuccess ? FFG_OK : FFG_CUDA_ERROR;
-    };
-    // about eight loads of each kind in flight per lane
-    if (elem32) {
-      if (ni == 1) return go(sell_slice_kernel<1, 2, true>);
-      if (ni == 2) return go(sell_slice_kernel<2, 1, true>);
-      if (ni == 3) return go(sell_slice_kernel<3, 1, true>);
-      return go(sell_slice_kernel<4, 1, true>);
-    }
-    if (ni == 1) return go(sell_slice_kernel<1, 2, false>);
-    if (ni == 2) return go(sell_slice_kernel<2, 1, false>);
-    if (ni == 3) return go(sell_slice_kernel<3, 1, false>);
-    return go(sell_slice_kernel<4, 1, false>);
+    return elem32 ? launch_slices<true>(A, lanes, slice_smem, s)
+                  : launch_slices<false>(A, lanes, slice_smem, s);
   }
 #define FFG_LAUNCH(FAM)                                                                        \
   do {                                                                                         \
