@@ -1287,6 +1287,8 @@ void ffg_problem_solve_batch(int count, const int *handles, const double *const 
     a.ref = P.dt.ref;
     a.load_basis = P.dt.load_basis;
     a.g = g ? g[i] : nullptr;
+    a.max_width = t.max_column;
+    a.perm = P.S.perm;
     a.iperm = P.S.iperm;
     a.free_index = P.dt.free_index;
     a.soff = P.S.soff;

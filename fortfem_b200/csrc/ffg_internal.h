@@ -363,6 +363,7 @@ int geo_stride_for(const Topology &t, const ElementTables &tab);
 constexpr int kMaxAsmBatch = 48;
 struct AsmSys {
   int n_cells = 0, nq = 0, stride = 0, nb = 0;
+  int max_width = 0;  // longest column
   int64_t n_free = 0, n_dofs = 0;
   const int *cells = nullptr;
   const double *verts = nullptr;
@@ -378,7 +379,7 @@ struct AsmSys {
   const uint16_t *slot = nullptr;
   const int *gd = nullptr;
   const double *ref = nullptr, *load_basis = nullptr, *g = nullptr;
-  const int *iperm = nullptr, *free_index = nullptr;
+  const int *perm = nullptr, *iperm = nullptr, *free_index = nullptr;
   const int64_t *soff = nullptr;
   double *val64 = nullptr, *dinv64 = nullptr, *rhs = nullptr, *x = nullptr, *solution = nullptr;
   float *val32 = nullptr, *dinv32 = nullptr;

@@ -2,7 +2,8 @@
 // matrices with orientation transform (K2), and the atomic-free,
 // column-owner scatter into the constrained CSC (K3).
 //
-// K3 gives every CSC column (a free global DoF j) to one thread.  The thread
+// K3 gives every CSC column (a free global DoF j) to one thread, or to a group
+// of lanes (the slice gather below), which works in the same order.  The thread
 // walks the cells incident to j in ascending cell order, computes column l(j)
 // of each element matrix and adds it into the column's slots through the
 // precomputed slot map.  Every CSC value is therefore the sum of its element
@@ -16,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <vector>
 
 #include "ffg_internal.h"
 #include "tet_geometry.h"
@@ -352,37 +354,48 @@ __global__ void csc_column_warp_kernel(int64_t n_free, int max_len,
   if (lane == 0) rhs[j] = b - lift;
 }
 
-// SELL rows of Nedelec elements (n_b >= 16), one part of a slice (R rows) at a
-// time in 256-thread CTAs that stay on their SM: LR lanes gather one row (free
-// column j = perm[row]) over the element's local rows i, as
-// csc_column_warp_kernel does for a CSC column, into the part's image in shared
-// memory (slot s of row r at s * (R + 1) + r), every entry receiving its terms
-// in ascending incidence order as in column_kernel; then the CTA writes the
-// part's FP64 and FP32 values (R * 8 contiguous bytes of FP64 per slot step)
-// and clears the image behind it.  Bound: it moves the element matrices, the
-// slots and the rows once (3.2 GB at order 3 on a 24^3 box, 0.5 ms of copy
-// bandwidth), and came to issue slots and load latency first, so there is one
-// instruction stream for 32 / LR rows, no branch per entry, and what the next
-// part needs is loaded a part ahead.  Measured, a warp per row with a branch
-// per entry and CTAs of one part against this: order 3 on 24^3 1096 against
-// 693 us, order 4 (FP32 element matrices) on 17 x 16 x 17 940 against 693 us;
-// order 6 on 12^3, which went a thread per column, 5406 against 2212 us.
+// SELL rows, one part of a slice (R rows) at a time in CTAs that stay on their
+// SM: LR lanes gather one row (free column j = perm[row]) over the element's
+// local rows i, as csc_column_warp_kernel does for a CSC column, into the
+// part's image in shared memory (slot s of row r at s * (R + 1) + r), every
+// entry receiving its terms in ascending incidence order as in column_kernel;
+// then the CTA writes the part's FP64 and FP32 values (R * 8 contiguous bytes
+// of FP64 per slot step) and clears the image behind it.  Bound: it moves the
+// element matrices (Nedelec; the other families' entries are made here), the
+// slots and the rows once, and came to issue slots and load latency first, so
+// there is one instruction stream for 32 / LR rows, no branch per entry, and
+// what the next part needs is loaded a part ahead.
+//
+// Nedelec (3.2 GB at order 3 on a 24^3 box, 0.5 ms of copy bandwidth), a warp
+// per row with a branch per entry and CTAs of one part against this: order 3
+// on 24^3 1096 against 693 us, order 4 (FP32 element matrices) on 17 x 16 x 17
+// 940 against 693 us; order 6 on 12^3, which went a thread per column, 5406
+// against 2212 us.  The other families, a thread per column with read-modify-
+// write through L2 (column_kernel) against this: P1 triangles on 64^2 8.5
+// against 4.7 us, P2 tetrahedra on 10^3, 21^3 and 48^3 91, 157 and 1197
+// against 21, 66 and 613 us, P3 on 14^3 791 against 356 us, Nedelec order 1
+// on 15^3 28 against 8 us, five P2 systems of 8^3 to 14^3 in one batch 154
+// against 47 us.  The tensor families are bound by L1 wavefronts of the
+// reference tensors: 7 NI loads of 32 / LR short segments per incidence step.
 struct SliceArgs {
   const int2 *range;  // per SELL row: [p0, p1) of its column's incidences
   int nb, ld32, max_width;
   int64_t cs32;  // FP32 element matrices: elements per cell
-  int64_t n, n_parts;  // rows (free DoFs), parts of all slices
+  int64_t n_free, n_parts;  // rows, parts of all slices
   const int64_t *soff;
   const int *inc_cell, *gd;
   const uint8_t *inc_local;
   const uint16_t *slot;
   const double *elem, *cell_rhs, *g;
+  const double *geo, *ref, *load_basis;  // tensor families and triangles (column_body)
+  int stride, nq;
   const float *elem32;
   double *val64, *dinv64, *rhs;
   float *val32, *dinv32;
 };
-constexpr int kSliceThreads = 256;
-constexpr int kSliceWarps = kSliceThreads / 32;
+// Threads of a CTA whose groups of LR lanes take one row each: parts of 8, 16
+// or 32 rows.
+__host__ __device__ constexpr int slice_threads(int lr) { return lr == 4 ? 128 : 256; }
 
 // One row: its incidence range [p0, p1) (empty past the last row) and its
 // first LR incidences' cells and local indices, one per lane of its group.
@@ -391,10 +404,16 @@ struct SliceRowHead {
 };
 
 __device__ __forceinline__ int2 slice_range(const SliceArgs &A, int64_t row) {
-  return row < A.n ? A.range[row] : make_int2(0, 0);
+  return row < A.n_free ? A.range[row] : make_int2(0, 0);
+}
+__device__ __forceinline__ int2 slice_range(const AsmSys &A, int64_t row) {
+  if (row >= A.n_free) return make_int2(0, 0);
+  const int j = A.perm[row];
+  return make_int2((int)A.inc_ptr[j], (int)A.inc_ptr[j + 1]);
 }
 
-__device__ __forceinline__ SliceRowHead slice_head(const SliceArgs &A, int2 rg, int i0) {
+template <class Args>
+__device__ __forceinline__ SliceRowHead slice_head(const Args &A, int2 rg, int i0) {
   SliceRowHead h{rg.x, rg.y, 0, 0};
   if (i0 < rg.y - rg.x) {
     h.e = A.inc_cell[(int64_t)rg.x + i0];
@@ -412,15 +431,30 @@ __global__ void inc_range_kernel(int64_t n, const int *perm, const int64_t *inc_
   range[r] = make_int2((int)inc_ptr[j], (int)inc_ptr[j + 1]);
 }
 
+// The load of local DoF l of cell e (as column_body sums it).
+template <int FAMILY, class Args>
+__device__ __forceinline__ double slice_load(const Args &A, int e, int l) {
+  if constexpr (FAMILY == FFG_TETRA_NEDELEC) {
+    return A.cell_rhs[(size_t)A.nb * e + l];
+  } else if constexpr (FAMILY == FFG_TRIANGLE_P1) {
+    return A.geo[10 * (size_t)e + 9];
+  } else {
+    const double *gg = A.geo + (size_t)A.stride * e + 7;
+    double F = 0.0;
+    for (int q = 0; q < A.nq; ++q) F += gg[q] * __ldg(A.load_basis + (size_t)q * A.nb + l);
+    return F;
+  }
+}
+
 // Row r of the part by the calling group of LR lanes (32 / LR rows per warp
 // side by side); the lane's local rows are i0, i0 + LR, ..., of which only the
 // last can be past nb.  Loads of U incidences are issued before any is added.
 // Constrained local rows are added to a slot behind the image that nothing
 // reads, so that the adds have no branches.
-template <int NI, int U, bool F32, int LR>
-__device__ __forceinline__ void slice_row(const SliceArgs &A, double *img, int r, int64_t row,
-                                          int i0, const SliceRowHead &h) {
-  constexpr int kPitch = kSliceWarps * (32 / LR) + 1;
+template <int FAMILY, int NI, int U, bool F32, int LR, class Args>
+__device__ __forceinline__ void slice_row(const Args &A, double *img, int r, int64_t row, int i0,
+                                          const SliceRowHead &h) {
+  constexpr int kPitch = slice_threads(LR) / LR + 1;
   constexpr unsigned kAll = 0xffffffffu;
   const int nb = A.nb;
   const bool tail = i0 + LR * (NI - 1) < nb;
@@ -436,9 +470,13 @@ __device__ __forceinline__ void slice_row(const SliceArgs &A, double *img, int r
       l = base + i0 < cnt ? A.inc_local[p] : 0;
     }
     // the lane's incidence: the offset of its element column and its load
-    const size_t my_col = F32 ? (size_t)e * (size_t)A.cs32 + (size_t)(A.ld32 * l)
-                              : ((size_t)e * nb + l) * (size_t)nb;
-    const double my_f = base + i0 < cnt ? A.cell_rhs[(size_t)nb * e + l] : 0.0;
+    size_t my_col = 0;
+    if constexpr (FAMILY == FFG_TETRA_NEDELEC)
+      my_col = F32 ? (size_t)e * (size_t)A.cs32 + (size_t)(A.ld32 * l)
+                   : ((size_t)e * nb + l) * (size_t)nb;
+    else if constexpr (FAMILY == FFG_TRIANGLE_P1)
+      my_col = 10 * (size_t)e + 3 * l;
+    const double my_f = base + i0 < cnt ? slice_load<FAMILY>(A, e, l) : 0.0;
     const uint16_t *slp = A.slot + ((size_t)h.p0 + base) * nb + i0;
     const int n = min(LR, all - base);
     for (int u0 = 0; u0 < n; u0 += U) {
@@ -447,13 +485,38 @@ __device__ __forceinline__ void slice_row(const SliceArgs &A, double *img, int r
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const bool live = base + u0 + u < cnt;
-        const size_t col = __shfl_sync(kAll, my_col, (u0 + u) & (LR - 1), LR) + i0;
+        const int from = (u0 + u) & (LR - 1);
 #pragma unroll
-        for (int c = 0; c < NI; ++c) {
-          const bool in = live && (c < NI - 1 || tail);
-          if (F32) kil[u][c] = in ? (double)__ldg(A.elem32 + col + LR * c) : 0.0;
-          else kil[u][c] = in ? __ldg(A.elem + col + LR * c) : 0.0;
-          sl[u][c] = in ? (int)__ldg(slp + LR * c) : (int)kConstrainedSlot;
+        for (int c = 0; c < NI; ++c)
+          sl[u][c] = live && (c < NI - 1 || tail) ? (int)__ldg(slp + LR * c)
+                                                  : (int)kConstrainedSlot;
+        if constexpr (FAMILY == FFG_TETRA_LAGRANGE) {
+          const double *gg = A.geo + (size_t)A.stride * __shfl_sync(kAll, e, from, LR);
+          const double *rf = A.ref + nb * __shfl_sync(kAll, l, from, LR) + i0;
+          double gco[7];
+#pragma unroll
+          for (int t = 0; t < 7; ++t) gco[t] = __ldg(gg + t);
+#pragma unroll
+          for (int c = 0; c < NI; ++c) {
+            kil[u][c] = 0.0;
+            if (c < NI - 1 || tail) {
+#pragma unroll
+              for (int t = 0; t < 7; ++t)
+                kil[u][c] += gco[t] * __ldg(rf + t * nb * nb + LR * c);
+            }
+          }
+        } else {
+          const size_t col = __shfl_sync(kAll, my_col, from, LR) + i0;
+#pragma unroll
+          for (int c = 0; c < NI; ++c) {
+            const bool in = live && (c < NI - 1 || tail);
+            if constexpr (FAMILY == FFG_TRIANGLE_P1)
+              kil[u][c] = in ? __ldg(A.geo + col + LR * c) : 0.0;
+            else if constexpr (F32)
+              kil[u][c] = in ? (double)__ldg(A.elem32 + col + LR * c) : 0.0;
+            else
+              kil[u][c] = in ? __ldg(A.elem + col + LR * c) : 0.0;
+          }
         }
         slp += nb;
       }
@@ -490,7 +553,7 @@ __device__ __forceinline__ void slice_row(const SliceArgs &A, double *img, int r
 #pragma unroll
     for (int o = LR / 2; o > 0; o >>= 1) lift += __shfl_xor_sync(kAll, lift, o);
   }
-  if (i0 == 0 && row < A.n) {
+  if (i0 == 0 && row < A.n_free) {
     const double d = dslot < A.max_width ? img[dslot * kPitch + r] : 0.0;
     const double di = (fabs(d) > 1.0e-14) ? 1.0 / d : 1.0;
     A.dinv64[row] = di;
@@ -499,39 +562,44 @@ __device__ __forceinline__ void slice_row(const SliceArgs &A, double *img, int r
   }
 }
 
+// The part's image to its slice, starting at entry `at`; the image is cleared.
+template <int LR, class Args>
+__device__ __forceinline__ void slice_write(const Args &A, double *img, int64_t at, int width) {
+  constexpr int R = slice_threads(LR) / LR;
+  for (int t = threadIdx.x; t < width * (R / 2); t += slice_threads(LR)) {
+    const int sl = t / (R / 2), rr = 2 * (t % (R / 2));
+    double *p = img + sl * (R + 1) + rr;
+    const double2 v = {p[0], p[1]};
+    p[0] = 0.0;
+    p[1] = 0.0;
+    const int64_t o = at + sl * kSliceRows + rr;
+    *reinterpret_cast<double2 *>(A.val64 + o) = v;
+    *reinterpret_cast<float2 *>(A.val32 + o) = make_float2((float)v.x, (float)v.y);
+  }
+}
+
 // The next part's incidences and the ranges of the one after it are loaded
 // while a part is gathered, so that the chain range -> incidence -> element
 // column costs one memory latency per part.
-template <int NI, int U, bool F32, int LR, int CTAS>
-__global__ void __launch_bounds__(kSliceThreads, CTAS)
+template <int FAMILY, int NI, int U, bool F32, int LR, int CTAS>
+__global__ void __launch_bounds__(slice_threads(LR), CTAS)
 sell_slice_kernel(const __grid_constant__ SliceArgs A) {
   extern __shared__ double img[];
-  constexpr int R = kSliceWarps * (32 / LR), kPitch = R + 1, kParts = kSliceRows / R;
+  constexpr int R = slice_threads(LR) / LR, kParts = kSliceRows / R;
   const int r = threadIdx.x / LR, i0 = threadIdx.x % LR;
   const int64_t step = gridDim.x;
   SliceRowHead h = slice_head(A, slice_range(A, blockIdx.x * (int64_t)R + r), i0);
   int2 rg = slice_range(A, (blockIdx.x + step) * R + r);
-  for (int q = threadIdx.x; q < (A.max_width + 1) * kPitch; q += kSliceThreads) img[q] = 0.0;
+  for (int q = threadIdx.x; q < (A.max_width + 1) * (R + 1); q += slice_threads(LR)) img[q] = 0.0;
   __syncthreads();
   for (int64_t part = blockIdx.x; part < A.n_parts; part += step) {
     const int64_t row = part * R + r;
     const int64_t s0 = A.soff[part / kParts], s1 = A.soff[part / kParts + 1];
     const SliceRowHead hn = slice_head(A, rg, i0);
     rg = slice_range(A, row + 2 * step * R);
-    slice_row<NI, U, F32, LR>(A, img, r, row, i0, h);
+    slice_row<FAMILY, NI, U, F32, LR>(A, img, r, row, i0, h);
     __syncthreads();
-    const int width = (int)((s1 - s0) / kSliceRows);
-    const int64_t at = s0 + (part % kParts) * R;
-    for (int t = threadIdx.x; t < width * (R / 2); t += kSliceThreads) {
-      const int sl = t / (R / 2), rr = 2 * (t % (R / 2));
-      double *p = img + sl * kPitch + rr;
-      const double2 v = {p[0], p[1]};
-      p[0] = 0.0;
-      p[1] = 0.0;
-      const int64_t o = at + sl * kSliceRows + rr;
-      *reinterpret_cast<double2 *>(A.val64 + o) = v;
-      *reinterpret_cast<float2 *>(A.val32 + o) = make_float2((float)v.x, (float)v.y);
-    }
+    slice_write<LR>(A, img, s0 + (part % kParts) * R, (int)((s1 - s0) / kSliceRows));
     __syncthreads();
     h = hn;
   }
@@ -574,6 +642,27 @@ __global__ void batch_geometry_kernel(const __grid_constant__ AsmBatch B) {
     p1_geometry_cell(c, S.cells, S.verts, S.ca, S.cb, S.cell_a, S.cell_b, S.samples, S.geo, S.err);
 }
 
+// The parts of every system's slices, one per CTA, and x = 0 for its solve.
+template <int FAMILY, int NI, int LR>
+__global__ void __launch_bounds__(slice_threads(LR))
+batch_slice_kernel(const __grid_constant__ AsmBatch B) {
+  extern __shared__ double img[];
+  constexpr int R = slice_threads(LR) / LR, kParts = kSliceRows / R;
+  const int s = batch_find(B.col_begin, B.count, blockIdx.x);
+  const AsmSys &S = B.sys[s];
+  const int64_t part = blockIdx.x - B.col_begin[s];
+  const int r = threadIdx.x / LR, i0 = threadIdx.x % LR;
+  const int64_t row = part * R + r;
+  const SliceRowHead h = slice_head(S, slice_range(S, row), i0);
+  const int64_t s0 = S.soff[part / kParts], s1 = S.soff[part / kParts + 1];
+  for (int q = threadIdx.x; q < (S.max_width + 1) * (R + 1); q += slice_threads(LR)) img[q] = 0.0;
+  if (i0 == 0 && row < S.n_free) S.x[row] = 0.0;
+  __syncthreads();
+  slice_row<FAMILY, NI, 1, false, LR>(S, img, r, row, i0, h);
+  __syncthreads();
+  slice_write<LR>(S, img, s0 + (part % kParts) * R, (int)((s1 - s0) / kSliceRows));
+}
+
 // the SELL-layout scatter of every system, and x = 0 for its solve
 template <int FAMILY>
 __global__ void batch_column_kernel(const __grid_constant__ AsmBatch B) {
@@ -603,28 +692,166 @@ __global__ void batch_solution_kernel(const __grid_constant__ AsmBatch B) {
 
 }  // namespace
 
+namespace {
+
+constexpr size_t kSliceImage = 224 * 1024;  // image bytes of an SM's CTAs
+
+// Lanes per row of the slice gather, 0 where a part's image does not fit on an
+// SM.  Narrow groups keep their lanes full on small elements and share one
+// instruction stream between more rows, but have more rows per image: the
+// narrowest for which three images fit on an SM, else a warp per row (16 lanes
+// for the tensor families) while one does.
+int slice_lanes(int family, int nb, int64_t max_column) {
+  auto image = [&](int lr) {
+    return sizeof(double) * (size_t)(max_column + 1) * (slice_threads(lr) / lr + 1);
+  };
+  if (max_column <= 0) return 0;
+  int first = 32, last = 32;
+  if (family == FFG_TETRA_NEDELEC) {
+    first = nb < 16 ? 8 : nb <= 96 ? 16 : 32;
+    last = nb < 16 ? 8 : 32;
+  } else if (family == FFG_TRIANGLE_P1) {
+    first = last = 4;
+  } else if (family == FFG_TETRA_LAGRANGE) {
+    first = nb == 4 ? 4 : 8;
+    last = nb == 4 ? 4 : 16;
+  } else {
+    return 0;
+  }
+  if (image(first) <= kSliceImage / 3) return first;
+  return image(last) <= kSliceImage ? last : 0;
+}
+size_t slice_bytes(int lr, int64_t max_column) {
+  return sizeof(double) * (size_t)(max_column + 1) * (slice_threads(lr) / lr + 1);
+}
+
+template <int FAMILY, bool F32>
+int launch_slices(const SliceArgs &A, int lanes, size_t smem, cudaStream_t s) {
+  auto go = [&](auto kern) -> int {
+    const int threads = slice_threads(lanes);
+    int dev = 0, sms = 0, ctas = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+            cudaSuccess ||
+        cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, kern, threads, smem) !=
+            cudaSuccess ||
+        ctas < 1)
+      return FFG_CUDA_ERROR;
+    const int64_t grid = std::min<int64_t>(A.n_parts, (int64_t)sms * ctas);
+    kern<<<(unsigned)grid, threads, smem, s>>>(A);
+    return cudaGetLastError() == cudaSuccess ? FFG_OK : FFG_CUDA_ERROR;
+  };
+  const int ni = (A.nb + lanes - 1) / lanes;
+  if constexpr (FAMILY == FFG_TETRA_NEDELEC) {
+    // U and the CTAs per SM (the registers) by timing orders 3, 4 and 6: more
+    // loads in flight per warp at fewer warps, or fewer at spilled registers,
+    // both measured 5 % to 40 % slower
+    if (lanes == 8) return go(sell_slice_kernel<FAMILY, 1, 2, F32, 8, 4>);
+    if (lanes == 16) {
+      if (ni == 2) return go(sell_slice_kernel<FAMILY, 2, 2, F32, 16, 4>);
+      if (ni == 3) return go(sell_slice_kernel<FAMILY, 3, 1, F32, 16, 5>);
+      if (ni == 6) return go(sell_slice_kernel<FAMILY, 6, 1, F32, 16, 4>);
+    } else {
+      if (ni == 1) return go(sell_slice_kernel<FAMILY, 1, 1, F32, 32, 4>);
+      if (ni == 2) return go(sell_slice_kernel<FAMILY, 2, 1, F32, 32, 4>);
+      if (ni == 3) return go(sell_slice_kernel<FAMILY, 3, 1, F32, 32, 4>);
+      if (ni == 5) return go(sell_slice_kernel<FAMILY, 5, 1, F32, 32, 4>);
+      if (ni == 7) return go(sell_slice_kernel<FAMILY, 7, 1, F32, 32, 3>);
+    }
+  } else if constexpr (FAMILY == FFG_TRIANGLE_P1) {
+    return go(sell_slice_kernel<FAMILY, 1, 1, false, 4, 8>);
+  } else {
+    if (lanes == 4) return go(sell_slice_kernel<FAMILY, 1, 1, false, 4, 8>);
+    if (lanes == 8) {
+      if (ni == 2) return go(sell_slice_kernel<FAMILY, 2, 1, false, 8, 4>);
+      if (ni == 3) return go(sell_slice_kernel<FAMILY, 3, 1, false, 8, 4>);
+      if (ni == 5) return go(sell_slice_kernel<FAMILY, 5, 1, false, 8, 4>);
+    } else {
+      if (ni == 1) return go(sell_slice_kernel<FAMILY, 1, 1, false, 16, 4>);
+      if (ni == 2) return go(sell_slice_kernel<FAMILY, 2, 1, false, 16, 4>);
+      if (ni == 3) return go(sell_slice_kernel<FAMILY, 3, 1, false, 16, 4>);
+    }
+  }
+  return FFG_INVALID_INPUT;
+}
+
+// The slices of the batch's systems, all of one nb and one lane count.
+int launch_batch_slices(int family, int lanes, AsmBatch &B, cudaStream_t s) {
+  const int rows = slice_threads(lanes) / lanes;
+  int max_width = 0;
+  for (int i = 0; i < B.count; ++i) {
+    max_width = std::max(max_width, B.sys[i].max_width);
+    B.col_begin[i + 1] = B.col_begin[i] + (B.sys[i].n_free + kSliceRows - 1) / kSliceRows *
+                                              (kSliceRows / rows);
+  }
+  const int64_t parts = B.col_begin[B.count];
+  if (!parts) return FFG_OK;
+  const size_t smem = slice_bytes(lanes, max_width);
+  auto go = [&](auto kern) -> int {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+        cudaSuccess)
+      return FFG_CUDA_ERROR;
+    kern<<<(unsigned)parts, slice_threads(lanes), smem, s>>>(B);
+    return cudaGetLastError() == cudaSuccess ? FFG_OK : FFG_CUDA_ERROR;
+  };
+  if (family == FFG_TRIANGLE_P1) return go(batch_slice_kernel<FFG_TRIANGLE_P1, 1, 4>);
+  const int ni = (B.sys[0].nb + lanes - 1) / lanes;
+  if (lanes == 4) return go(batch_slice_kernel<FFG_TETRA_LAGRANGE, 1, 4>);
+  if (lanes == 8) {
+    if (ni == 2) return go(batch_slice_kernel<FFG_TETRA_LAGRANGE, 2, 8>);
+    if (ni == 3) return go(batch_slice_kernel<FFG_TETRA_LAGRANGE, 3, 8>);
+    if (ni == 5) return go(batch_slice_kernel<FFG_TETRA_LAGRANGE, 5, 8>);
+  } else {
+    if (ni == 1) return go(batch_slice_kernel<FFG_TETRA_LAGRANGE, 1, 16>);
+    if (ni == 2) return go(batch_slice_kernel<FFG_TETRA_LAGRANGE, 2, 16>);
+    if (ni == 3) return go(batch_slice_kernel<FFG_TETRA_LAGRANGE, 3, 16>);
+  }
+  return FFG_INVALID_INPUT;
+}
+
+}  // namespace
+
 int launch_batch_assembly(int family, int count, const AsmSys *sys, cudaStream_t s) {
   if (family != FFG_TETRA_LAGRANGE && family != FFG_TRIANGLE_P1) return FFG_INVALID_INPUT;
-  for (int c0 = 0; c0 < count; c0 += kMaxAsmBatch) {
+  // one launch per phase for the systems of one element size and lane count
+  // (a system is gathered here as it is alone)
+  std::vector<int> left(count);
+  for (int i = 0; i < count; ++i) left[i] = i;
+  auto lanes_of = [&](int i) { return slice_lanes(family, sys[i].nb, sys[i].max_width); };
+  while (!left.empty()) {
+    const int nb = sys[left[0]].nb, lanes = lanes_of(left[0]);
     AsmBatch B;
-    B.count = std::min(kMaxAsmBatch, count - c0);
+    B.count = 0;
     B.cell_begin[0] = B.col_begin[0] = B.dof_begin[0] = 0;
-    for (int i = 0; i < B.count; ++i) {
-      B.sys[i] = sys[c0 + i];
-      B.cell_begin[i + 1] = B.cell_begin[i] + B.sys[i].n_cells;
-      B.col_begin[i + 1] = B.col_begin[i] + B.sys[i].n_free;
-      B.dof_begin[i + 1] = B.dof_begin[i] + B.sys[i].n_dofs;
+    std::vector<int> rest;
+    for (int i : left) {
+      if (sys[i].nb != nb || lanes_of(i) != lanes || B.count == kMaxAsmBatch) {
+        rest.push_back(i);
+        continue;
+      }
+      const int k = B.count++;
+      B.sys[k] = sys[i];
+      B.cell_begin[k + 1] = B.cell_begin[k] + sys[i].n_cells;
+      B.col_begin[k + 1] = B.col_begin[k] + sys[i].n_free;
+      B.dof_begin[k + 1] = B.dof_begin[k] + sys[i].n_dofs;
     }
+    left.swap(rest);
     batch_prep_kernel<<<1, kMaxAsmBatch, 0, s>>>(B);
     const int64_t nc = B.cell_begin[B.count], nf = B.col_begin[B.count];
     if (family == FFG_TETRA_LAGRANGE) {
       if (nc) batch_geometry_kernel<FFG_TETRA_LAGRANGE><<<blocks_for(nc, 128), 128, 0, s>>>(B);
-      if (nf) batch_column_kernel<FFG_TETRA_LAGRANGE><<<blocks_for(nf, 128), 128, 0, s>>>(B);
+      if (nf && !lanes)
+        batch_column_kernel<FFG_TETRA_LAGRANGE><<<blocks_for(nf, 128), 128, 0, s>>>(B);
     } else {
       if (nc) batch_geometry_kernel<FFG_TRIANGLE_P1><<<blocks_for(nc, 128), 128, 0, s>>>(B);
-      if (nf) batch_column_kernel<FFG_TRIANGLE_P1><<<blocks_for(nf, 128), 128, 0, s>>>(B);
+      if (nf && !lanes)
+        batch_column_kernel<FFG_TRIANGLE_P1><<<blocks_for(nf, 128), 128, 0, s>>>(B);
     }
     if (cudaGetLastError() != cudaSuccess) return FFG_CUDA_ERROR;
+    if (lanes) {
+      if (int st = launch_batch_slices(family, lanes, B, s)) return st;
+    }
   }
   return FFG_OK;
 }
@@ -674,46 +901,6 @@ int launch_nedelec(const Topology &t, const ElementTables &tab, const DeviceTopo
   return launch_nedelec_oriented(t, *dt.ort, dt, in, elem, cell_rhs, err, s, load_only);
 }
 
-namespace {
-
-constexpr size_t kSliceImage = 224 * 1024;  // image bytes of an SM's CTAs
-
-template <bool F32>
-int launch_slices(const SliceArgs &A, int lanes, size_t smem, cudaStream_t s) {
-  auto go = [&](auto kern) -> int {
-    int dev = 0, sms = 0, ctas = 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess ||
-        cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, kern, kSliceThreads, smem) !=
-            cudaSuccess ||
-        ctas < 1)
-      return FFG_CUDA_ERROR;
-    const int64_t grid = std::min<int64_t>(A.n_parts, (int64_t)sms * ctas);
-    kern<<<(unsigned)grid, kSliceThreads, smem, s>>>(A);
-    return cudaGetLastError() == cudaSuccess ? FFG_OK : FFG_CUDA_ERROR;
-  };
-  const int ni = (A.nb + lanes - 1) / lanes;
-  // U and the CTAs per SM (the registers) by timing orders 3, 4 and 6: more
-  // loads in flight per warp at fewer warps, or fewer at spilled registers,
-  // both measured 5 % to 40 % slower
-  if (lanes == 16) {
-    if (ni == 2) return go(sell_slice_kernel<2, 2, F32, 16, 4>);
-    if (ni == 3) return go(sell_slice_kernel<3, 1, F32, 16, 5>);
-    if (ni == 6) return go(sell_slice_kernel<6, 1, F32, 16, 4>);
-  } else {
-    if (ni == 1) return go(sell_slice_kernel<1, 1, F32, 32, 4>);
-    if (ni == 2) return go(sell_slice_kernel<2, 1, F32, 32, 4>);
-    if (ni == 3) return go(sell_slice_kernel<3, 1, F32, 32, 4>);
-    if (ni == 5) return go(sell_slice_kernel<5, 1, F32, 32, 4>);
-    if (ni == 7) return go(sell_slice_kernel<7, 1, F32, 32, 3>);
-  }
-  return FFG_INVALID_INPUT;
-}
-
-}  // namespace
-
 int launch_columns(const Topology &t, const ElementTables &tab, const DeviceTopology &dt,
                    const AssemblyInputs &in, const double *geo, int stride,
                    const double *cell_rhs, const double *elem, const int64_t *col_ptr,
@@ -739,17 +926,11 @@ int launch_columns(const Topology &t, const ElementTables &tab, const DeviceTopo
   const bool by_warp = !sell && t.nb >= 16 && t.family != FFG_TRIANGLE_P1 && t.max_column > 0 &&
                        col_bytes <= kColSmem;
   const int wpb = by_warp ? std::max(1, std::min(8, kColSmem / col_bytes)) : 0;
-  // Nedelec SELL rows: 16 lanes per row up to order 4 (their last step is
-  // fuller than a warp's), a warp per row above or where fewer than three
-  // images of 16 rows fit on an SM
-  const size_t row_smem = ((size_t)t.max_column + 1) * sizeof(double);
-  const int lanes = t.nb <= 96 && row_smem * 17 <= kSliceImage / 3 ? 16 : 32;
-  const int part_rows = kSliceThreads / lanes;
-  const size_t slice_smem = row_smem * (part_rows + 1);
+  // SELL rows by the slice gather
+  const int lanes = sell && sell->perm ? slice_lanes(t.family, t.nb, t.max_column) : 0;
   // incidence ranges stored as int32 (every incidence index below 2^31)
-  const int64_t n_inc = t.n_free() > 0 ? (int64_t)t.nb * t.n_cells : 0;
-  if (sell && t.family == FFG_TETRA_NEDELEC && t.nb >= 16 && t.max_column > 0 &&
-      slice_smem <= kSliceImage && sell->perm && n_inc < (int64_t)INT32_MAX) {
+  const int64_t n_inc = (int64_t)t.nb * t.n_cells;
+  if (lanes && n_inc < (int64_t)INT32_MAX) {
     if (!sell->inc_range) {
       if (cudaMalloc((void **)&sell->inc_range, sizeof(int2) * (size_t)F) != cudaSuccess)
         return FFG_OUT_OF_MEMORY;
@@ -762,8 +943,8 @@ int launch_columns(const Topology &t, const ElementTables &tab, const DeviceTopo
     A.ld32 = ld32;
     A.max_width = t.max_column;
     A.cs32 = cs32;
-    A.n = F;
-    A.n_parts = sell->n_slices * (kSliceRows / part_rows);
+    A.n_free = F;
+    A.n_parts = sell->n_slices * (kSliceRows * lanes / slice_threads(lanes));
     A.soff = sell->soff;
     A.inc_cell = dt.inc_cell;
     A.gd = dt.gd;
@@ -772,14 +953,24 @@ int launch_columns(const Topology &t, const ElementTables &tab, const DeviceTopo
     A.elem = elem;
     A.cell_rhs = cell_rhs;
     A.g = in.g;
+    A.geo = geo;
+    A.ref = dt.ref;
+    A.load_basis = dt.load_basis;
+    A.stride = stride;
+    A.nq = tab.nq_load;
     A.elem32 = elem32;
     A.val64 = sell->val64;
     A.dinv64 = sell->dinv64;
     A.rhs = rhs;
     A.val32 = sell->val32;
     A.dinv32 = sell->dinv32;
-    return elem32 ? launch_slices<true>(A, lanes, slice_smem, s)
-                  : launch_slices<false>(A, lanes, slice_smem, s);
+    const size_t smem = slice_bytes(lanes, t.max_column);
+    if (t.family == FFG_TETRA_LAGRANGE)
+      return launch_slices<FFG_TETRA_LAGRANGE, false>(A, lanes, smem, s);
+    if (t.family == FFG_TRIANGLE_P1)
+      return launch_slices<FFG_TRIANGLE_P1, false>(A, lanes, smem, s);
+    return elem32 ? launch_slices<FFG_TETRA_NEDELEC, true>(A, lanes, smem, s)
+                  : launch_slices<FFG_TETRA_NEDELEC, false>(A, lanes, smem, s);
   }
 #define FFG_LAUNCH(FAM)                                                                        \
   do {                                                                                         \

@@ -14,6 +14,7 @@ import oracle
 import fortfem_b200 as ff
 from fortfem_b200 import _capi as K
 from fortfem_b200 import synth
+from fortfem_b200.api import solve_batch
 
 pytestmark = pytest.mark.gpu
 
@@ -37,7 +38,7 @@ def box(n):
     return synth.jitter_interior(v, 1.0 / n, 0.1, 5), t
 
 
-def operator(prob, v, ca, cb, cell_a, src, g, x):
+def operator(prob, v, ca, cb, cell_a, src, g, x, assemble=True):
     """rhs, 1 / diagonal and A x, in the order of the free DoFs."""
     import torch
 
@@ -52,8 +53,9 @@ def operator(prob, v, ca, cb, cell_a, src, g, x):
     assert st.value == 0
     xs = torch.as_tensor(x[perm], device="cuda")
     rhs, dinv, y = (torch.zeros(prob.n_free, dtype=torch.float64, device="cuda") for _ in range(3))
-    lib.ffg_problem_assemble(prob.handle, p(dev[0]), ca, cb, p(dev[1]), None, p(dev[2]), p(dev[3]),
-                             1, None, ctypes.byref(st))
+    if assemble:
+        lib.ffg_problem_assemble(prob.handle, p(dev[0]), ca, cb, p(dev[1]), None, p(dev[2]),
+                                 p(dev[3]), 1, None, ctypes.byref(st))
     assert st.value == 0
     lib.ffg_problem_system_arrays(prob.handle, p(rhs), p(dinv), 1, None, ctypes.byref(st))
     assert st.value == 0
@@ -68,8 +70,9 @@ def operator(prob, v, ca, cb, cell_a, src, g, x):
     return out
 
 
-NEDELEC = [  # 16 lanes per row, 32 where the order or a long row asks for it
-    (2, "box", 2), (3, "box", 2), (4, "box", 2), (5, "box", 1), (6, "box", 1),
+NEDELEC = [  # 8 lanes per row at order 1, 16 per row, 32 where the order or a long row asks for it
+    (1, "box", 2), (2, "box", 2), (3, "box", 2), (4, "box", 2), (5, "box", 1), (6, "box", 1),
+    (1, "fan", 40),
     (2, "fan", 24), (2, "fan", 70), (3, "fan", 40), (4, "fan", 20), (4, "fan", 60), (5, "fan", 9),
 ]
 
@@ -87,6 +90,74 @@ def test_nedelec_rows_match_oracle(k, mesh, n):
     check(ff.Problem(K.FFG_TETRA_NEDELEC, k, t, len(v), boundary=mask.astype(np.uint8)), v, 1.7,
           0.9, cell, src, g, mask, oracle.nedelec_csc(v, t, k, 1.7, 0.9, cell, None),
           oracle.nedelec_load_samples(v, t, k, src), {5: 1e-11, 6: 1e-10}.get(k, 1e-12), rng)
+
+
+LAGRANGE = [  # 4 lanes per row (p = 1), 8, 16 where a long row asks for it, a thread
+    (1, "box", 2), (2, "box", 2), (3, "box", 2), (4, "box", 1), (1, "fan", 70), (2, "fan", 60),
+    (2, "fan", 90), (3, "fan", 40), (4, "fan", 20), (4, "fan", 100),
+]
+
+
+def lagrange_case(p, mesh, n):
+    v, t = box(n) if mesh == "box" else fan(n)
+    q = p + 2
+    rng = np.random.default_rng(10 * p + n)
+    n_dofs = oracle.lagrange_csc(v, t, p, 0, q)[0]
+    mask = rng.random(n_dofs) < 0.15
+    cell = rng.uniform(0.5, 2.0, len(t))
+    pts = oracle.lagrange_quadrature_points(v, t, 0, q)
+    src = np.sin(pts[..., 0]) * np.cos(2 * pts[..., 1]) + pts[..., 2]
+    g = np.where(mask, rng.standard_normal(n_dofs), 0.0)
+    prob = ff.Problem(K.FFG_TETRA_LAGRANGE, p, t, len(v), quadrature_degree=q,
+                      boundary=mask.astype(np.uint8))
+    return prob, v, t, q, cell, src, g, mask, rng
+
+
+@pytest.mark.parametrize("p, mesh, n", LAGRANGE)
+def test_lagrange_rows_match_oracle(p, mesh, n):
+    prob, v, t, q, cell, src, g, mask, rng = lagrange_case(p, mesh, n)
+    check(prob, v, 1.7, 0.9, cell, src, g, mask, oracle.lagrange_csc(v, t, p, 0, q, 1.7, 0.9, cell),
+          oracle.lagrange_load_samples(v, t, p, src, 0, q), 1e-12, rng)
+
+
+@pytest.mark.parametrize("n", [3, 40])
+def test_p1_triangle_rows_match_oracle(n):
+    if n == 3:
+        v, t = oracle.unit_square_mesh(n + 1)
+    else:  # n triangles around one vertex
+        a = 2 * np.pi * np.arange(n) / n
+        v = np.concatenate([[[0.1, 0.0]], np.stack([np.cos(a), np.sin(a)], -1)])
+        i = np.arange(n)
+        t = np.stack([0 * i, 1 + i, 1 + (i + 1) % n], -1).astype(np.int32)
+    rng = np.random.default_rng(n)
+    mask = rng.random(len(v)) < 0.15
+    mask[0] = False
+    cell = rng.uniform(0.5, 2.0, len(t))
+    g = np.where(mask, rng.standard_normal(len(v)), 0.0)
+    check(ff.Problem(K.FFG_TRIANGLE_P1, 1, t, len(v), boundary=mask.astype(np.uint8)), v, 1.7, 0.9,
+          cell, np.ones(len(t)), g, mask, oracle.p1_csc(v, t, 0.9, 1.7, cell),
+          oracle.p1_load(v, t), 1e-12, rng)
+
+
+def test_batched_rows_are_the_bits_of_a_system_alone():
+    import torch
+
+    cases = [lagrange_case(*c) for c in [(2, "box", 2), (1, "box", 2), (3, "fan", 40),
+                                         (2, "fan", 90), (2, "fan", 60)]]
+    for i, _ in enumerate(cases):
+        rng = np.random.default_rng(i)
+        prob, v, t, q, cell, src, g, mask, _ = cases[i]
+        x = rng.standard_normal(prob.n_free)
+        cases[i] = (prob, v, cell, src, g, x, operator(prob, v, 1.7, 0.9, cell, src, g, x))
+    probs = [c[0] for c in cases]
+    dev = [[torch.as_tensor(c[k], device="cuda") for c in cases] for k in (1, 2, 3, 4)]
+    sol = [torch.zeros(p.n_dofs, dtype=torch.float64, device="cuda") for p in probs]
+    solve_batch(probs, dev[0], sol, [1.7] * 5, [0.9] * 5, dev[1], None, dev[2], dev[3])
+    torch.cuda.synchronize()
+    for prob, v, cell, src, g, x, alone in cases:
+        for a, b in zip(alone, operator(prob, v, 1.7, 0.9, cell, src, g, x, assemble=False)):
+            assert np.array_equal(a, b)
+        prob.close()
 
 
 def check(problem, v, ca, cb, cell, src, g, mask, csc, load, tol, rng):
