@@ -167,23 +167,46 @@ def unit_square_mesh(n: int):
 
 # -------------------------------------------------------- drop-in assembly
 
-def _csc_call(fn, args, where, capacity_hint=None):
+# A call's arrays are made for the largest possible pattern up to this many
+# bytes; untouched pages of them are never backed by memory.
+_CSC_BOUND_BYTES = 1 << 30
+
+
+def _csc_call(fn, args, where, n_cells=0, nb=0):
+    """One call of a CSC entry point.  With the element size nb given, the
+    arrays are made for the largest pattern that n_cells elements can have and
+    cut to the one returned: asking for the size first builds the topology
+    twice, which is most of the call."""
     lib = K.load()
     nd = C.c_int(0)
     nz = C.c_int64(0)
     st = C.c_int(0)
-    getattr(lib, fn)(*args, C.c_int64(0), C.byref(nd), C.byref(nz), None, None, None, C.byref(st))
-    if st.value not in (K.FFG_OK, K.FFG_CAPACITY):
-        return None, Status.of(st.value, where)
-    n = nd.value
-    cp = np.zeros(n + 1, np.int64)
-    ri = np.zeros(nz.value, np.int32)
-    val = np.zeros(nz.value)
-    getattr(lib, fn)(*args, C.c_int64(nz.value), C.byref(nd), C.byref(nz), _ptr(cp), _ptr(ri),
+    cap = n_cells * nb * nb
+    if not (0 < nb and 0 < cap * 12 <= _CSC_BOUND_BYTES):
+        getattr(lib, fn)(*args, C.c_int64(0), C.byref(nd), C.byref(nz), None, None, None,
+                         C.byref(st))
+        if st.value not in (K.FFG_OK, K.FFG_CAPACITY):
+            return None, Status.of(st.value, where)
+        n, cap = nd.value, nz.value
+    else:
+        n = n_cells * nb
+    cp = np.empty(n + 1, np.int64)
+    ri = np.empty(cap, np.int32)
+    val = np.empty(cap)
+    getattr(lib, fn)(*args, C.c_int64(cap), C.byref(nd), C.byref(nz), _ptr(cp), _ptr(ri),
                      _ptr(val), C.byref(st))
     if st.value:
         return None, Status.of(st.value, where)
-    return CscMatrix(n, n, cp, ri, val), Status()
+    n = nd.value
+    return CscMatrix(n, n, cp[:n + 1], ri[:nz.value], val[:nz.value]), Status()
+
+
+def _lagrange_nb(p):
+    return (p + 1) * (p + 2) * (p + 3) // 6 if 1 <= p <= 4 else 0
+
+
+def _nedelec_nb(k):
+    return k * (k + 2) * (k + 3) // 2 if 1 <= k <= 6 else 0
 
 
 def assemble_tetra_lagrange_stiffness_csc(mesh_vertices, tetrahedra, degree, quadrature_degree,
@@ -201,7 +224,7 @@ def assemble_tetra_lagrange_stiffness_csc(mesh_vertices, tetrahedra, degree, qua
             1.0 if stiffness_coefficient is None else float(stiffness_coefficient),
             0.0 if mass_coefficient is None else float(mass_coefficient), _ptr(cs), _ptr(cm)]
     return _csc_call("ffg_assemble_tetra_lagrange_stiffness_csc", args,
-                     "Tetrahedral H1 sparse assembly failed")
+                     "Tetrahedral H1 sparse assembly failed", len(t), _lagrange_nb(int(degree)))
 
 
 def assemble_tetra_lagrange_stiffness_csc_jvp(mesh_vertices, tetrahedra, degree, quadrature_degree,
@@ -223,7 +246,8 @@ def assemble_tetra_lagrange_stiffness_csc_jvp(mesh_vertices, tetrahedra, degree,
     args = [len(v), _ptr(v), len(t), _ptr(t), int(degree), int(rule), int(quadrature_degree),
             float(stiffness_coefficient), float(mass_coefficient), _ptr(vd),
             float(stiffness_coefficient_dot), float(mass_coefficient_dot)]
-    return _csc_call("ffg_assemble_tetra_lagrange_stiffness_csc_jvp", args, where)
+    return _csc_call("ffg_assemble_tetra_lagrange_stiffness_csc_jvp", args, where, len(t),
+                     _lagrange_nb(int(degree)))
 
 
 def assemble_tetra_lagrange_stiffness_csc_vjp(mesh_vertices, tetrahedra, degree, quadrature_degree,
@@ -282,7 +306,7 @@ def assemble_tetra_nedelec_curl_mass_csc(mesh_vertices, tetrahedra, curl_coeffic
             1.0 if mass_coefficient is None else float(mass_coefficient),
             _ptr(_opt(cell_curl, len(t))), _ptr(_opt(cell_mass, len(t)))]
     return _csc_call("ffg_assemble_tetra_nedelec_curl_mass_csc", args,
-                     "Tetrahedral Nedelec assembly failed")
+                     "Tetrahedral Nedelec assembly failed", len(t), _nedelec_nb(args[4]))
 
 
 def cell_tensors(coefficient, vertices, tetrahedra) -> np.ndarray:
@@ -332,7 +356,8 @@ def assemble_tetra_nedelec_curl_mass_csc_jvp(mesh_vertices, tetrahedra, order, c
     args = [len(v), _ptr(v), len(t), _ptr(t), int(order), float(curl_coefficient),
             float(mass_coefficient), _ptr(vd), float(curl_coefficient_dot),
             float(mass_coefficient_dot)]
-    return _csc_call("ffg_assemble_tetra_nedelec_curl_mass_csc_jvp", args, where)
+    return _csc_call("ffg_assemble_tetra_nedelec_curl_mass_csc_jvp", args, where, len(t),
+                     _nedelec_nb(int(order)))
 
 
 def assemble_tetra_nedelec_curl_mass_csc_vjp(mesh_vertices, tetrahedra, order, curl_coefficient,

@@ -59,6 +59,10 @@ int upload(T **p, const std::vector<T> &h) {
 
 // One device-resident problem: topology, tables, pattern, work buffers.
 struct Problem {
+  ProblemUse use = kUseSolve;
+  // device arrays of a problem of one call (use != kUseSolve): its topology,
+  // and what is made in the memory of the topology's scratch after it
+  DeviceArena arena, scratch;
   Topology topo;
   ElementTables tab;
   DeviceTopology dt;
@@ -97,8 +101,9 @@ struct Problem {
                     in_cell_a, in_cell_b, in_samples, in_g, free_dofs, cell_tensor, geo_w,
                     err, eval.lag_idx,
                     eval.terms, eval.coef};
-    for (void *p : ptrs)
-      if (p) cudaFree(p);
+    if (use == kUseSolve)
+      for (void *p : ptrs)
+        if (p) cudaFree(p);
     free_sell(S);
     tc_free_plan(tc);
     ort_free(ort);
@@ -140,9 +145,66 @@ void report(int verbosity, const std::string &msg) {
   if (verbosity > 0 && !msg.empty()) std::fprintf(stderr, "fortfem_gpu: %s\n", msg.c_str());
 }
 
+// An array of n entries of a problem of one call.
+template <class T>
+int arena_alloc(Problem &P, T **p, size_t n) {
+  *p = (T *)P.scratch.take(sizeof(T) * std::max<size_t>(n, 1));
+  return *p ? FFG_OK : FFG_OUT_OF_MEMORY;
+}
+
+// The tables and per-call arrays of a problem that serves one assembly into
+// the CSC or one adjoint.
+int alloc_for_call(Problem &P) {
+  const Topology &t = P.topo;
+  DeviceTopology &dt = P.dt;
+  int st;
+  auto table = [&](double **p, const std::vector<double> &h) -> int {
+    if (h.empty()) return FFG_OK;
+    if (int e = arena_alloc(P, p, h.size())) return e;
+    return cudaMemcpy(*p, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice) ==
+                   cudaSuccess
+               ? FFG_OK
+               : FFG_CUDA_ERROR;
+  };
+  if ((st = table(&dt.face_blocks, P.tab.face_blocks))) return st;
+  if ((st = table(&dt.ref, P.tab.ref))) return st;
+  if ((st = table(&dt.load_basis, P.tab.load_basis))) return st;
+  const size_t nc = (size_t)t.n_cells;
+  if (t.family == FFG_TETRA_NEDELEC) {
+    if ((st = ort_build(t, P.tab, P.ort))) return st;
+    dt.ort = &P.ort;
+    if ((st = arena_alloc(P, &P.cell_rhs, nc * t.nb))) return st;
+    if ((st = arena_alloc(P, &P.elem, nc * t.nb * t.nb))) return st;
+  }
+  if ((st = arena_alloc(P, &P.in_vertices, (size_t)t.n_vertices * P.dim))) return st;
+  if ((st = arena_alloc(P, &P.err, 4))) return st;
+  if (P.use == kUseAdjoint) return FFG_OK;
+  if ((st = arena_alloc(P, &P.geo, nc * std::max(P.geo_stride, 1)))) return st;
+  if ((st = arena_alloc(P, &P.rhs, (size_t)t.n_free()))) return st;
+  if ((st = arena_alloc(P, &P.in_cell_a, nc))) return st;
+  if ((st = arena_alloc(P, &P.in_cell_b, nc))) return st;
+  return arena_alloc(P, &P.csc_val, (size_t)t.nnz());
+}
+
+// The pattern of a problem of one call into the caller's arrays.
+int copy_pattern(const Problem &P, int64_t *col_ptr, int *row_ind) {
+  const Topology &t = P.topo;
+  if (P.use == kUseSolve) {
+    std::memcpy(col_ptr, t.col_ptr.data(), sizeof(int64_t) * t.col_ptr.size());
+    std::memcpy(row_ind, t.row_idx.data(), sizeof(int) * t.row_idx.size());
+    return FFG_OK;
+  }
+  return cudaMemcpy(col_ptr, P.csc_col_ptr, sizeof(int64_t) * ((size_t)t.n_free() + 1),
+                    cudaMemcpyDeviceToHost) == cudaSuccess &&
+                 cudaMemcpy(row_ind, P.csc_row, sizeof(int) * (size_t)t.nnz(),
+                            cudaMemcpyDeviceToHost) == cudaSuccess
+             ? FFG_OK
+             : FFG_CUDA_ERROR;
+}
+
 int create_problem(int family, int degree, int n_vertices, int n_cells, const int *cells, int rule,
                    int qdeg, int boundary_mode, const uint8_t *mask, std::shared_ptr<Problem> &out,
-                   std::string &msg) {
+                   std::string &msg, ProblemUse use = kUseSolve) {
   int st = device_ready();
   if (st) return st;
   auto P = std::make_shared<Problem>();
@@ -161,6 +223,8 @@ int create_problem(int family, int degree, int n_vertices, int n_cells, const in
   // triangles on the host
   const bool on_device =
       family == FFG_TETRA_LAGRANGE || family == FFG_TRIANGLE_P1 || family == FFG_TETRA_NEDELEC;
+  if (!on_device) use = kUseSolve;
+  P->use = use;
   if (on_device) {
     if (!validate_cells(t, msg)) return FFG_INVALID_INPUT;
     if (family == FFG_TRIANGLE_P1 && (t.vpc != 3 || degree != 1)) {
@@ -168,7 +232,9 @@ int create_problem(int family, int degree, int n_vertices, int n_cells, const in
       return FFG_INVALID_INPUT;
     }
     if ((st = build_topology_device(t, boundary_mode, mask, grid, P->dt, &P->csc_col_ptr,
-                                    &P->csc_row, P->S, msg)))
+                                    &P->csc_row, P->S, msg, use,
+                                    use == kUseSolve ? nullptr : &P->arena,
+                                    use == kUseSolve ? nullptr : &P->scratch)))
       return st;
   } else {
     if ((st = build_dofs(t, msg))) return st;
@@ -197,6 +263,11 @@ int create_problem(int family, int degree, int n_vertices, int n_cells, const in
     if ((st = upload(&P->csc_row, t.row_idx))) return st;
     build_sell(t.col_ptr, t.row_idx, kSellSigma, P->hsell);
     if ((st = upload_sell(P->hsell, grid, P->S))) return st;
+  }
+  if (use != kUseSolve) {
+    if ((st = alloc_for_call(*P))) return st;
+    out = P;
+    return FFG_OK;
   }
   if (!P->tab.face_blocks.empty() && (st = upload(&dt.face_blocks, P->tab.face_blocks))) return st;
   if (!P->tab.ref.empty() && (st = upload(&dt.ref, P->tab.ref))) return st;
@@ -1452,15 +1523,14 @@ static void full_csc(int family, int degree, int nv, const double *verts, int nt
   std::shared_ptr<Problem> P;
   std::string msg;
   int st = create_problem(family, degree, nv, nt, cells, rule, qdeg, FFG_BOUNDARY_NONE, nullptr, P,
-                          msg);
+                          msg, kUseCsc);
   if (st) { *status = st; return; }
   if (n_dofs) *n_dofs = (int)P->topo.n_dofs;
   if (nnz) *nnz = P->topo.nnz();
   if (cap < P->topo.nnz() || !col_ptr || !row_ind || !values) { *status = FFG_CAPACITY; return; }
   st = assemble(*P, verts, ca, cb, cell_a, cell_b, nullptr, nullptr, 0, false, 0, msg);
   if (st) { *status = st; return; }
-  std::memcpy(col_ptr, P->topo.col_ptr.data(), sizeof(int64_t) * P->topo.col_ptr.size());
-  std::memcpy(row_ind, P->topo.row_idx.data(), sizeof(int) * P->topo.row_idx.size());
+  if ((st = copy_pattern(*P, col_ptr, row_ind))) { *status = st; return; }
   if (cudaMemcpy(values, P->csc_val, sizeof(double) * (size_t)P->topo.nnz(), cudaMemcpyDeviceToHost) !=
       cudaSuccess) {
     *status = FFG_CUDA_ERROR;
@@ -1508,7 +1578,7 @@ static void tangent_csc(int family, int degree, int nv, const double *verts, int
   std::string msg;
   if (!verts || !verts_dot) { *status = FFG_INVALID_INPUT; return; }
   int st = create_problem(family, degree, nv, nt, cells, rule, qdeg, FFG_BOUNDARY_NONE, nullptr, P,
-                          msg);
+                          msg, kUseCsc);
   if (st) { *status = st; return; }
   const Topology &t = P->topo;
   if (n_dofs) *n_dofs = (int)t.n_dofs;
@@ -1516,12 +1586,7 @@ static void tangent_csc(int family, int degree, int nv, const double *verts, int
   if (cap < t.nnz() || !col_ptr || !row_ind || !values_dot) { *status = FFG_CAPACITY; return; }
   double *vdot = nullptr;
   const size_t vbytes = sizeof(double) * 3 * (size_t)nv;
-  if ((st = dalloc(&vdot, 3 * (size_t)nv))) { *status = st; return; }
-  if (!P->csc_val && (st = dalloc(&P->csc_val, (size_t)std::max<int64_t>(t.nnz(), 1)))) {
-    cudaFree(vdot);
-    *status = st;
-    return;
-  }
+  if ((st = arena_alloc(*P, &vdot, 3 * (size_t)nv))) { *status = st; return; }
   AssemblyInputs in;
   in.vertices = P->in_vertices;
   in.coef_a = ca;
@@ -1552,11 +1617,8 @@ static void tangent_csc(int family, int degree, int nv, const double *verts, int
         st = FFG_CUDA_ERROR;
     }
   }
-  cudaFree(vdot);
-  if (st) { *status = st; return; }
-  std::memcpy(col_ptr, t.col_ptr.data(), sizeof(int64_t) * t.col_ptr.size());
-  std::memcpy(row_ind, t.row_idx.data(), sizeof(int) * t.row_idx.size());
-  *status = FFG_OK;
+  if (!st) st = copy_pattern(*P, col_ptr, row_ind);
+  *status = st;
 }
 
 // Adjoint (VJP) of a stiffness/curl + mass CSC: vertex and coefficient
@@ -1575,16 +1637,14 @@ static void adjoint_csc(int family, int degree, int nv, const double *verts, int
   std::shared_ptr<Problem> P;
   std::string msg;
   int st = create_problem(family, degree, nv, nt, cells, rule, qdeg, FFG_BOUNDARY_NONE, nullptr, P,
-                          msg);
+                          msg, kUseAdjoint);
   if (st) { *status = st; return; }
   const Topology &t = P->topo;
   if (nnz != t.nnz()) { *status = FFG_INVALID_INPUT; return; }
   double *vb = nullptr, *dvbar = nullptr, *coef = nullptr;
   const size_t vcount = 3 * (size_t)nv;
-  if ((st = dalloc(&vb, (size_t)std::max<int64_t>(nnz, 1))) || (st = dalloc(&dvbar, vcount)) ||
-      (st = dalloc(&coef, 2))) {
-    for (double *p : {vb, dvbar, coef})
-      if (p) cudaFree(p);
+  if ((st = arena_alloc(*P, &vb, (size_t)nnz)) || (st = arena_alloc(*P, &dvbar, vcount)) ||
+      (st = arena_alloc(*P, &coef, 2))) {
     *status = st;
     return;
   }
@@ -1599,9 +1659,9 @@ static void adjoint_csc(int family, int degree, int nv, const double *verts, int
   } else {
     st = family == FFG_TETRA_LAGRANGE
              ? lagrange_vjp(t, P->dt, P->csc_col_ptr, P->csc_row, P->in_vertices, vb, ca, cb,
-                            dvbar, coef, P->err, 0)
+                            dvbar, coef, P->err, 0, P->scratch)
              : nedelec_vjp(t, P->tab, P->dt, P->csc_col_ptr, P->csc_row, P->in_vertices, vb, ca,
-                           cb, P->elem, dvbar, coef, P->err, 0);
+                           cb, P->elem, dvbar, coef, P->err, 0, P->scratch);
     if (!st) {
       if (cudaMemcpy(&herr, P->err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
         st = FFG_CUDA_ERROR;
@@ -1613,7 +1673,6 @@ static void adjoint_csc(int family, int degree, int nv, const double *verts, int
         st = FFG_CUDA_ERROR;
     }
   }
-  for (double *p : {vb, dvbar, coef}) cudaFree(p);
   if (st) {
     std::memset(verts_bar, 0, sizeof(double) * vcount);
     *status = st;

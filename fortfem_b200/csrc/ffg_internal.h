@@ -49,8 +49,43 @@ struct Topology {
   std::vector<uint8_t> inc_local;
   std::vector<uint16_t> slot;        // inc_count * nb
   int max_column = 0;
-  int64_t n_free() const { return (int64_t)free_dofs.size(); }
-  int64_t nnz() const { return (int64_t)row_idx.size(); }
+  // Sizes of a topology whose lists stay on the device (ProblemUse); -1: the
+  // sizes of the lists above.
+  int64_t device_free = -1, device_nnz = -1;
+  int64_t n_free() const { return device_free >= 0 ? device_free : (int64_t)free_dofs.size(); }
+  int64_t nnz() const { return device_nnz >= 0 ? device_nnz : (int64_t)row_idx.size(); }
+};
+
+// What a problem is built for: everything a solve needs; one assembly into the
+// CSC (no solver operator, no work vectors, no host copies of the topology);
+// one adjoint of the CSC (besides, no incidences and slots).
+enum ProblemUse { kUseSolve, kUseCsc, kUseAdjoint };
+
+// Device memory handed out from a few large allocations and returned all at
+// once, or down to a mark.  A chunk never moves.  For one thread and for work
+// on one stream.
+class DeviceArena {
+ public:
+  struct Mark {
+    size_t chunk, used;
+  };
+  DeviceArena() = default;
+  DeviceArena(const DeviceArena &) = delete;
+  DeviceArena &operator=(const DeviceArena &) = delete;
+  ~DeviceArena();
+  void *take(size_t bytes);  // 256-byte aligned; nullptr: out of memory
+  void expect(size_t bytes) { expect_ = bytes; }  // how much the next chunk should hold
+  Mark mark() const { return {at_, at_ < chunks_.size() ? chunks_[at_].used : 0}; }
+  void release(const Mark &m);
+
+ private:
+  struct Chunk {
+    unsigned char *p;
+    size_t size, used;
+  };
+  std::vector<Chunk> chunks_;
+  size_t at_ = 0;  // the chunk being handed out; those behind it are unused
+  size_t expect_ = 0;
 };
 
 // Edge signs (6) and face permutation indices (4) of a Nedelec cell from its
@@ -278,10 +313,14 @@ int ort_class(const int *v);
 // Lagrange / P1 topology built on the device (topology_gpu.cu): the arrays of
 // build_dofs + build_constraints + build_pattern + build_sell, equal entry for
 // entry, written straight into the device structures; the host Topology gets
-// gd, constrained, free_dofs, col_ptr, row_idx, n_dofs and max_column.
+// gd, constrained, free_dofs, col_ptr, row_idx, n_dofs and max_column.  For
+// kUseCsc and kUseAdjoint the device structures that the use has no need of
+// stay empty, those made are `keep`'s, the build's scratch is taken from
+// `scratch` and given back to it, and the host gets the sizes alone.
 int build_topology_device(Topology &t, int boundary_mode, const uint8_t *mask, int grid,
                           DeviceTopology &dt, int64_t **csc_col_ptr, int **csc_row,
-                          DeviceSell &S, std::string &msg);
+                          DeviceSell &S, std::string &msg, ProblemUse use = kUseSolve,
+                          DeviceArena *keep = nullptr, DeviceArena *scratch = nullptr);
 
 // Launch shapes chosen by the autotuner (ffg_problem_autotune); zero fields
 // keep the built-in defaults.
@@ -412,14 +451,16 @@ int launch_lagrange_geometry_jvp(const Topology &t, const DeviceTopology &dt,
                                  int *err, cudaStream_t s);
 int lagrange_vjp(const Topology &t, const DeviceTopology &dt, const int64_t *col_ptr,
                  const int *row_idx, const double *vertices, const double *values_bar, double ca,
-                 double cb, double *vertices_bar, double *coef_bar, int *err, cudaStream_t s);
+                 double cb, double *vertices_bar, double *coef_bar, int *err, cudaStream_t s,
+                 DeviceArena &scratch);
 // Reverse mode of the Nedelec curl + mass assembly, same outputs; `elem`
 // (n_cells * nb * nb) is the work space of orders whose element matrix does
 // not fit in shared memory.
 int nedelec_vjp(const Topology &t, const ElementTables &tab, const DeviceTopology &dt,
                 const int64_t *col_ptr, const int *row_idx, const double *vertices,
                 const double *values_bar, double ca, double cb, double *elem,
-                double *vertices_bar, double *coef_bar, int *err, cudaStream_t s);
+                double *vertices_bar, double *coef_bar, int *err, cudaStream_t s,
+                DeviceArena &scratch);
 
 // ------------------------------------------------------------ complex PML
 // The twelve Nedelec contraction weights of the complex PML forms per cell,

@@ -414,11 +414,9 @@ inline int blocks_for(int64_t n, int t) { return (int)((n + t - 1) / t); }
 
 struct Scratch {
   void *p = nullptr;
-  ~Scratch() {
-    if (p) cudaFree(p);
-  }
-  int alloc(size_t bytes) {
-    return cudaMalloc(&p, std::max<size_t>(bytes, 16)) == cudaSuccess ? FFG_OK : FFG_OUT_OF_MEMORY;
+  int alloc(DeviceArena &arena, size_t bytes) {
+    p = arena.take(bytes);
+    return p ? FFG_OK : FFG_OUT_OF_MEMORY;
   }
 };
 
@@ -439,13 +437,15 @@ namespace {
 
 // Scratch of the reverse mode: per-cell adjoints and the sorted incidences.
 struct VjpScratch {
+  DeviceArena &arena;
   Scratch cell_bar, keys, inc, inc_in, temp;
+  explicit VjpScratch(DeviceArena &a) : arena(a) {}
   int alloc(int64_t nc) {
     int st;
-    if ((st = cell_bar.alloc(sizeof(double) * kCellBar * nc))) return st;
-    if ((st = keys.alloc(sizeof(int) * 4 * nc))) return st;
-    if ((st = inc.alloc(sizeof(int) * 4 * nc))) return st;
-    return inc_in.alloc(sizeof(int) * 4 * nc);
+    if ((st = cell_bar.alloc(arena, sizeof(double) * kCellBar * nc))) return st;
+    if ((st = keys.alloc(arena, sizeof(int) * 4 * nc))) return st;
+    if ((st = inc.alloc(arena, sizeof(int) * 4 * nc))) return st;
+    return inc_in.alloc(arena, sizeof(int) * 4 * nc);
   }
 };
 
@@ -462,7 +462,7 @@ int finish_vjp(const Topology &t, const DeviceTopology &dt, VjpScratch &w, doubl
                                       s) != cudaSuccess)
     return FFG_CUDA_ERROR;
   int st;
-  if ((st = w.temp.alloc(temp_bytes))) return st;
+  if ((st = w.temp.alloc(w.arena, temp_bytes))) return st;
   if (cub::DeviceRadixSort::SortPairs(w.temp.p, temp_bytes, dt.cells, (int *)w.keys.p,
                                       (const int *)w.inc_in.p, (int *)w.inc.p, n_inc, 0, end_bit,
                                       s) != cudaSuccess)
@@ -480,9 +480,10 @@ int finish_vjp(const Topology &t, const DeviceTopology &dt, VjpScratch &w, doubl
 
 int lagrange_vjp(const Topology &t, const DeviceTopology &dt, const int64_t *col_ptr,
                  const int *row_idx, const double *vertices, const double *values_bar, double ca,
-                 double cb, double *vertices_bar, double *coef_bar, int *err, cudaStream_t s) {
+                 double cb, double *vertices_bar, double *coef_bar, int *err, cudaStream_t s,
+                 DeviceArena &scratch) {
   if (t.family != FFG_TETRA_LAGRANGE) return FFG_INVALID_INPUT;
-  VjpScratch w;
+  VjpScratch w(scratch);
   int st;
   if ((st = w.alloc(t.n_cells))) return st;
   const int warps_per_block = 8;
@@ -496,7 +497,8 @@ int lagrange_vjp(const Topology &t, const DeviceTopology &dt, const int64_t *col
 int nedelec_vjp(const Topology &t, const ElementTables &tab, const DeviceTopology &dt,
                 const int64_t *col_ptr, const int *row_idx, const double *vertices,
                 const double *values_bar, double ca, double cb, double *elem,
-                double *vertices_bar, double *coef_bar, int *err, cudaStream_t s) {
+                double *vertices_bar, double *coef_bar, int *err, cudaStream_t s,
+                DeviceArena &scratch) {
   if (t.family != FFG_TETRA_NEDELEC || tab.n_terms != 12) return FFG_INVALID_INPUT;
   NedVjpDims D;
   D.k = t.degree;
@@ -514,7 +516,7 @@ int nedelec_vjp(const Topology &t, const ElementTables &tab, const DeviceTopolog
       cudaFuncSetAttribute(nedelec_cell_vjp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem) != cudaSuccess)
     return FFG_CUDA_ERROR;
-  VjpScratch w;
+  VjpScratch w(scratch);
   int st;
   if ((st = w.alloc(t.n_cells))) return st;
   int dev = 0, sms = 148;

@@ -26,34 +26,55 @@ constexpr int kT = 256;
 constexpr int kMaxLocalDofs = 216;  // Nedelec order 6 (Lagrange degree 4: 35)
 inline unsigned nblk(int64_t n) { return (unsigned)((n + kT - 1) / kT); }
 
-// Device buffer that frees itself.
+// Device memory of one build: `scratch` for what the build alone needs (given
+// back at the end of a Scope, at the latest with the build) and the arena of
+// the arrays that stay, if the caller keeps them in one.  An allocation and
+// its synchronising free cost 0.1 to 0.6 ms here, eighty of them per build
+// several times its kernels.
+struct Temp {
+  DeviceArena own, *scratch, *keep;
+  Temp(DeviceArena *scratch_, DeviceArena *keep_)
+      : scratch(scratch_ ? scratch_ : &own), keep(keep_) {}
+  struct Scope {
+    DeviceArena &a;
+    DeviceArena::Mark m;
+    explicit Scope(Temp &t) : a(*t.scratch), m(a.mark()) {}
+    ~Scope() { a.release(m); }
+  };
+};
+
+// Scratch of the build.
 template <class T>
 struct Buf {
   T *p = nullptr;
-  Buf() = default;
-  Buf(const Buf &) = delete;
-  ~Buf() {
-    if (p) cudaFree(p);
+  bool alloc(size_t n, Temp &t) {
+    p = (T *)t.scratch->take(sizeof(T) * std::max<size_t>(n, 1));
+    return p != nullptr;
   }
-  bool alloc(size_t n) {
-    if (p) cudaFree(p);
-    p = nullptr;
-    return cudaMalloc((void **)&p, sizeof(T) * std::max<size_t>(n, 1)) == cudaSuccess;
+};
+
+// An array that stays: the caller's arena's, or its own and freed unless
+// released.
+template <class T>
+struct Own {
+  T *p = nullptr;
+  bool owned = false;
+  Own() = default;
+  Own(const Own &) = delete;
+  ~Own() {
+    if (p && owned) cudaFree(p);
+  }
+  bool alloc(size_t n, Temp &t) {
+    const size_t bytes = sizeof(T) * std::max<size_t>(n, 1);
+    owned = t.keep == nullptr;
+    if (!owned) p = (T *)t.keep->take(bytes);
+    else if (cudaMalloc((void **)&p, bytes) != cudaSuccess) p = nullptr;
+    return p != nullptr;
   }
   T *release() {
     T *q = p;
     p = nullptr;
     return q;
-  }
-};
-
-struct Temp {
-  Buf<unsigned char> b;
-  size_t bytes = 0;
-  bool ensure(size_t n) {
-    if (n <= bytes) return true;
-    bytes = n;
-    return b.alloc(n);
   }
 };
 
@@ -66,7 +87,7 @@ struct Temp {
   } while (0)
 #define FFG_ALLOC(buf, n)                                      \
   do {                                                         \
-    if (!(buf).alloc(n)) {                                     \
+    if (!(buf).alloc(n, tmp)) {                                     \
       cudaGetLastError();                                      \
       return FFG_OUT_OF_MEMORY;                                \
     }                                                          \
@@ -77,8 +98,10 @@ int sort_pairs(Temp &tmp, const uint64_t *kin, uint64_t *kout, const int *vin, i
                int end_bit = 64) {
   size_t need = 0;
   FFG_TRY(cub::DeviceRadixSort::SortPairs(nullptr, need, kin, kout, vin, vout, n, 0, end_bit));
-  if (!tmp.ensure(need)) return FFG_OUT_OF_MEMORY;
-  FFG_TRY(cub::DeviceRadixSort::SortPairs(tmp.b.p, need, kin, kout, vin, vout, n, 0, end_bit));
+  Temp::Scope cub_scope(tmp);
+  void *cub_temp = tmp.scratch->take(need);
+  if (!cub_temp) return FFG_OUT_OF_MEMORY;
+  FFG_TRY(cub::DeviceRadixSort::SortPairs(cub_temp, need, kin, kout, vin, vout, n, 0, end_bit));
   return FFG_OK;
 }
 
@@ -86,8 +109,10 @@ template <class T>
 int exclusive_sum(Temp &tmp, const T *in, T *out, int n) {
   size_t need = 0;
   FFG_TRY(cub::DeviceScan::ExclusiveSum(nullptr, need, in, out, n));
-  if (!tmp.ensure(need)) return FFG_OUT_OF_MEMORY;
-  FFG_TRY(cub::DeviceScan::ExclusiveSum(tmp.b.p, need, in, out, n));
+  Temp::Scope cub_scope(tmp);
+  void *cub_temp = tmp.scratch->take(need);
+  if (!cub_temp) return FFG_OUT_OF_MEMORY;
+  FFG_TRY(cub::DeviceScan::ExclusiveSum(cub_temp, need, in, out, n));
   return FFG_OK;
 }
 
@@ -98,8 +123,32 @@ struct MaxOp {
 int inclusive_max(Temp &tmp, const int *in, int *out, int n) {
   size_t need = 0;
   FFG_TRY(cub::DeviceScan::InclusiveScan(nullptr, need, in, out, MaxOp(), n));
-  if (!tmp.ensure(need)) return FFG_OUT_OF_MEMORY;
-  FFG_TRY(cub::DeviceScan::InclusiveScan(tmp.b.p, need, in, out, MaxOp(), n));
+  Temp::Scope cub_scope(tmp);
+  void *cub_temp = tmp.scratch->take(need);
+  if (!cub_temp) return FFG_OUT_OF_MEMORY;
+  FFG_TRY(cub::DeviceScan::InclusiveScan(cub_temp, need, in, out, MaxOp(), n));
+  return FFG_OK;
+}
+
+int sort_keys(Temp &tmp, const uint64_t *in, uint64_t *out, int n) {
+  size_t need = 0;
+  FFG_TRY(cub::DeviceRadixSort::SortKeys(nullptr, need, in, out, n));
+  Temp::Scope cub_scope(tmp);
+  void *cub_temp = tmp.scratch->take(need);
+  if (!cub_temp) return FFG_OUT_OF_MEMORY;
+  FFG_TRY(cub::DeviceRadixSort::SortKeys(cub_temp, need, in, out, n));
+  return FFG_OK;
+}
+
+// op over in[0..n) from `init` into *out (device)
+template <class Op>
+int reduce_to(Temp &tmp, const int *in, int *out, int n, Op op, int init) {
+  size_t need = 0;
+  FFG_TRY(cub::DeviceReduce::Reduce(nullptr, need, in, out, n, op, init));
+  Temp::Scope cub_scope(tmp);
+  void *cub_temp = tmp.scratch->take(need);
+  if (!cub_temp) return FFG_OUT_OF_MEMORY;
+  FFG_TRY(cub::DeviceReduce::Reduce(cub_temp, need, in, out, n, op, init));
   return FFG_OK;
 }
 
@@ -517,9 +566,44 @@ __global__ void sell_fill_kernel(int64_t n, int64_t n_slices, const int64_t *sof
 
 }  // namespace
 
+DeviceArena::~DeviceArena() {
+  for (const Chunk &c : chunks_) cudaFree(c.p);
+}
+
+void *DeviceArena::take(size_t bytes) {
+  constexpr size_t kChunk = (size_t)8 << 20;
+  bytes = (bytes + 255) / 256 * 256;
+  for (; at_ < chunks_.size(); ++at_) {
+    Chunk &c = chunks_[at_];
+    if (c.size - c.used >= bytes) {
+      c.used += bytes;
+      return c.p + c.used - bytes;
+    }
+    if (at_ + 1 < chunks_.size()) chunks_[at_ + 1].used = 0;
+  }
+  for (const size_t want : {std::max({bytes, kChunk, expect_}), bytes}) {
+    unsigned char *p = nullptr;
+    if (cudaMalloc((void **)&p, want) == cudaSuccess) {
+      chunks_.push_back({p, want, bytes});
+      expect_ = 0;
+      at_ = chunks_.size() - 1;
+      return p;
+    }
+    cudaGetLastError();
+  }
+  at_ = chunks_.empty() ? 0 : chunks_.size() - 1;
+  return nullptr;
+}
+
+void DeviceArena::release(const Mark &m) {
+  at_ = m.chunk;
+  if (at_ < chunks_.size()) chunks_[at_].used = m.used;
+}
+
 int build_topology_device(Topology &t, int mode, const uint8_t *mask, int grid,
                           DeviceTopology &dt, int64_t **csc_col_ptr, int **csc_row,
-                          DeviceSell &S, std::string &msg) {
+                          DeviceSell &S, std::string &msg, ProblemUse use, DeviceArena *keep,
+                          DeviceArena *scratch) {
   const bool p1 = t.family == FFG_TRIANGLE_P1;
   const bool ned = t.family == FFG_TETRA_NEDELEC;
   if (!p1 && !ned && t.family != FFG_TETRA_LAGRANGE) {
@@ -543,8 +627,13 @@ int build_topology_device(Topology &t, int mode, const uint8_t *mask, int grid,
   const int nb = t.nb;
   const int64_t nl = (int64_t)nc * nb;
   if (nl >= (int64_t)1 << 31) { msg = "mesh too large for the device topology"; return FFG_INVALID_INPUT; }
-  Temp tmp;
-  Buf<int> cells, d_idx, gd;
+  Temp tmp(scratch, keep);
+  // the pattern's keys, their sorted copy and the sort's own, and the lists of
+  // the numbering
+  Temp::Scope build_scope(tmp);
+  tmp.scratch->expect((size_t)nl * ((size_t)24 * nb + 80) + ((size_t)4 << 20));
+  Buf<int> d_idx;
+  Own<int> cells, gd;
   FFG_ALLOC(cells, (size_t)t.vpc * nc);
   FFG_TRY(cudaMemcpy(cells.p, t.cells.data(), sizeof(int) * t.cells.size(), cudaMemcpyHostToDevice));
   FFG_ALLOC(gd, (size_t)nl);
@@ -552,8 +641,8 @@ int build_topology_device(Topology &t, int mode, const uint8_t *mask, int grid,
   // Nedelec face keys stay for the boundary faces
   Buf<uint64_t> nfa, nfb_sorted;
   Buf<int> nford;
-  Buf<int8_t> esign;
-  Buf<uint8_t> fperm;
+  Own<int8_t> esign;
+  Own<uint8_t> fperm;
   // ---- DoF numbering
   if (p1) {
     FFG_TRY(cudaMemcpy(gd.p, cells.p, sizeof(int) * nl, cudaMemcpyDeviceToDevice));
@@ -561,6 +650,8 @@ int build_topology_device(Topology &t, int mode, const uint8_t *mask, int grid,
   } else if (ned) {
     const int k = t.degree, fdc = k * (k - 1), cdc = k * (k - 1) * (k - 2) / 2;
     const int64_t nle = 6 * (int64_t)nc, nlf = 4 * (int64_t)nc;
+    FFG_ALLOC(nfa, nlf); FFG_ALLOC(nfb_sorted, nlf); FFG_ALLOC(nford, nlf);
+    Temp::Scope scope(tmp);
     // edges by first appearance
     Buf<uint64_t> ek, eks;
     Buf<int> epos, eord, est, erun, efirst, eflag, eid;
@@ -581,8 +672,8 @@ int build_topology_device(Topology &t, int mode, const uint8_t *mask, int grid,
     // faces by first appearance
     Buf<uint64_t> fkb, fk1;
     Buf<int> fpos, fo1, fst, frun, ffirst, fflag2, fid;
-    FFG_ALLOC(nfa, nlf); FFG_ALLOC(fkb, nlf); FFG_ALLOC(fk1, nlf); FFG_ALLOC(nfb_sorted, nlf);
-    FFG_ALLOC(fpos, nlf); FFG_ALLOC(fo1, nlf); FFG_ALLOC(nford, nlf); FFG_ALLOC(fperm, nlf);
+    FFG_ALLOC(fkb, nlf); FFG_ALLOC(fk1, nlf);
+    FFG_ALLOC(fpos, nlf); FFG_ALLOC(fo1, nlf); FFG_ALLOC(fperm, nlf);
     ned_face_keys_kernel<<<nblk(nlf), kT>>>(nc, cells.p, nfa.p, fkb.p, fpos.p, fperm.p);
     if ((st = sort_pairs(tmp, nfa.p, fk1.p, fpos.p, fo1.p, (int)nlf))) return st;
     gather_u64_kernel<<<nblk(nlf), kT>>>(nlf, fkb.p, fo1.p, fk1.p);
@@ -607,6 +698,7 @@ int build_topology_device(Topology &t, int mode, const uint8_t *mask, int grid,
   } else {
     FFG_ALLOC(d_idx, idx.size());
     FFG_TRY(cudaMemcpy(d_idx.p, idx.data(), sizeof(int) * idx.size(), cudaMemcpyHostToDevice));
+    Temp::Scope scope(tmp);
     Buf<uint64_t> ka, kb, k1, k2;
     Buf<int> pos, o1, o2, runst, run, first, flag, id;
     FFG_ALLOC(ka, nl); FFG_ALLOC(kb, nl); FFG_ALLOC(k1, nl); FFG_ALLOC(k2, nl);
@@ -634,6 +726,7 @@ int build_topology_device(Topology &t, int mode, const uint8_t *mask, int grid,
   FFG_TRY(cudaMemset(con.p, 0, (size_t)N));
   if (mode == FFG_BOUNDARY_MASK) {
     if (!mask) { msg = "boundary mask missing"; return FFG_INVALID_INPUT; }
+    Temp::Scope scope(tmp);
     Buf<uint8_t> m;
     FFG_ALLOC(m, (size_t)N);
     FFG_TRY(cudaMemcpy(m.p, mask, (size_t)N, cudaMemcpyHostToDevice));
@@ -644,6 +737,7 @@ int build_topology_device(Topology &t, int mode, const uint8_t *mask, int grid,
                                                         nford.p, t.degree, gd.p, con.p);
     } else if (p1) {
       const int64_t ne = 3 * (int64_t)nc;
+      Temp::Scope scope(tmp);
       Buf<uint64_t> k, ks;
       Buf<int> v, vs;
       FFG_ALLOC(k, ne); FFG_ALLOC(ks, ne); FFG_ALLOC(v, ne); FFG_ALLOC(vs, ne);
@@ -652,6 +746,7 @@ int build_topology_device(Topology &t, int mode, const uint8_t *mask, int grid,
       p1_boundary_kernel<<<nblk(ne), kT>>>(ne, ks.p, con.p);
     } else {
       const int64_t nf = 4 * (int64_t)nc;
+      Temp::Scope scope(tmp);
       Buf<uint64_t> ka, kb, k1, k2;
       Buf<int> v, o1, o2;
       FFG_ALLOC(ka, nf); FFG_ALLOC(kb, nf); FFG_ALLOC(k1, nf); FFG_ALLOC(k2, nf);
@@ -667,7 +762,8 @@ int build_topology_device(Topology &t, int mode, const uint8_t *mask, int grid,
     return FFG_INVALID_INPUT;
   }
   // ---- free numbering
-  Buf<int> fflag, fi, free_index, free_dofs;
+  Buf<int> fflag, fi, free_dofs;
+  Own<int> free_index;
   FFG_ALLOC(fflag, N); FFG_ALLOC(fi, N); FFG_ALLOC(free_index, N);
   free_flag_kernel<<<nblk(N), kT>>>(N, con.p, fflag.p);
   if ((st = exclusive_sum(tmp, fflag.p, fi.p, (int)N))) return st;
@@ -678,24 +774,29 @@ int build_topology_device(Topology &t, int mode, const uint8_t *mask, int grid,
   free_index_kernel<<<nblk(N), kT>>>(N, con.p, fi.p, free_index.p, free_dofs.p);
   if (F == 0) { msg = "device topology: no free DoFs"; return FFG_INVALID_INPUT; }
   // ---- incidences (free column, cell ascending)
-  Buf<int> iflag, iat;
-  FFG_ALLOC(iflag, nl); FFG_ALLOC(iat, nl);
-  inc_flag_kernel<<<nblk(nl), kT>>>(nl, gd.p, free_index.p, iflag.p);
-  if ((st = exclusive_sum(tmp, iflag.p, iat.p, (int)nl))) return st;
-  int n_inc = 0, lasti = 0;
-  if ((st = read1(iat.p + nl - 1, n_inc)) || (st = read1(iflag.p + nl - 1, lasti))) return st;
-  n_inc += lasti;
-  Buf<uint64_t> ik, iks;
-  Buf<int> iv, ivs, inc_cell, inc_col;
-  Buf<uint8_t> inc_local;
-  Buf<int64_t> inc_ptr;
-  FFG_ALLOC(ik, n_inc); FFG_ALLOC(iks, n_inc); FFG_ALLOC(iv, n_inc); FFG_ALLOC(ivs, n_inc);
-  inc_pairs_kernel<<<nblk(nl), kT>>>(nl, nb, gd.p, free_index.p, iat.p, ik.p, iv.p);
-  if ((st = sort_pairs(tmp, ik.p, iks.p, iv.p, ivs.p, n_inc))) return st;
-  FFG_ALLOC(inc_cell, n_inc); FFG_ALLOC(inc_col, n_inc); FFG_ALLOC(inc_local, n_inc);
-  FFG_ALLOC(inc_ptr, (size_t)F + 1);
-  inc_unpack_kernel<<<nblk(n_inc), kT>>>(n_inc, iks.p, ivs.p, inc_cell.p, inc_local.p, inc_col.p,
-                                         inc_ptr.p);
+  Own<int> inc_cell;
+  Buf<int> inc_col;
+  Own<uint8_t> inc_local;
+  Own<int64_t> inc_ptr;
+  int n_inc = 0;
+  if (use != kUseAdjoint) {
+    Buf<int> iflag, iat;
+    FFG_ALLOC(iflag, nl); FFG_ALLOC(iat, nl);
+    inc_flag_kernel<<<nblk(nl), kT>>>(nl, gd.p, free_index.p, iflag.p);
+    if ((st = exclusive_sum(tmp, iflag.p, iat.p, (int)nl))) return st;
+    int lasti = 0;
+    if ((st = read1(iat.p + nl - 1, n_inc)) || (st = read1(iflag.p + nl - 1, lasti))) return st;
+    n_inc += lasti;
+    Buf<uint64_t> ik, iks;
+    Buf<int> iv, ivs;
+    FFG_ALLOC(ik, n_inc); FFG_ALLOC(iks, n_inc); FFG_ALLOC(iv, n_inc); FFG_ALLOC(ivs, n_inc);
+    inc_pairs_kernel<<<nblk(nl), kT>>>(nl, nb, gd.p, free_index.p, iat.p, ik.p, iv.p);
+    if ((st = sort_pairs(tmp, ik.p, iks.p, iv.p, ivs.p, n_inc))) return st;
+    FFG_ALLOC(inc_cell, n_inc); FFG_ALLOC(inc_col, n_inc); FFG_ALLOC(inc_local, n_inc);
+    FFG_ALLOC(inc_ptr, (size_t)F + 1);
+    inc_unpack_kernel<<<nblk(n_inc), kT>>>(n_inc, iks.p, ivs.p, inc_cell.p, inc_local.p, inc_col.p,
+                                           inc_ptr.p);
+  }
   // ---- pattern of the constrained system
   Buf<int> ccnt, cat;
   FFG_ALLOC(ccnt, nc); FFG_ALLOC(cat, nc);
@@ -705,27 +806,25 @@ int build_topology_device(Topology &t, int mode, const uint8_t *mask, int grid,
   if ((st = read1(cat.p + nc - 1, npairs)) || (st = read1(ccnt.p + nc - 1, lastc))) return st;
   if ((int64_t)npairs + lastc >= ((int64_t)1 << 31)) { msg = "device topology: too many couplings"; return FFG_INVALID_INPUT; }
   npairs += lastc;
-  Buf<int64_t> col_ptr;
-  Buf<int> row;
+  Own<int64_t> col_ptr;
+  Own<int> row;
   int64_t nnz = 0;
   {
+    Temp::Scope scope(tmp);
     Buf<uint64_t> pk, pks;
     FFG_ALLOC(pk, npairs); FFG_ALLOC(pks, npairs);
     pattern_pairs_kernel<<<nblk(nc), kT>>>(nc, nb, gd.p, free_index.p, cat.p, pk.p);
-    size_t need = 0;
-    FFG_TRY(cub::DeviceRadixSort::SortKeys(nullptr, need, pk.p, pks.p, npairs));
-    if (!tmp.ensure(need)) return FFG_OUT_OF_MEMORY;
-    FFG_TRY(cub::DeviceRadixSort::SortKeys(tmp.b.p, need, pk.p, pks.p, npairs));
-    Buf<int> uf, uat;
-    FFG_ALLOC(uf, npairs); FFG_ALLOC(uat, npairs);
-    unique_flag_kernel<<<nblk(npairs), kT>>>(npairs, pks.p, uf.p);
-    if ((st = exclusive_sum(tmp, uf.p, uat.p, npairs))) return st;
+    if ((st = sort_keys(tmp, pk.p, pks.p, npairs))) return st;
+    // the unsorted keys' memory for the flags and their sums
+    int *uf = (int *)pk.p, *uat = uf + npairs;
+    unique_flag_kernel<<<nblk(npairs), kT>>>(npairs, pks.p, uf);
+    if ((st = exclusive_sum(tmp, uf, uat, npairs))) return st;
     int lastu = 0, lasta = 0;
-    if ((st = read1(uat.p + npairs - 1, lasta)) || (st = read1(uf.p + npairs - 1, lastu))) return st;
+    if ((st = read1(uat + npairs - 1, lasta)) || (st = read1(uf + npairs - 1, lastu))) return st;
     nnz = (int64_t)lasta + lastu;
     FFG_ALLOC(row, nnz);
     FFG_ALLOC(col_ptr, (size_t)F + 1);
-    pattern_unpack_kernel<<<nblk(npairs), kT>>>(npairs, pks.p, uf.p, uat.p, row.p, col_ptr.p);
+    pattern_unpack_kernel<<<nblk(npairs), kT>>>(npairs, pks.p, uf, uat, row.p, col_ptr.p);
   }
   Buf<int> clen;
   FFG_ALLOC(clen, F);
@@ -734,25 +833,43 @@ int build_topology_device(Topology &t, int mode, const uint8_t *mask, int grid,
   {
     Buf<int> mx;
     FFG_ALLOC(mx, 1);
-    size_t need = 0;
-    FFG_TRY(cub::DeviceReduce::Max(nullptr, need, clen.p, mx.p, F));
-    if (!tmp.ensure(need)) return FFG_OUT_OF_MEMORY;
-    FFG_TRY(cub::DeviceReduce::Max(tmp.b.p, need, clen.p, mx.p, F));
+    if ((st = reduce_to(tmp, clen.p, mx.p, F, MaxOp(), 0))) return st;
     if ((st = read1(mx.p, maxc))) return st;
   }
   if (maxc > kMaxColumnLength) { msg = "a CSC column exceeds 65534 entries"; return FFG_INVALID_INPUT; }
   // ---- slot maps
-  Buf<uint16_t> slot;
-  FFG_ALLOC(slot, (size_t)n_inc * nb);
-  slot_kernel<<<nblk((int64_t)n_inc * nb), kT>>>(n_inc, nb, inc_col.p, inc_cell.p, gd.p,
-                                                  free_index.p, col_ptr.p, row.p, slot.p);
+  Own<uint16_t> slot;
+  if (use != kUseAdjoint) {
+    FFG_ALLOC(slot, (size_t)n_inc * nb);
+    slot_kernel<<<nblk((int64_t)n_inc * nb), kT>>>(n_inc, nb, inc_col.p, inc_cell.p, gd.p,
+                                                    free_index.p, col_ptr.p, row.p, slot.p);
+  }
+  if (use != kUseSolve) {
+    FFG_TRY(cudaDeviceSynchronize());
+    t.device_free = F;
+    t.device_nnz = nnz;
+    t.max_column = maxc;
+    dt.cells = cells.release();
+    dt.gd = gd.release();
+    dt.edge_sign = esign.release();
+    dt.face_perm = fperm.release();
+    dt.free_index = free_index.release();
+    dt.inc_ptr = inc_ptr.release();
+    dt.inc_cell = inc_cell.release();
+    dt.inc_local = inc_local.release();
+    dt.slot = slot.release();
+    *csc_col_ptr = col_ptr.release();
+    *csc_row = row.release();
+    return FFG_OK;
+  }
   // ---- SELL-32-sigma layout (build_sell)
   free_sell(S);
   S.n = F;
   S.n_slices = (F + kSliceRows - 1) / kSliceRows;
   S.grid = grid;
-  Buf<int> perm, iperm;
+  Own<int> perm, iperm;
   {
+    Temp::Scope scope(tmp);
     Buf<uint64_t> sk, sks;
     Buf<int> sv;
     FFG_ALLOC(sk, F); FFG_ALLOC(sks, F); FFG_ALLOC(sv, F); FFG_ALLOC(perm, F); FFG_ALLOC(iperm, F);
@@ -760,7 +877,8 @@ int build_topology_device(Topology &t, int mode, const uint8_t *mask, int grid,
     if ((st = sort_pairs(tmp, sk.p, sks.p, sv.p, perm.p, F))) return st;
     iperm_kernel<<<nblk(F), kT>>>(F, perm.p, iperm.p);
   }
-  Buf<int64_t> widths, soff;
+  Buf<int64_t> widths;
+  Own<int64_t> soff;
   FFG_ALLOC(widths, (size_t)S.n_slices + 1); FFG_ALLOC(soff, (size_t)S.n_slices + 1);
   slice_width_kernel<<<nblk(S.n_slices), kT>>>(F, S.n_slices, perm.p, clen.p, widths.p);
   FFG_TRY(cudaMemset(widths.p + S.n_slices, 0, sizeof(int64_t)));
@@ -768,27 +886,23 @@ int build_topology_device(Topology &t, int mode, const uint8_t *mask, int grid,
   if ((st = read1(soff.p + S.n_slices, S.padded))) return st;
   bool narrow;
   {
+    Temp::Scope scope(tmp);
     Buf<int> lo, hi, r;
     FFG_ALLOC(lo, F); FFG_ALLOC(hi, F); FFG_ALLOC(r, 1);
     span_kernel<<<nblk(F), kT>>>(F, col_ptr.p, row.p, iperm.p, lo.p, hi.p);
-    size_t need = 0;
-    FFG_TRY(cub::DeviceReduce::Reduce(nullptr, need, lo.p, r.p, F, MinOp(), 0));
-    if (!tmp.ensure(need)) return FFG_OUT_OF_MEMORY;
-    FFG_TRY(cub::DeviceReduce::Reduce(tmp.b.p, need, lo.p, r.p, F, MinOp(), 0));
+    if ((st = reduce_to(tmp, lo.p, r.p, F, MinOp(), 0))) return st;
     int dmin = 0, dmax = 0;
     if ((st = read1(r.p, dmin))) return st;
-    FFG_TRY(cub::DeviceReduce::Max(nullptr, need, hi.p, r.p, F));
-    if (!tmp.ensure(need)) return FFG_OUT_OF_MEMORY;
-    FFG_TRY(cub::DeviceReduce::Max(tmp.b.p, need, hi.p, r.p, F));
+    if ((st = reduce_to(tmp, hi.p, r.p, F, MaxOp(), 0))) return st;
     if ((st = read1(r.p, dmax))) return st;
     narrow = dmin >= -32768 && dmax <= 32767;
   }
   const size_t P = (size_t)std::max<int64_t>(S.padded, 1);
-  Buf<int16_t> dcol;
-  Buf<int> colw;
-  Buf<double> v64, d64;
-  Buf<float> v32, d32;
-  Buf<int> cta, wsl, wof;
+  Own<int16_t> dcol;
+  Own<int> colw;
+  Own<double> v64, d64;
+  Own<float> v32, d32;
+  Own<int> cta, wsl, wof;
   if (narrow) FFG_ALLOC(dcol, P);
   else FFG_ALLOC(colw, P);
   FFG_ALLOC(v64, P); FFG_ALLOC(v32, P); FFG_ALLOC(d64, F); FFG_ALLOC(d32, F);

@@ -172,3 +172,21 @@ def check(problem, v, ca, cb, cell, src, g, mask, csc, load, tol, rng):
     assert size(y - A @ x) <= tol * size(abs(A) @ abs(x))
     assert size(1.0 / dinv - A.diagonal()) <= tol * size(val)
     assert size(rhs - b) <= tol * (size(load) + size(lifted))
+
+
+@pytest.mark.parametrize("nedelec", [False, True])
+def test_csc_in_one_call_is_the_csc_by_size(nedelec, monkeypatch):
+    from fortfem_b200 import api
+
+    v, t = box(2)
+    def call():
+        if nedelec:
+            return ff.assemble_tetra_nedelec_curl_mass_csc(v, t, 1.7, 0.9, order=2)
+        return ff.assemble_tetra_lagrange_stiffness_csc(v, t, 3, 5, 1.7, 0.9)
+    one, st = call()
+    assert st.code == 0
+    monkeypatch.setattr(api, "_CSC_BOUND_BYTES", 0)
+    two, st = call()
+    assert st.code == 0 and one.nrow == two.nrow and one.ncol == two.ncol
+    for a in ("col_ptr", "row_idx", "val"):
+        assert np.array_equal(getattr(one, a), getattr(two, a))
