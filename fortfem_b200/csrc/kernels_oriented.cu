@@ -229,7 +229,11 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-constexpr int kOrtLfPitch = kOrtTileCells + 2;  // even: 16-byte aligned rows of LF
+// row pitch of LF: the stores of sixteen points (3 rows apart) in distinct
+// banks, the reads of a step's four rows nearly so
+constexpr int kOrtLfPitch = kOrtTileCells + 3;
+
+__host__ __device__ constexpr int ort_split_pitch(int nt) { return 8 * nt + 4; }  // likewise
 
 template <int Q>
 struct OrtLoadSmem {
@@ -247,13 +251,23 @@ __device__ __forceinline__ void dmma_8x8x4(double &d0, double &d1, double a, dou
                : "d"(a), "d"(b));
 }
 
-template <int NT, int Q>
-__global__ void __launch_bounds__(kOrtThreads, 2) ort_load_kernel(const __grid_constant__ OrtArgs A) {
+// Orders whose entries take more than one pass (SPLIT: n_b 140 and 216, even)
+// have a CTA per tile and pass, which stages its own columns of the table rows
+// alone: order 6 on 12^3 (162 tiles, a little over one per SM) 1052 us with one
+// CTA per tile, passes of 12 entry tiles (the last nearly empty) and all columns
+// staged in each, 501 us so.  The FP64 MMA rate allows 0.2 ms; shared-memory
+// reads of both operands take as long, and the stages' barriers separate them.
+template <int NT, int Q, bool SPLIT, int CTAS>
+__global__ void __launch_bounds__(kOrtThreads, CTAS)
+ort_load_kernel(const __grid_constant__ OrtArgs A) {
   extern __shared__ __align__(16) unsigned char ort_raw[];
   OrtLoadSmem<Q> &S = *reinterpret_cast<OrtLoadSmem<Q> *>(ort_raw);
   const int nb = A.nb, nql = A.nql;
   // two buffers of 3 Q table rows (an even count of doubles each)
-  const int rows_cap = (3 * Q * nb + 1) & ~1;
+  constexpr int kSplitPitch = ort_split_pitch(NT);
+  const int pitch = SPLIT ? kSplitPitch : nb;
+  const int rows_cap = (3 * Q * pitch + 1) & ~1;
+  const int base = SPLIT ? 8 * NT * blockIdx.y : 0;
   double *Lb = reinterpret_cast<double *>(ort_raw + sizeof(OrtLoadSmem<Q>));
   constexpr int kPairs = kOrtTileCells * Q / kOrtThreads;  // (cell, point) pairs per thread
   const int4 tile = A.tiles[blockIdx.x];
@@ -281,10 +295,17 @@ __global__ void __launch_bounds__(kOrtThreads, 2) ort_load_kernel(const __grid_c
   auto stage = [&](int ci) {
     if (ci < n_chunks) {
       const int q0 = ci * Q, nq = min(Q, nql - q0);
-      const int pieces = (3 * nq * nb + 1) / 2;
-      const double *src = L + (size_t)3 * q0 * nb;
+      const double *src = L + (size_t)3 * q0 * nb + base;
       double *dst = Lb + (size_t)(ci & 1) * rows_cap;
-      for (int i = tid; i < pieces; i += kOrtThreads) cp_async16(dst + 2 * i, src + 2 * i);
+      if (SPLIT) {
+        for (int i = tid; i < 3 * nq * 4 * NT; i += kOrtThreads) {
+          const int r = i / (4 * NT), c = 2 * (i % (4 * NT));
+          if (base + c < nb) cp_async16(dst + r * kSplitPitch + c, src + (size_t)r * nb + c);
+        }
+      } else {
+        const int pieces = (3 * nq * nb + 1) / 2;
+        for (int i = tid; i < pieces; i += kOrtThreads) cp_async16(dst + 2 * i, src + 2 * i);
+      }
     }
     cp_async_commit();
   };
@@ -303,52 +324,49 @@ __global__ void __launch_bounds__(kOrtThreads, 2) ort_load_kernel(const __grid_c
   // warp w: cells 8w .. 8w+7 (M), NT tiles of 8 entries (N) per pass, 4 table
   // rows (K) per step
   const int kr = lane & 3, cc = lane >> 2;
-  for (int base = 0; base < nb; base += 8 * NT) {
-    double acc[NT][2];
+  double acc[NT][2];
 #pragma unroll
-    for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = 0.0;
-    __syncthreads();  // the previous pass has consumed both buffers
-    stage(0);
-    fetch(0);
-    for (int ci = 0; ci < n_chunks; ++ci) {
-      const int q0 = ci * Q, nq = min(Q, nql - q0);
-      __syncthreads();  // chunk ci - 1 consumed: its buffer and LF may be rewritten
-      stage(ci + 1);
+  for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = 0.0;
+  stage(0);
+  fetch(0);
+  for (int ci = 0; ci < n_chunks; ++ci) {
+    const int q0 = ci * Q, nq = min(Q, nql - q0);
+    __syncthreads();  // chunk ci - 1 consumed: its buffer and LF may be rewritten
+    stage(ci + 1);
 #pragma unroll
-      for (int u = 0; u < kPairs; ++u) {
-        const int p = tid + kOrtThreads * u, c = p / Q, q = p % Q;
-        const double d = S.det[c];
+    for (int u = 0; u < kPairs; ++u) {
+      const int p = tid + kOrtThreads * u, c = p / Q, q = p % Q;
+      const double d = S.det[c];
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
-          S.LF[3 * q + a][c] =
-              d * (S.Ji[a][c] * f[u][0] + S.Ji[a + 3][c] * f[u][1] + S.Ji[a + 6][c] * f[u][2]);
-      }
-      cp_async_wait1();  // this thread's pieces of chunk ci have landed
-      __syncthreads();   // everyone's pieces and factors are visible
-      if (ci + 1 < n_chunks) fetch(q0 + Q);
-      const double *rows = Lb + (size_t)(ci & 1) * rows_cap;
-      const int nk = 3 * nq;
-      for (int k0 = 0; k0 < nk; k0 += 4) {
-        const int qa = k0 + kr;
-        const bool kin = qa < nk;
-        const double av = kin ? S.LF[qa][8 * warp + cc] : 0.0;
-        const double *row = rows + (size_t)(kin ? qa : 0) * nb;
-#pragma unroll
-        for (int t = 0; t < NT; ++t) {
-          const int i = base + 8 * t + cc;
-          const double bv = (kin && i < nb) ? row[i] : 0.0;
-          dmma_8x8x4(acc[t][0], acc[t][1], av, bv);
-        }
-      }
+      for (int a = 0; a < 3; ++a)
+        S.LF[3 * q + a][c] =
+            d * (S.Ji[a][c] * f[u][0] + S.Ji[a + 3][c] * f[u][1] + S.Ji[a + 6][c] * f[u][2]);
     }
-    const int cell = S.cell[8 * warp + cc];
-    if (cell >= 0) {
+    cp_async_wait1();  // this thread's pieces of chunk ci have landed
+    __syncthreads();   // everyone's pieces and factors are visible
+    if (ci + 1 < n_chunks) fetch(q0 + Q);
+    const double *rows = Lb + (size_t)(ci & 1) * rows_cap;
+    const int nk = 3 * nq;
+    for (int k0 = 0; k0 < nk; k0 += 4) {
+      const int qa = k0 + kr;
+      const bool kin = qa < nk;
+      const double av = kin ? S.LF[qa][8 * warp + cc] : 0.0;
+      const double *row = rows + (size_t)(kin ? qa : 0) * pitch;
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
-        const int i = base + 8 * t + 2 * kr;
-        if (i < nb) A.cell_rhs[(size_t)nb * cell + i] = acc[t][0];
-        if (i + 1 < nb) A.cell_rhs[(size_t)nb * cell + i + 1] = acc[t][1];
+        const int i = 8 * t + cc;
+        const double bv = (kin && base + i < nb) ? row[i] : 0.0;
+        dmma_8x8x4(acc[t][0], acc[t][1], av, bv);
       }
+    }
+  }
+  const int cell = S.cell[8 * warp + cc];
+  if (cell >= 0) {
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      const int i = base + 8 * t + 2 * kr;
+      if (i < nb) A.cell_rhs[(size_t)nb * cell + i] = acc[t][0];
+      if (i + 1 < nb) A.cell_rhs[(size_t)nb * cell + i + 1] = acc[t][1];
     }
   }
   cp_async_wait_all();
@@ -551,25 +569,29 @@ int launch_nedelec_oriented(const Topology &t, const OrientedTables &o, const De
   if (!load_only)
     ort_matrix_kernel<<<(unsigned)((int64_t)o.n_tiles * A.parts), kOrtThreads, 0, s>>>(A);
   if (in.samples) {
-    auto go = [&](auto kern, int Q, size_t fixed) -> int {
-      const size_t smem = fixed + 2 * sizeof(double) * (((size_t)3 * Q * o.nb + 1) & ~(size_t)1);
+    const int tiles = load_tiles(o.nb);
+    auto go = [&](auto kern, int Q, size_t fixed, bool split) -> int {
+      const int pitch = split ? ort_split_pitch(tiles) : o.nb;
+      const size_t smem = fixed + 2 * sizeof(double) * (((size_t)3 * Q * pitch + 1) & ~(size_t)1);
       if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
           cudaSuccess)
         return FFG_CUDA_ERROR;
-      kern<<<o.n_tiles, kOrtThreads, smem, s>>>(A);
+      const dim3 grid((unsigned)o.n_tiles, split ? (unsigned)((o.nb + 8 * tiles - 1) / (8 * tiles)) : 1u);
+      kern<<<grid, kOrtThreads, smem, s>>>(A);
       return FFG_OK;
     };
-    // Q = 16 points per stage up to order 4, 8 above (shared memory)
-    const bool wide = o.nb > 84;
+    // Q points per stage and CTAs per SM by timing: order 3 on 24^3 282 us at
+    // (16, 2) and 285 at (8, 3), order 4 on 17 x 16 x 17 223 and 218, order 6
+    // on 12^3 501 and 573
     const size_t f16 = sizeof(OrtLoadSmem<16>), f8 = sizeof(OrtLoadSmem<8>);
     int st;
-    switch (load_tiles(o.nb)) {
-      case 1: st = go(ort_load_kernel<1, 16>, 16, f16); break;
-      case 3: st = go(ort_load_kernel<3, 16>, 16, f16); break;
-      case 6: st = go(ort_load_kernel<6, 16>, 16, f16); break;
-      case 7: st = wide ? go(ort_load_kernel<7, 8>, 8, f8) : go(ort_load_kernel<7, 16>, 16, f16); break;
-      case 11: st = wide ? go(ort_load_kernel<11, 8>, 8, f8) : go(ort_load_kernel<11, 16>, 16, f16); break;
-      default: st = wide ? go(ort_load_kernel<12, 8>, 8, f8) : go(ort_load_kernel<12, 16>, 16, f16); break;
+    switch (tiles) {
+      case 1: st = go(ort_load_kernel<1, 16, false, 2>, 16, f16, false); break;
+      case 3: st = go(ort_load_kernel<3, 16, false, 2>, 16, f16, false); break;
+      case 6: st = go(ort_load_kernel<6, 16, false, 2>, 16, f16, false); break;
+      case 11: st = go(ort_load_kernel<11, 8, false, 3>, 8, f8, false); break;
+      case 9: st = go(ort_load_kernel<9, 16, true, 2>, 16, f16, true); break;
+      default: return FFG_INVALID_INPUT;
     }
     if (st) return st;
   } else if (cudaMemsetAsync(cell_rhs, 0, sizeof(double) * t.nb * (size_t)t.n_cells, s) !=
