@@ -422,15 +422,6 @@ __device__ __forceinline__ SliceRowHead slice_head(const Args &A, int2 rg, int i
   return h;
 }
 
-// Incidence range of every SELL row's column (the slice gather's heads).
-__global__ void inc_range_kernel(int64_t n, const int *perm, const int64_t *inc_ptr,
-                                 int2 *range) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  const int j = perm[r];
-  range[r] = make_int2((int)inc_ptr[j], (int)inc_ptr[j + 1]);
-}
-
 // The load of local DoF l of cell e (as column_body sums it).
 template <int FAMILY, class Args>
 __device__ __forceinline__ double slice_load(const Args &A, int e, int l) {
@@ -927,16 +918,8 @@ int launch_columns(const Topology &t, const ElementTables &tab, const DeviceTopo
                        col_bytes <= kColSmem;
   const int wpb = by_warp ? std::max(1, std::min(8, kColSmem / col_bytes)) : 0;
   // SELL rows by the slice gather
-  const int lanes = sell && sell->perm ? slice_lanes(t.family, t.nb, t.max_column) : 0;
-  // incidence ranges stored as int32 (every incidence index below 2^31)
-  const int64_t n_inc = (int64_t)t.nb * t.n_cells;
-  if (lanes && n_inc < (int64_t)INT32_MAX) {
-    if (!sell->inc_range) {
-      if (cudaMalloc((void **)&sell->inc_range, sizeof(int2) * (size_t)F) != cudaSuccess)
-        return FFG_OUT_OF_MEMORY;
-      inc_range_kernel<<<blocks_for(F, 256), 256, 0, s>>>(F, sell->perm, dt.inc_ptr,
-                                                         sell->inc_range);
-    }
+  const int lanes = sell && sell->inc_range ? slice_lanes(t.family, t.nb, t.max_column) : 0;
+  if (lanes) {
     SliceArgs A;
     A.range = sell->inc_range;
     A.nb = t.nb;

@@ -564,6 +564,15 @@ __global__ void sell_fill_kernel(int64_t n, int64_t n_slices, const int64_t *sof
   }
 }
 
+// Incidence range of every SELL row's column (the slice gather's heads).
+__global__ void inc_range_kernel(int64_t n, const int *perm, const int64_t *inc_ptr,
+                                 int2 *range) {
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= n) return;
+  const int j = perm[r];
+  range[r] = make_int2((int)inc_ptr[j], (int)inc_ptr[j + 1]);
+}
+
 }  // namespace
 
 DeviceArena::~DeviceArena() {
@@ -877,6 +886,9 @@ int build_topology_device(Topology &t, int mode, const uint8_t *mask, int grid,
     if ((st = sort_pairs(tmp, sk.p, sks.p, sv.p, perm.p, F))) return st;
     iperm_kernel<<<nblk(F), kT>>>(F, perm.p, iperm.p);
   }
+  Own<int2> range;  // fewer than 2^31 incidences, as local DoFs
+  FFG_ALLOC(range, F);
+  inc_range_kernel<<<nblk(F), kT>>>(F, perm.p, inc_ptr.p, range.p);
   Buf<int64_t> widths;
   Own<int64_t> soff;
   FFG_ALLOC(widths, (size_t)S.n_slices + 1); FFG_ALLOC(soff, (size_t)S.n_slices + 1);
@@ -962,6 +974,7 @@ int build_topology_device(Topology &t, int mode, const uint8_t *mask, int grid,
   S.dinv64 = d64.release();
   S.dinv32 = d32.release();
   S.perm = perm.release();
+  S.inc_range = range.release();
   S.iperm = iperm.release();
   S.cta_slice = cta.release();
   S.wslice = wsl.release();
