@@ -33,6 +33,7 @@
 #include <climits>
 #include <mutex>
 
+#include "cluster_phase.h"
 #include "pcg_common.cuh"
 
 namespace ffg {
@@ -119,6 +120,8 @@ __device__ __forceinline__ double block_sums(const double (&v)[kVals]) {
 // receiver's mbarrier, which the receiver alone waits for (with its own
 // bound): 1300 cycles for two sums over 8 CTAs of 512 threads, against 1600
 // with plain remote stores and barrier.cluster (16 CTAs: 1450 against 2050).
+// Every phase waits for a message of every CTA, sums or not (cluster_phase.h):
+// the two slot sets and mbarriers are safe to reuse only then.
 template <int NT>
 struct ClusterSync {
   int rank, n;
@@ -138,6 +141,7 @@ struct ClusterSync {
                                        const void *base = nullptr, unsigned slice_bytes = 0) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4, l = lane & 15;
     const unsigned par = ++phase & 1u;
+    constexpr int NM = phase_messages(NV);
     const unsigned mbar = smem_addr(&gSh.mbar[par]);
     // the rows written by ordinary stores are read by the copy engine
     if (base) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -158,9 +162,9 @@ struct ClusterSync {
     if (warp == 0) {
       if (lane == 0)
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar),
-                     "r"(8u * NV * n + (base ? gSh.need * slice_bytes : 0u))
+                     "r"(phase_bytes(NV, n, base ? gSh.need * slice_bytes : 0u))
                      : "memory");
-      if (l < n && half < NV)
+      if (l < n && half < NM)
         asm volatile(
             "st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
                 mapa(smem_addr(&gSh.slot[par][half][rank]), l)),

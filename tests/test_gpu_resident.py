@@ -88,3 +88,28 @@ def test_resident_hard_system_falls_back_like_the_staged_kernel(precision):
     # FP64 rounding of one evaluation of b - A x
     floor = 1e-16 * np.linalg.norm(np.abs(A) @ np.abs(x)) / np.linalg.norm(b)
     assert abs(res - st.true_relative_residual) <= 1e-3 * res + 20 * floor
+
+
+@pytest.mark.parametrize("n", [5, 40, 479, 4096, 6001])
+@pytest.mark.parametrize("block", [1, 4])
+def test_cluster_fp64_without_coupling_between_ctas(n, block):
+    """Operators of which no CTA reads another's rows: the FP64 loop's exchange
+    then copies nothing and is only held together by its messages.  Blocks of 4
+    consecutive rows, so equal rows keep a slice's blocks together."""
+    rng = np.random.default_rng(n + block)
+    blocks = []
+    for k in range(0, n, block):
+        m = min(block, n - k)
+        a = rng.uniform(-1.0, 1.0, (m, m))
+        a = np.triu(a, 1) + np.triu(a, 1).T
+        blocks.append(a + np.diag(2.0 * abs(a).sum(axis=1) + rng.uniform(1.0, 4.0, m)))
+    A = sp.block_diag([sp.coo_matrix(k) for k in blocks]).tocsc()
+    xs = rng.standard_normal(n)
+    b = A @ xs
+    x, st = solve(A, b, "fp64")
+    assert st.converged and st.true_relative_residual <= 1.01 * TOL
+    # |A^-1| <= 1 (diagonal less the rest of the row), |A| <= 13 (diagonal at most
+    # 2 * 3 + 4, the rest 3)
+    assert np.linalg.norm(x - xs) <= 1.01 * 13 * TOL * np.linalg.norm(xs)
+    y, _ = solve(A, b, "fp64")
+    assert np.array_equal(x, y)
