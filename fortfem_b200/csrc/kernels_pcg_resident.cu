@@ -469,6 +469,9 @@ struct Solve {
     return sizeof(V) == 4 ? reinterpret_cast<V *>(gP.zf) : reinterpret_cast<V *>(gP.rd);
   }
   // Row `row` of the published vector, for every CTA to read after exchange().
+  // A replica's rows are the source of the copies of the exchange before: a
+  // phase of sums or a barrier lies between the two, after which every CTA has
+  // received them.
   template <typename V> __device__ __forceinline__ void publish(int row, V v) {
     published<V>()[row] = v;
   }
@@ -907,11 +910,13 @@ struct Solve {
       ++o.updates;
       t0 = stamp();
       fold();
+      // x becomes visible, and the copies of z have landed everywhere
+      if (IDX == kAbs16 && !barrier()) { o.aborted = 1; return; }
       if (!direct) {
         for_rows([&](int li, int row) { publish<float>(row, p[li]); });
         if (IDX == kAbs16 && !exchange<float, 0>(part, red)) { o.aborted = 1; return; }
       }
-      if (!barrier()) { o.aborted = 1; return; }
+      if (IDX != kAbs16 && !barrier()) { o.aborted = 1; return; }
       unfolded = false;
       part[0] = direct ? residual<false>(nullptr) : residual<true>(q);
       if (!S.template sums<1>(part, red)) { o.aborted = 1; return; }
@@ -932,7 +937,10 @@ struct Solve {
         if (!direct) publish<float>(row, zz);
         part[0] += (double)rr2 * (double)zz;
       });
-      if (!exchange<float, 1>(part, red)) { o.aborted = 1; return; }
+      if (!(direct ? S.template sums<1>(part, red) : exchange<float, 1>(part, red))) {
+        o.aborted = 1;
+        return;
+      }
       tm.u += stamp() - t0;
       beta = grew ? 0.0 : red[0] / (rz * ratio);
       rz = red[0];

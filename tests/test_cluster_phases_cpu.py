@@ -3,8 +3,9 @@ mbarriers, slots and messages of kernels_pcg_resident.cu.
 
 The model interleaves the CTAs' steps and the deliveries of their messages in
 every order (two CTAs) or in random ones (four).  A phase's sum must be that of
-the phase's own messages, and no CTA may wait for ever.  The number of messages
-and the bytes that a phase expects come from the kernel's header.
+the phase's own messages, no row is published while a copy of it is under way,
+and no CTA may wait for ever.  The number of messages and the bytes that a
+phase expects come from the kernel's header.
 """
 import ctypes as C
 import os
@@ -27,26 +28,33 @@ def header(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I" + CSRC, str(src), "-o", str(so)],
                    check=True)
     lib = C.CDLL(str(so))
-    return lib.messages, lambda nv, n: lib.bytes(nv, n, C.c_uint(0))
+    return lib.messages, lambda nv, n, copied: lib.bytes(nv, n, C.c_uint(copied))
+
+
+COPY = 128  # bytes of a copied slice
 
 
 class Model:
-    """n CTAs that run the same list of phases (their counts of sums), no copies.
+    """n CTAs that run the same program, a list of
+      S0 S1 S2  a phase of that many sums;
+      X0 X1 X2  the same with the exchange: CTA c copies a slice to CTA c + 1 alone;
+      P         publish: the source of the copies is written;
+      B         the barrier of the cluster.
+    Steps of a phase: send (arrive with the expected bytes, a message to every CTA
+    and the copy), wait, read.  States are plain tuples, so that they can be hashed."""
 
-    Steps of CTA c in phase k: send (arrive with the expected bytes, one message
-    to every CTA), wait, read.  State is a plain tuple so that it can be hashed."""
-
-    def __init__(self, n, phases, messages, bytes_):
-        self.n, self.phases, self.messages, self.bytes = n, phases, messages, bytes_
+    def __init__(self, n, program, messages, bytes_):
+        self.n, self.program = n, program.split()
+        self.messages, self.bytes = messages, bytes_
 
     def start(self):
-        # per CTA: (phase, step), two mbarriers (completed, pending, bytes), two
-        # slot sets of n phases; the messages in flight
-        cta = ((1, 0), ((0, 1, 0), (0, 1, 0)), ((0,) * self.n, (0,) * self.n))
+        # per CTA: (operation, step, phase), two mbarriers (completed, pending,
+        # bytes), two slot sets of n phases; what is in flight
+        cta = ((0, 0, 1), ((0, 1, 0), (0, 1, 0)), ((0,) * self.n, (0,) * self.n))
         return (cta,) * self.n, ()
 
     def done(self, state):
-        return all(c[0][0] > len(self.phases) for c in state[0])
+        return all(c[0][0] == len(self.program) for c in state[0])
 
     @staticmethod
     def _bar(bars, par, arrive, tx):
@@ -62,33 +70,50 @@ class Model:
         """The states that one step of a CTA or one delivery leads to."""
         ctas, flight = state
         for c in range(self.n):
-            (k, step), bars, slots = ctas[c]
-            if k > len(self.phases):
+            (at, step, k), bars, slots = ctas[c]
+            if at == len(self.program):
                 continue
-            par, nv = k % 2, self.phases[k - 1]
-            sent = flight
-            if step == 0:
-                bars = self._bar(bars, par, 1, self.bytes(nv, self.n))
-                sent = flight + tuple((d, c, k) for d in range(self.n)) * self.messages(nv)
+            op, sent, last = self.program[at], flight, False
+            nv, par = int(op[1]) if len(op) > 1 else 0, k % 2
+            if op == "P":
+                assert not any(f[0] == "copy" and f[2] == c for f in flight), \
+                    f"CTA {c} overwrites what is being copied (operation {at})"
+                last = True
+            elif op == "B":
+                # step 0 arrives; the wait ends when all have arrived here or are past it
+                if step == 1:
+                    if any((o[0][0], o[0][1]) < (at, 1) for o in ctas):
+                        continue
+                    last = True
+            elif step == 0:
+                copies = ()
+                if op[0] == "X":
+                    copies = (("copy", (c + 1) % self.n, c, k),)
+                    assert not any(f[:3] == copies[0][:3] for f in flight), \
+                        f"two copies of CTA {c} to one place (operation {at})"
+                bars = self._bar(bars, par, 1, self.bytes(nv, self.n, COPY * len(copies)))
+                sent = flight + copies + tuple(
+                    ("sum", d, c, k) for d in range(self.n)) * self.messages(nv)
             elif step == 1:
                 # try_wait.parity: true while the barrier is in the other parity
                 if bars[par][0] % 2 == ((k - 1) >> 1) % 2:
                     continue
             else:
-                got = slots[par]
-                if nv > 0 and any(g != k for g in got):
-                    raise AssertionError(f"CTA {c} sums {got} in phase {k}")
-            pos = (k, step + 1) if step < 2 else (k + 1, 0)
+                assert nv == 0 or all(g == k for g in slots[par]), \
+                    f"CTA {c} sums {slots[par]} in phase {k}"
+                k, last = k + 1, True
+            pos = (at + 1, 0, k) if last else (at, step + 1, k)
             yield ctas[:c] + ((pos, bars, slots),) + ctas[c + 1:], tuple(sorted(sent))
-        for i, (d, c, k) in enumerate(flight):
+        for i, (kind, d, c, k) in enumerate(flight):
             if i and flight[i - 1] == flight[i]:
                 continue
             pos, bars, slots = ctas[d]
-            row = list(slots[k % 2])
-            row[c] = k
-            slots = (row, slots[1]) if k % 2 == 0 else (slots[0], row)
-            new = (pos, self._bar(bars, k % 2, 0, -8), tuple(map(tuple, slots)))
-            yield ctas[:d] + (new,) + ctas[d + 1:], flight[:i] + flight[i + 1:]
+            if kind == "sum":
+                row = list(slots[k % 2])
+                row[c] = k
+                slots = (tuple(row), slots[1]) if k % 2 == 0 else (slots[0], tuple(row))
+            bars = self._bar(bars, k % 2, 0, -8 if kind == "sum" else -COPY)
+            yield ctas[:d] + ((pos, bars, slots),) + ctas[d + 1:], flight[:i] + flight[i + 1:]
 
     def explore(self):
         todo, seen = [self.start()], set()
@@ -110,25 +135,41 @@ class Model:
             s = rng.choice(after)
 
 
-# sums per phase: the FP64 loop (exchange of p, (p, q), then (r, r) and (r, z)),
-# the mixed loop, and a direct one that looks at the wall limit
-LOOPS = [[2, 1, 0, 1, 2, 0, 1, 2], [2, 1, 1, 2, 1, 2, 0, 1, 1], [1, 2, 1, 0, 1, 2, 1, 0]]
+# The cluster's loops in kernels_pcg_resident.cu, the published vector replicated.
+LOOPS = {
+    # residual norms, (r, z); then two iterations
+    "fp64": "S2 S1 P X0 S1 S2 P X0 S1 S2",
+    "mixed": "S2 P X1 S1 P X2 S1 P X2",
+    # an iteration, its reliable update, the next iteration
+    "update": "P X1 S1 P X2 B P X0 S1 P X1 S1 P X2",
+    # the update that changes to the direct form, an iteration, an update in it
+    "direct": "P X1 S1 P X2 B P X0 S1 S1 P X0 S1 S2 B S1 S1 P X0 S1 S2",
+    # a look at the wall limit between the phases
+    "limit": "P X0 S1 S2 S1 P X0 S1 S2",
+}
 
 
-@pytest.mark.parametrize("phases", LOOPS)
-def test_every_interleaving_of_two_ctas_sums_its_own_phase(header, phases):
-    assert Model(2, phases, *header).explore() > 100
+@pytest.mark.parametrize("loop", LOOPS)
+def test_every_interleaving_of_two_ctas(header, loop):
+    assert Model(2, LOOPS[loop], *header).explore() > 100
 
 
-@pytest.mark.parametrize("phases", LOOPS)
-def test_random_interleavings_of_four_ctas(header, phases):
-    rng = random.Random(len(phases))
+@pytest.mark.parametrize("loop", LOOPS)
+def test_random_interleavings_of_four_ctas(header, loop):
+    rng = random.Random(len(loop))
     for _ in range(60):
-        Model(4, phases, *header).walk(rng)
+        Model(4, LOOPS[loop], *header).walk(rng)
 
 
 def test_the_model_finds_the_phase_that_waits_for_nobody():
     """Without a message in a phase of no sums, a CTA overtakes another by two."""
-    quiet = Model(2, LOOPS[0], lambda nv: nv, lambda nv, n: 8 * nv * n)
-    with pytest.raises(AssertionError):
+    quiet = Model(3, "S2 S0 S1 S2", lambda nv: nv, lambda nv, n, copied: 8 * nv * n + copied)
+    with pytest.raises(AssertionError, match="sums"):
         quiet.explore()
+
+
+@pytest.mark.parametrize("loop", ["S1 P X2 P X0 B S1 P X1 S1 P X2",   # p published at once
+                                  "P X0 S1 P X1 P X0 S1 S2"])         # z copied, then p
+def test_the_model_finds_a_publish_during_the_copies(header, loop):
+    with pytest.raises(AssertionError, match="cop"):
+        Model(2, loop, *header).explore()

@@ -12,7 +12,9 @@ import numpy as np
 import pytest
 import scipy.sparse as sp
 
+import oracle
 import fortfem_b200 as ff
+from fortfem_b200 import _capi as K
 
 pytestmark = pytest.mark.gpu
 TOL = 1e-10
@@ -113,3 +115,62 @@ def test_cluster_fp64_without_coupling_between_ctas(n, block):
     assert np.linalg.norm(x - xs) <= 1.01 * 13 * TOL * np.linalg.norm(xs)
     y, _ = solve(A, b, "fp64")
     assert np.array_equal(x, y)
+
+
+def _hard(family, n, relabel):
+    """A problem whose mixed solve stagnates, its inputs and options: P1 on n^2
+    vertices with log-normal coefficients to the end of FP64's reach, or order-1
+    Nedelec with a small mass."""
+    rng = np.random.default_rng(n)
+    if family == K.FFG_TRIANGLE_P1:
+        v, t = oracle.unit_square_mesh(n)
+        if relabel:
+            new = rng.permutation(len(v))
+            w = np.empty_like(v)
+            w[new] = v
+            v, t = w, new[t].astype(t.dtype)
+        prob = ff.Problem(family, 1, t, len(v))
+        inputs = (v, 1.0, 0.0, np.exp(rng.standard_normal(len(t))), None,
+                  np.sin(3 * prob.sample_points(v)[..., 0]), None)
+        tol = 1e-13
+    else:
+        v, t = oracle.box_mesh([n, n, n])
+        prob = ff.Problem(family, 1, t, len(v))
+        p = prob.sample_points(v)
+        inputs = (v, 1.0, 1e-4, None, None,
+                  np.stack([np.sin(3 * p[..., 1]), np.cos(p[..., 2]), p[..., 0]], -1), None)
+        tol = 1e-10
+    return prob, inputs, ff.SolverOptions(method="pcg", preconditioner="jacobi", tolerance=tol,
+                                          precision="mixed", max_iterations=200000,
+                                          breakdown_guard="spd")
+
+
+@pytest.mark.parametrize("family,n,relabel", [
+    (K.FFG_TETRA_NEDELEC, 8, False),    # both replicas fit a CTA
+    (K.FFG_TETRA_NEDELEC, 16, False),   # FP64's published vector in global memory
+    (K.FFG_TRIANGLE_P1, 160, False),    # the same, 16-bit column differences
+    (K.FFG_TRIANGLE_P1, 190, True),     # the same, int32 columns
+])
+def test_cluster_mixed_solve_continues_in_fp64(family, n, relabel):
+    """Direct form, reliable updates and the FP64 continuation of the cluster
+    kernel: the continuation runs, the reported residual is the solution's, and it
+    meets the tolerance or what FP64 can tell from zero.  Error of b - A x in FP64
+    with m terms a row: (m + 1) u (|A| |x| + |b|); a solve ends when an update of x
+    no longer halves the residual, so at no more than about twice that and the
+    rounding of x itself, u |A| |x|."""
+    prob, inputs, opts = _hard(family, n, relabel)
+    with prob:
+        sol, st = prob.solve(*inputs, opts)
+        assert prob.phase_times()["fp64_continuation"]
+        again, st2 = prob.solve(*inputs, opts)
+        assert np.array_equal(sol, again) and st.iterations == st2.iterations
+        A, rhs, free = prob.reduced_system(*inputs)[:3]
+    M = sp.csc_matrix((A.val, A.row_idx, A.col_ptr), shape=(len(rhs), len(rhs)))
+    x = sol[free]
+    norm = np.linalg.norm(rhs)
+    terms = np.diff(M.indptr).max()
+    level = 1.2e-16 * np.linalg.norm(abs(M) @ abs(x) + abs(rhs)) / norm
+    res = np.linalg.norm(rhs - M @ x) / norm
+    assert abs(res - st.true_relative_residual) <= 2 * (terms + 1) * level
+    assert st.converged or family == K.FFG_TRIANGLE_P1
+    assert res <= max(1.01 * opts.tolerance, 2 * (terms + 2) * level)
