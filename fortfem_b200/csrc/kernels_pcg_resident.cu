@@ -44,6 +44,7 @@ constexpr int kGridThreads = 512;
 constexpr int kMaxCluster = 16;
 constexpr int kBatch = 8;          // columns of a row in flight
 constexpr int kPoolMax = 225 * 1024;
+constexpr unsigned long long kLandNs = 1000000;  // far above a message's time of about 1 us
 
 // Before the grid's first poll of a sync: the polls of 148 CTAs hit the same few
 // L2 lines and slow the messages and the fences they wait for (P1, 85,800
@@ -65,6 +66,7 @@ struct ResShared {
   double red[kVals][16], res[kVals];
   double slot[2][kVals][kMaxCluster];
   unsigned long long mbar[2];
+  unsigned long long mbar_all[2];  // the cluster's barrier
   int ok, items, rows;
   int need;               // slices that arrive in an exchange
   int2 send[kMaxCluster]; // this CTA's slices [x, y) that CTA k reads
@@ -122,15 +124,61 @@ __device__ __forceinline__ double block_sums(const double (&v)[kVals]) {
 // with plain remote stores and barrier.cluster (16 CTAs: 1450 against 2050).
 // Every phase waits for a message of every CTA, sums or not (cluster_phase.h):
 // the two slot sets and mbarriers are safe to reuse only then.
+// Every wait is bounded, so every CTA comes to rendezvous() at the kernel's end,
+// also after it or another one gave up: barrier.cluster has no bound, and a
+// barrier of the solve that used it would pair with the last one of a CTA that
+// gave up, let that CTA leave, and have later sums sent to its shared memory.
 template <int NT>
 struct ClusterSync {
   int rank, n;
-  unsigned phase;
+  unsigned phase, turn;  // turn: barriers so far
 
-  __device__ __forceinline__ void barrier_only() {
+  // At the kernel's start and end alone.
+  __device__ __forceinline__ void rendezvous() {
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+
+  // Warp 0 waits, for kBarrierLimitNs, for the mbarrier's phase of this parity.
+  __device__ __forceinline__ void wait(unsigned mbar, unsigned parity) {
+    unsigned long long t0 = 0;
+    for (unsigned spin = 1;; ++spin) {
+      unsigned done;
+      asm volatile(
+          "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+          " selp.u32 %0, 1, 0, p;\n}"
+          : "=r"(done)
+          : "r"(mbar), "r"(parity)
+          : "memory");
+      if (__all_sync(0xffffffffu, done)) return;
+      if ((spin & 255u) == 0) {
+        if (t0 == 0) t0 = globaltimer();
+        if (__any_sync(0xffffffffu, globaltimer() - t0 > kBarrierLimitNs)) {
+          if ((threadIdx.x & 31) == 0) gSh.ok = 0;
+          return;
+        }
+      }
+    }
+  }
+
+  // All writes of the cluster before it are visible after it.  Two mbarriers in
+  // turn: a CTA arrives again at one of them only after the barrier between,
+  // for which every CTA has finished its wait here.
+  __device__ __forceinline__ bool barrier() {
+    const int lane = threadIdx.x & 31;
+    const unsigned mbar = smem_addr(&gSh.mbar_all[++turn & 1u]);
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      if (lane < n)
+        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(
+                         mapa(mbar, lane))
+                     : "memory");
+      __syncwarp();
+      wait(mbar, ((turn - 1) >> 1) & 1u);
+    }
+    __syncthreads();
+    return gSh.ok != 0;
   }
 
   // sums<NV>, and with `base` the exchange of a replicated vector of
@@ -171,26 +219,8 @@ struct ClusterSync {
             "l"(__double_as_longlong(x)), "r"(mapa(mbar, l))
             : "memory");
       __syncwarp();
-      // bounded wait for everything this phase expects
-      const unsigned parity = ((phase - 1) >> 1) & 1u;
-      unsigned long long t0 = 0;
-      for (unsigned spin = 1;; ++spin) {
-        unsigned done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-            " selp.u32 %0, 1, 0, p;\n}"
-            : "=r"(done)
-            : "r"(mbar), "r"(parity)
-            : "memory");
-        if (__all_sync(0xffffffffu, done)) break;
-        if ((spin & 255u) == 0) {
-          if (t0 == 0) t0 = globaltimer();
-          if (__any_sync(0xffffffffu, globaltimer() - t0 > kBarrierLimitNs)) {
-            if (lane == 0) gSh.ok = 0;
-            break;
-          }
-        }
-      }
+      // for everything this phase expects
+      wait(mbar, ((phase - 1) >> 1) & 1u);
     }
     __syncthreads();
     if (NV > 0) {
@@ -205,7 +235,7 @@ struct ClusterSync {
 
   template <int NV>
   __device__ __forceinline__ bool reduce(const double (&v)[kVals], double (&out)[kVals]) {
-    barrier_only();
+    if (!barrier()) return false;
     return NV > 0 ? sums<NV>(v, out) : true;
   }
 };
@@ -461,7 +491,7 @@ struct Solve {
                      : "memory");
       }
     }
-    S.barrier_only();
+    S.barrier();  // what fails here is seen by the sums that follow
   }
 
   template <typename V> __device__ __forceinline__ V *published() {
@@ -1042,7 +1072,7 @@ struct Solve {
 };
 
 template <class Sync, int IDX, int NT>
-__device__ __noinline__ unsigned run_mixed(Share h, Sync sync, unsigned long long t_start,
+__device__ __noinline__ Sync run_mixed(Share h, Sync sync, unsigned long long t_start,
                                            Outcome &out, Timing &tmo) {
   Solve<Sync, IDX, NT> X;
   X.init(h, sync);
@@ -1051,11 +1081,11 @@ __device__ __noinline__ unsigned run_mixed(Share h, Sync sync, unsigned long lon
   X.mixed(t_start, o, tm);
   out = o;
   tmo = tm;
-  return X.S.phase;
+  return X.S;
 }
 
 template <class Sync, int IDX, int NT>
-__device__ __noinline__ unsigned run_fp64(Share h, Sync sync, unsigned long long t_start,
+__device__ __noinline__ Sync run_fp64(Share h, Sync sync, unsigned long long t_start,
                                           bool continuation, Outcome &out, Timing &tmo) {
   Solve<Sync, IDX, NT> X;
   X.init(h, sync);
@@ -1068,7 +1098,7 @@ __device__ __noinline__ unsigned run_fp64(Share h, Sync sync, unsigned long long
   else X.fp64(t_start, continuation, o, tm);
   out = o;
   tmo = tm;
-  return X.S.phase;
+  return X.S;
 }
 
 // The whole solve of gP by the CTAs of `sync`.  gP.staged: bit 0, the mixed
@@ -1085,13 +1115,13 @@ __device__ __forceinline__ void run_solve(const Share &h, Sync sync) {
     bool done = false;
     if constexpr (kShared) {
       if (gP.staged & 1) {
-        sync.phase = run_mixed<Sync, kAbs16, NT>(h, sync, t_start, o, tm);
+        sync = run_mixed<Sync, kAbs16, NT>(h, sync, t_start, o, tm);
         done = true;
       }
     }
     if (done) {
-    } else if (gP.dcol) sync.phase = run_mixed<Sync, kRel16, NT>(h, sync, t_start, o, tm);
-    else sync.phase = run_mixed<Sync, kAbs32, NT>(h, sync, t_start, o, tm);
+    } else if (gP.dcol) sync = run_mixed<Sync, kRel16, NT>(h, sync, t_start, o, tm);
+    else sync = run_mixed<Sync, kAbs32, NT>(h, sync, t_start, o, tm);
     if (!o.aborted && o.stagnated && !o.converged && o.status == FFG_OK) {
       continued = o.restart ? 2 : 1;
       fp64 = continuation = true;
@@ -1153,17 +1183,23 @@ __global__ void __launch_bounds__(NT, 1) pcg_cluster_kernel(const __grid_constan
   if (threadIdx.x == 0) {
     gP = B.sys[blockIdx.x / size];
     gSh.ok = 1;
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < 2; ++i) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&gSh.mbar[i])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&gSh.mbar_all[i])), "r"(size));
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
   const int C = (int)size, r = (int)rank, s0 = gP.cta_slice[r];
   const Share h{s0, gP.cta_slice[r + 1] - s0, gP.share_slices, kPoolMax, (unsigned)gP.part_bytes};
-  ClusterSync<NT> S{r, C, 0u};
-  S.barrier_only();  // every CTA's mbarriers are ready
+  ClusterSync<NT> S{r, C, 0u, 0u};
+  S.rendezvous();  // every CTA's mbarriers are ready
   run_solve<ClusterSync<NT>, true, NT>(h, S);
-  S.barrier_only();  // no CTA leaves while others may still store into it
+  S.rendezvous();  // no CTA leaves while others may still store into it
+  // A wait that gave up may have left messages under way, all of them sent
+  // before the rendezvous: time for them to land.
+  if (threadIdx.x == 0 && ld_volatile_int(gP.control) != 0)
+    for (const unsigned long long t0 = globaltimer(); globaltimer() - t0 < kLandNs;) __nanosleep(1000);
   // what comes after this launch comes after the launch it overlapped with too
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
