@@ -219,10 +219,10 @@ struct SolveWork {
   float *xf = nullptr;                      // mixed-mode FP32 step of x not yet folded in
   float2 *zpf0 = nullptr, *zpf1 = nullptr;  // mixed-mode (z, p) pairs once q = A p is direct
   unsigned int *barrier = nullptr;
+  double *result = nullptr;  // device statistics block, the control word behind it
   int *control = nullptr;    // [0] error status
-  double *result = nullptr;  // device statistics block
-  double *result_host = nullptr;  // pinned copy of the statistics block
-  int *control_host = nullptr;    // pinned copy of the control word
+  double *result_host = nullptr;  // pinned copies of both
+  int *control_host = nullptr;
   int grid = 0;
   int64_t n = 0;
   // last solve: [0] FP64 continuation taken, then device seconds seen by CTA 0

@@ -1094,6 +1094,7 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_batch_kernel(const __grid_con
     Ps = B.sys[blockIdx.x];
     Ps.cta0 = (int)blockIdx.x;
     Ps.ncta = 1;
+    Ps.control[0] = 0;  // as every launch begins
   }
   __syncthreads();
   pcg_body(Ps);
@@ -1404,16 +1405,13 @@ int solve_work_alloc(SolveWork &w, int64_t n, int grid) {
   A((void **)&w.zpf1, N * sizeof(float2));
   A((void **)&w.partial, partial_bytes(grid));
   A((void **)&w.barrier, 64);
-  A((void **)&w.control, 64);
-  A((void **)&w.result, kResultDoubles * sizeof(double));
-  if (!bad && (cudaMallocHost((void **)&w.result_host, kResultDoubles * sizeof(double)) != cudaSuccess ||
-               cudaMallocHost((void **)&w.control_host, 2 * sizeof(int)) != cudaSuccess))
-    bad = true;
+  A((void **)&w.result, kStateBytes);
+  if (!bad && cudaMallocHost((void **)&w.result_host, kStateBytes) != cudaSuccess) bad = true;
   if (!bad) {
-    std::memset(w.result_host, 0, kResultDoubles * sizeof(double));
-    w.control_host[0] = w.control_host[1] = 0;
-    if (cudaMemset(w.control, 0, 64) != cudaSuccess)
-      bad = true;
+    w.control = reinterpret_cast<int *>(w.result + kResultDoubles);
+    w.control_host = reinterpret_cast<int *>(w.result_host + kResultDoubles);
+    std::memset(w.result_host, 0, kStateBytes);
+    if (cudaMemset(w.result, 0, kStateBytes) != cudaSuccess) bad = true;
   }
   if (bad) {
     solve_work_free(w);
@@ -1425,12 +1423,20 @@ int solve_work_alloc(SolveWork &w, int64_t n, int grid) {
 
 void solve_work_free(SolveWork &w) {
   void *ptrs[] = {w.r64, w.rd, w.qd, w.zpd0, w.zpd1, w.rf, w.zf, w.pf, w.qf, w.xf, w.zpf0, w.zpf1,
-                  w.partial, w.barrier, w.control, w.result};
+                  w.partial, w.barrier, w.result};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (w.result_host) cudaFreeHost(w.result_host);
-  if (w.control_host) cudaFreeHost(w.control_host);
   w = SolveWork();
+}
+
+// The statistics and the control word before a launch and after it.
+static bool clear_state(SolveWork &w, cudaStream_t s) {
+  return cudaMemsetAsync(w.result, 0, kStateBytes, s) == cudaSuccess;
+}
+static bool fetch_state(SolveWork &w, cudaStream_t s) {
+  return cudaMemcpyAsync(w.result_host, w.result, kStateBytes, cudaMemcpyDeviceToHost, s) ==
+         cudaSuccess;
 }
 
 namespace {
@@ -1490,9 +1496,7 @@ int pcg_launch(const DeviceSell &A, const double *b, double *x, const ffg_solver
     return FFG_INVALID_INPUT;
   }
   PcgParams P = make_params(A, b, x, opts, w);
-  if (cudaMemsetAsync(w.control, 0, 64, stream) != cudaSuccess) return FFG_CUDA_ERROR;
-  if (cudaMemsetAsync(w.result, 0, kResultDoubles * sizeof(double), stream) != cudaSuccess)
-    return FFG_CUDA_ERROR;
+  if (!clear_state(w, stream)) return FFG_CUDA_ERROR;
   cudaError_t e;
   const int cluster = pcg_cluster_size(A, opts.precision, false);
   if (cluster) {
@@ -1513,12 +1517,7 @@ int pcg_launch(const DeviceSell &A, const double *b, double *x, const ffg_solver
     cudaGetLastError();
     return FFG_CUDA_ERROR;
   }
-  if (cudaMemcpyAsync(w.result_host, w.result, kResultDoubles * sizeof(double),
-                      cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
-      cudaMemcpyAsync(w.control_host, w.control, 2 * sizeof(int), cudaMemcpyDeviceToHost,
-                      stream) != cudaSuccess)
-    return FFG_CUDA_ERROR;
-  return FFG_OK;
+  return fetch_state(w, stream) ? FFG_OK : FFG_CUDA_ERROR;
 }
 
 int pcg_launch_batch(int count, const DeviceSell *const *A, const double *const *b,
@@ -1541,7 +1540,6 @@ int pcg_launch_batch(int count, const DeviceSell *const *A, const double *const 
   for (int i : order) {
     const PcgParams P = make_params(*A[i], b[i], x[i], opts, *w[i]);
     const int c = pcg_cluster_size(*A[i], opts.precision, true);
-    w[i]->control_host[0] = 0;
     (c == 16 ? clustered[0] : c == 8 ? clustered[1] : single).push_back(P);
   }
   bool overlap = false;
@@ -1571,9 +1569,7 @@ int pcg_launch_batch(int count, const DeviceSell *const *A, const double *const 
     }
   }
   for (int i = 0; i < count; ++i)
-    if (cudaMemcpyAsync(w[i]->result_host, w[i]->result, kResultDoubles * sizeof(double),
-                        cudaMemcpyDeviceToHost, stream) != cudaSuccess)
-      return FFG_CUDA_ERROR;
+    if (!fetch_state(*w[i], stream)) return FFG_CUDA_ERROR;
   return FFG_OK;
 }
 
@@ -1603,14 +1599,11 @@ int pcg_launch_groups(int count, const DeviceSell *const *A, const double *const
   std::stable_sort(order.begin(), order.end(), [&](int i, int j) { return length(i) > length(j); });
   std::vector<char> done((size_t)count, 0);
   for (int i : order) {
-    w[i]->control_host[0] = 0;
     if (!ctas[i]) {
       // no group holds it on chip: the whole device
       if ((st = pcg_launch(*A[i], b[i], x[i], opts, *w[i], stream, msg))) return st;
       done[i] = 1;
-    } else if (cudaMemsetAsync(w[i]->control, 0, 64, stream) != cudaSuccess ||
-               cudaMemsetAsync(w[i]->result, 0, kResultDoubles * sizeof(double), stream) !=
-                   cudaSuccess ||
+    } else if (!clear_state(*w[i], stream) ||
                cudaMemsetAsync(w[i]->partial, 0, pcg_message_bytes(ctas[i]), stream) !=
                    cudaSuccess) {
       return FFG_CUDA_ERROR;
@@ -1639,12 +1632,7 @@ int pcg_launch_groups(int count, const DeviceSell *const *A, const double *const
     }
   }
   for (int k = 0; k < count; ++k)
-    if (ctas[k] && (cudaMemcpyAsync(w[k]->result_host, w[k]->result,
-                                    kResultDoubles * sizeof(double), cudaMemcpyDeviceToHost,
-                                    stream) != cudaSuccess ||
-                    cudaMemcpyAsync(w[k]->control_host, w[k]->control, 2 * sizeof(int),
-                                    cudaMemcpyDeviceToHost, stream) != cudaSuccess))
-      return FFG_CUDA_ERROR;
+    if (ctas[k] && !fetch_state(*w[k], stream)) return FFG_CUDA_ERROR;
   return FFG_OK;
 }
 

@@ -1188,6 +1188,7 @@ __global__ void __launch_bounds__(NT, 1) pcg_cluster_kernel(const __grid_constan
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&gSh.mbar_all[i])), "r"(size));
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (rank == 0) gP.control[0] = 0;  // as every launch begins, before any CTA's first wait
   }
   __syncthreads();
   const int C = (int)size, r = (int)rank, s0 = gP.cta_slice[r];

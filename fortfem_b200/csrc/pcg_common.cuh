@@ -10,6 +10,8 @@
 namespace ffg {
 
 constexpr int kResultDoubles = 16;
+// What a solve reports: its statistics and behind them the control word
+constexpr size_t kStateBytes = kResultDoubles * sizeof(double) + 2 * sizeof(int);
 constexpr int kMinWindow = 256;  // iterations before a plateau forces a reliable update
 constexpr unsigned long long kBarrierLimitNs = 4000000000ull;  // 4 s per barrier wait
 

@@ -1,0 +1,96 @@
+// Cases of test_launch_cpu.py: the library's launch code on fake_cudart.h.
+#include "fake_cudart.h"
+#include "ffg_internal.h"
+
+using namespace ffg;
+
+namespace ffg {
+int launch_nedelec_oriented(const Topology &, const OrientedTables &, const DeviceTopology &,
+                            const AssemblyInputs &, double *, double *, int *, cudaStream_t, bool) {
+  return FFG_OK;
+}
+}  // namespace ffg
+
+namespace {
+
+// `rows` rows of `width` entries, 148 CTAs.
+struct System {
+  DeviceSell A;
+  SolveWork w;
+  std::vector<double> x, b;
+  System(int64_t rows, int width) : x(rows), b(rows) {
+    A.n = rows;
+    A.n_slices = (rows + kSliceRows - 1) / kSliceRows;
+    A.grid = 148;
+    std::vector<int64_t> soff(A.n_slices + 1);
+    for (int64_t s = 0; s <= A.n_slices; ++s) soff[s] = s * kSliceRows * width;
+    A.padded = soff.back();
+    std::vector<int> cs, ws, wo;
+    sell_partition(soff.data(), A.n_slices, A.grid, cs, ws, wo);
+    CHECK(sell_shares(soff.data(), cs, A) == FFG_OK);
+    static int16_t dcol[1];
+    A.dcol = dcol;
+    CHECK(solve_work_alloc(w, rows, A.grid) == FFG_OK);
+  }
+};
+
+struct Batch {
+  std::vector<const DeviceSell *> A;
+  std::vector<const double *> b;
+  std::vector<double *> x;
+  std::vector<SolveWork *> w;
+  explicit Batch(std::vector<System> &s) {
+    for (auto &k : s) {
+      A.push_back(&k.A);
+      b.push_back(k.b.data());
+      x.push_back(k.x.data());
+      w.push_back(&k.w);
+    }
+  }
+};
+
+ffg_solver_options options(int precision) {
+  ffg_solver_options o;
+  std::memset(&o, 0, sizeof(o));
+  o.precision = precision;
+  o.tolerance = 1e-10;
+  o.max_iterations = 100;
+  return o;
+}
+
+bool named(const Launch &l, const char *part) { return l.name.find(part) != std::string::npos; }
+
+// A wait that ran out is seen by whichever CTA it ran out in: that CTA writes
+// the control word, the first CTA may still have reported convergence.
+void batch_reports_a_wait_that_ran_out(int precision) {
+  std::vector<System> s;
+  for (int k = 0; k < 3; ++k) s.emplace_back(1000 + 500 * k, 7);
+  Batch B(s);
+  on_launch = [&](const Launch &l, void **) {
+    if (!named(l, "pcg_")) return;
+    for (auto &k : s) {
+      k.w.control[0] = 0;  // the kernels' first store
+      k.w.result[0] = 1.0;
+    }
+    s[1].w.control[0] = FFG_TIMEOUT;
+  };
+  std::string msg;
+  for (int rep = 0; rep < 2; ++rep) {
+    CHECK(pcg_launch_batch(3, B.A.data(), B.b.data(), B.x.data(), options(precision), B.w.data(), 0,
+                           msg) == FFG_OK);
+    ffg_solver_stats st;
+    CHECK(pcg_collect(s[0].w, &st, msg) == FFG_OK && st.converged);
+    CHECK(pcg_collect(s[1].w, &st, msg) == FFG_TIMEOUT);
+    CHECK(pcg_collect(s[2].w, &st, msg) == FFG_OK && st.converged);
+  }
+}
+
+}  // namespace
+
+int main(int argc, char **argv) {
+  const std::string which = argc > 1 ? argv[1] : "";
+  if (which == "batch_status_cluster") batch_reports_a_wait_that_ran_out(FFG_PRECISION_MIXED);
+  else if (which == "batch_status_single") batch_reports_a_wait_that_ran_out(FFG_PRECISION_MIXED16);
+  else return 2;
+  return 0;
+}
