@@ -716,14 +716,20 @@ size_t slice_bytes(int lr, int64_t max_column) {
   return sizeof(double) * (size_t)(max_column + 1) * (slice_threads(lr) / lr + 1);
 }
 
+// Opts a kernel into the largest image.  Always into the same size: another
+// thread may be between this and its launch of the same kernel for another mesh.
+template <class Kernel>
+bool allow_images(Kernel kern) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)kSliceImage) == cudaSuccess;
+}
+
 template <int FAMILY, bool F32>
 int launch_slices(const SliceArgs &A, int lanes, size_t smem, cudaStream_t s) {
   auto go = [&](auto kern) -> int {
     const int threads = slice_threads(lanes);
     int dev = 0, sms = 0, ctas = 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess ||
-        cudaGetDevice(&dev) != cudaSuccess ||
+    if (!allow_images(kern) || cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, kern, threads, smem) !=
             cudaSuccess ||
@@ -780,9 +786,7 @@ int launch_batch_slices(int family, int lanes, AsmBatch &B, cudaStream_t s) {
   if (!parts) return FFG_OK;
   const size_t smem = slice_bytes(lanes, max_width);
   auto go = [&](auto kern) -> int {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-      return FFG_CUDA_ERROR;
+    if (!allow_images(kern)) return FFG_CUDA_ERROR;
     kern<<<(unsigned)parts, slice_threads(lanes), smem, s>>>(B);
     return cudaGetLastError() == cudaSuccess ? FFG_OK : FFG_CUDA_ERROR;
   };

@@ -85,12 +85,63 @@ void batch_reports_a_wait_that_ran_out(int precision) {
   }
 }
 
+struct Mesh {
+  Topology t;
+  ElementTables tab;
+  DeviceTopology dt;
+  DeviceSell A;
+  AssemblyInputs in;
+  int2 range[1];
+  Mesh(int family, int nb, int max_column) {
+    t.family = family;
+    t.nb = nb;
+    t.device_free = 100;
+    t.max_column = max_column;
+    A.n = 100;
+    A.n_slices = 4;
+    A.inc_range = range;
+  }
+  int columns() {
+    return launch_columns(t, tab, dt, in, nullptr, 8, nullptr, nullptr, nullptr, nullptr, &A,
+                          nullptr, nullptr, 0);
+  }
+  int batch() {
+    AsmSys s;
+    s.nb = t.nb;
+    s.n_free = 100;
+    s.max_width = t.max_column;
+    return launch_batch_assembly(t.family, 1, &s, 0);
+  }
+};
+
+// Another thread assembles a mesh of shorter columns between this one's calls
+// to the runtime.
+void assembly_beside_another(int family, int nb, bool batch) {
+  Mesh big(family, nb, 200), small(family, nb, 9);
+  auto go = [&](Mesh &m) { return batch ? m.batch() : m.columns(); };
+  bool inside = false;
+  on_attribute = [&](const void *) {
+    if (inside) return;
+    inside = true;
+    CHECK(go(small) == FFG_OK);
+    inside = false;
+  };
+  CHECK(go(big) == FFG_OK);
+  int slices = 0;
+  for (const Launch &l : launches) slices += named(l, "slice_kernel");
+  CHECK(slices == 2);
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
   const std::string which = argc > 1 ? argv[1] : "";
   if (which == "batch_status_cluster") batch_reports_a_wait_that_ran_out(FFG_PRECISION_MIXED);
   else if (which == "batch_status_single") batch_reports_a_wait_that_ran_out(FFG_PRECISION_MIXED16);
+  else if (which == "threads_p1") assembly_beside_another(FFG_TRIANGLE_P1, 3, false);
+  else if (which == "threads_p2") assembly_beside_another(FFG_TETRA_LAGRANGE, 10, false);
+  else if (which == "threads_nedelec") assembly_beside_another(FFG_TETRA_NEDELEC, 45, false);
+  else if (which == "threads_batch") assembly_beside_another(FFG_TETRA_LAGRANGE, 10, true);
   else return 2;
   return 0;
 }

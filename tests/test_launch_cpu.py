@@ -35,3 +35,10 @@ def test_batch_reports_a_wait_that_ran_out(program, kernel):
     """Of three systems the second's control word says that a CTA other than the
     first gave up: it alone is reported so, and again by the next batch."""
     run(program, "batch_status_" + kernel)
+
+
+@pytest.mark.parametrize("what", ["p1", "p2", "nedelec", "batch"])
+def test_assembly_beside_another_thread(program, what):
+    """A thread that assembles a mesh of short columns comes between the calls of
+    one with long columns: both launches are accepted."""
+    run(program, "threads_" + what)
