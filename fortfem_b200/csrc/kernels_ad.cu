@@ -509,12 +509,13 @@ int nedelec_vjp(const Topology &t, const ElementTables &tab, const DeviceTopolog
     return sizeof(double) * ((oglobal ? 0 : (size_t)D.nb * D.nb) + (size_t)D.nb * D.fdc +
                              (size_t)D.fdc * D.fdc);
   };
-  D.oglobal = smem_for(false) > 200 * 1024 ? 1 : 0;
+  constexpr size_t kMaxSmem = 200 * 1024;
+  D.oglobal = smem_for(false) > kMaxSmem ? 1 : 0;
   const size_t smem = smem_for(D.oglobal != 0);
   if (D.oglobal && !elem) return FFG_INVALID_INPUT;
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(nedelec_cell_vjp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
+  // the same limit for every order: another thread may be before its launch
+  if (cudaFuncSetAttribute(nedelec_cell_vjp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)kMaxSmem) != cudaSuccess)
     return FFG_CUDA_ERROR;
   VjpScratch w(scratch);
   int st;

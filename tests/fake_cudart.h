@@ -84,6 +84,10 @@ cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const
 }
 cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr, int) { *v = 148; return cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetDeviceCount(int *n) { *n = 1; return cudaSuccess; }
+cudaError_t cudaFuncGetAttributes(cudaFuncAttributes *, const void *) { return cudaErrorUnknown; }
+cudaError_t cudaPeekAtLastError(void) { return cudaSuccess; }
 cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t) { return "error"; }
 cudaError_t cudaMalloc(void **p, size_t n) { *p = std::calloc(n, 1); return cudaSuccess; }

@@ -9,6 +9,8 @@ int launch_nedelec_oriented(const Topology &, const OrientedTables &, const Devi
                             const AssemblyInputs &, double *, double *, int *, cudaStream_t, bool) {
   return FFG_OK;
 }
+DeviceArena::~DeviceArena() {}
+void *DeviceArena::take(size_t bytes) { return std::malloc(bytes); }
 }  // namespace ffg
 
 namespace {
@@ -132,6 +134,42 @@ void assembly_beside_another(int family, int nb, bool batch) {
   CHECK(slices == 2);
 }
 
+// The cell kernel of an adjoint of this order: true when its launch was accepted.
+bool adjoint(int order) {
+  Topology t;
+  ElementTables tab;
+  DeviceTopology dt;
+  DeviceArena scratch;
+  t.family = FFG_TETRA_NEDELEC;
+  t.degree = order;
+  t.nb = order * (order + 2) * (order + 3) / 2;
+  t.n_cells = 1;
+  tab.n_terms = 12;
+  double elem[1];
+  struct Launched {};
+  on_launch = [](const Launch &l, void **) {
+    if (named(l, "nedelec_cell_vjp")) throw Launched();
+  };
+  try {
+    nedelec_vjp(t, tab, dt, nullptr, nullptr, nullptr, nullptr, 1, 1, elem, nullptr, nullptr,
+                nullptr, 0, scratch);
+  } catch (Launched) {
+    return true;
+  }
+  return false;
+}
+
+void adjoints_of_different_orders() {
+  bool inside = false;
+  on_attribute = [&](const void *) {
+    if (inside) return;
+    inside = true;
+    CHECK(adjoint(6));
+    inside = false;
+  };
+  CHECK(adjoint(5));
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -142,6 +180,7 @@ int main(int argc, char **argv) {
   else if (which == "threads_p2") assembly_beside_another(FFG_TETRA_LAGRANGE, 10, false);
   else if (which == "threads_nedelec") assembly_beside_another(FFG_TETRA_NEDELEC, 45, false);
   else if (which == "threads_batch") assembly_beside_another(FFG_TETRA_LAGRANGE, 10, true);
+  else if (which == "threads_adjoint") adjoints_of_different_orders();
   else return 2;
   return 0;
 }

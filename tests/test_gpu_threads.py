@@ -52,3 +52,21 @@ def test_assemblies_of_meshes_with_different_columns():
         return lambda: prob.solve(v, 1.0, 1.0, None, None, src, None, opts)[0]
 
     together([solver(fan_v, fan_t, "none"), solver(sq_v, sq_t, "none")], 100)
+
+
+def test_adjoints_of_different_orders():
+    """Nedelec adjoints of orders 5 (182 KB of shared memory) and 6 (59 KB)."""
+    v, t = oracle.box_mesh([1, 1, 1])
+
+    def adjoint(order):
+        A, st = ff.assemble_tetra_nedelec_curl_mass_csc(v, t, order=order)
+        assert st.code == 0, st.message
+        bar = np.random.default_rng(order).standard_normal(len(A.val))
+
+        def call():
+            out = ff.assemble_tetra_nedelec_curl_mass_csc_vjp(v, t, order, 1.0, 1.0, bar)
+            assert out[-1].code == 0, out[-1].message
+            return out[0]
+        return call
+
+    together([adjoint(5), adjoint(6)], 40)

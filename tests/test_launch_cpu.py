@@ -9,7 +9,8 @@ import pytest
 from fortfem_b200 import build
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-OBJECTS = ["kernels_pcg.cu.o", "kernels_pcg_resident.cu.o", "kernels_assemble.cu.o"]
+OBJECTS = ["kernels_pcg.cu.o", "kernels_pcg_resident.cu.o", "kernels_assemble.cu.o",
+           "kernels_ad.cu.o"]
 
 
 @pytest.fixture(scope="module")
@@ -35,6 +36,11 @@ def test_batch_reports_a_wait_that_ran_out(program, kernel):
     """Of three systems the second's control word says that a CTA other than the
     first gave up: it alone is reported so, and again by the next batch."""
     run(program, "batch_status_" + kernel)
+
+
+def test_adjoint_beside_another_thread(program):
+    """Orders 5 (182 KB of shared memory) and 6 (59 KB) run the same kernel."""
+    run(program, "threads_adjoint")
 
 
 @pytest.mark.parametrize("what", ["p1", "p2", "nedelec", "batch"])
