@@ -130,12 +130,19 @@ __device__ void write_partials(const PcgParams &P, unsigned int phase, const dou
   }
 }
 
+// Whether the wall limit has passed, by the first CTA: beside the partials of
+// the phase that write_partials is called for.
+__device__ __forceinline__ double *limit_slot(const PcgParams &P, unsigned int phase) {
+  return P.partial + (size_t)2 * kSlots * P.ncta + (phase & 1);
+}
+
 // Sum the partials of the phase that just completed (identical on every CTA).
 // Warp s reduces slot s; its loads are issued before the adds so they overlap,
 // and the summation order is fixed (lane-strided, then a butterfly), so every
-// CTA obtains the same bits.
-__device__ void read_partials(const PcgParams &P, unsigned int phase, double *out, int nslot) {
-  __shared__ double res[kSlots];
+// CTA obtains the same bits.  late: also the first CTA's verdict on the limit.
+__device__ void read_partials(const PcgParams &P, unsigned int phase, double *out, int nslot,
+                              bool *late = nullptr) {
+  __shared__ double res[kSlots + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp < nslot) {
     const int G = P.ncta;
@@ -154,9 +161,12 @@ __device__ void read_partials(const PcgParams &P, unsigned int phase, double *ou
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (lane == 0) res[warp] = acc;
+  } else if (late && threadIdx.x == 32 * kSlots) {
+    res[kSlots] = __ldcg(limit_slot(P, phase));
   }
   __syncthreads();
   for (int s = 0; s < nslot; ++s) out[s] = res[s];
+  if (late) *late = res[kSlots] != 0.0;
   __syncthreads();
 }
 
@@ -172,16 +182,18 @@ __device__ __forceinline__ bool sync_sums(const PcgParams &P, unsigned int &phas
   return true;
 }
 
-// Whether the wall limit has passed, judged by the first CTA every kLimitEvery
-// iterations; `ok` is false when the sync gave up.
-__device__ __forceinline__ bool past_limit(const PcgParams &P, unsigned int &phase, int iteration,
-                                           unsigned long long t_start, bool &ok) {
-  ok = true;
-  if (iteration % kLimitEvery != 0) return false;
-  double v[kVals] = {0.0, 0.0}, out[kVals];
-  if (cta_of(P) == 0 && threadIdx.x == 0 && globaltimer() - t_start > P.limit_ns) v[0] = 1.0;
-  ok = sync_sums<1>(P, phase, v, out);
-  return ok && out[0] != 0.0;
+// sync_sums<2> at the end of an iteration, with the first CTA's verdict on the
+// wall limit to every thread.
+__device__ __forceinline__ bool sync_sums_limit(const PcgParams &P, unsigned int &phase,
+                                                unsigned long long t_start,
+                                                const double (&v)[kVals], double (&out)[kVals],
+                                                bool &late) {
+  if (cta_of(P) == 0 && threadIdx.x == 0)
+    *limit_slot(P, phase + 1) = globaltimer() - t_start > P.limit_ns ? 1.0 : 0.0;
+  write_partials(P, phase, v, 2);
+  if (!grid_barrier(P, phase)) return false;
+  read_partials(P, phase, out, 2, &late);
+  return true;
 }
 
 // Slices [s0, s1) of the calling CTA.
@@ -734,7 +746,8 @@ __device__ __noinline__ void cg64(const PcgParams &P, unsigned int &phase,
           });
     }
     t1 = stamp(P);
-    if (!sync_sums<2>(P, phase, part, red)) { o.aborted = 1; return; }
+    bool late;
+    if (!sync_sums_limit(P, phase, t_start, part, red, late)) { o.aborted = 1; return; }
     t2 = stamp(P);
     tm.b += t1 - t0;
     tm.bw += t2 - t1;
@@ -742,9 +755,7 @@ __device__ __noinline__ void cg64(const PcgParams &P, unsigned int &phase,
     double rz_new = red[1];
     est2 = red[0];
     const bool reached = est2 <= target2;
-    bool ok;
-    if (past_limit(P, phase, o.iterations, t_start, ok)) { o.status = FFG_TIMEOUT; break; }
-    if (!ok) { o.aborted = 1; return; }
+    if (late) { o.status = FFG_TIMEOUT; break; }
     if (reached && !continuation) { converged = 1; break; }
     ++cycle_its;
     bool restart = false;
@@ -925,7 +936,8 @@ __device__ __noinline__ void cg_mixed(const PcgParams &P, unsigned int &phase,
         for_rows_even_batched(P, [&](int row, int u) { load(row, u); pv[u] = p[row]; }, step);
     }
     t1 = stamp(P);
-    if (!sync_sums<2>(P, phase, part, red)) { o.aborted = 1; return; }
+    bool late;
+    if (!sync_sums_limit(P, phase, t_start, part, red, late)) { o.aborted = 1; return; }
     t2 = stamp(P);
     tm.b += t1 - t0;
     tm.bw += t2 - t1;
@@ -933,13 +945,11 @@ __device__ __noinline__ void cg_mixed(const PcgParams &P, unsigned int &phase,
     unfolded = true;
     if (direct) cur ^= 1;
     const double rr = red[0], rz_new = red[1];
-    bool ok;
-    if (past_limit(P, phase, o.iterations, t_start, ok)) {
+    if (late) {
       o.status = FFG_TIMEOUT;
       true_res = sqrt(rr) * scale;
       break;
     }
-    if (!ok) { o.aborted = 1; return; }
     // reliable update: replace the recursive residual with b - A x in FP64
     // when it has fallen by delta, claims convergence, has grown tenfold
     // past the last true residual (the FP32 recurrence is diverging; the
@@ -1376,10 +1386,10 @@ void free_sell(DeviceSell &d) {
   d = DeviceSell();
 }
 
-// Partial sums of pcg_kernel ([2][kSlots][grid] doubles) or messages of the
-// resident kernel.
+// Partial sums of pcg_kernel ([2][kSlots][grid] doubles, and two for the wall
+// limit) or messages of the resident kernel.
 static size_t partial_bytes(int grid) {
-  return std::max(2 * kSlots * (size_t)grid * sizeof(double), pcg_message_bytes(grid));
+  return std::max((2 * kSlots * (size_t)grid + 2) * sizeof(double), pcg_message_bytes(grid));
 }
 
 int solve_work_alloc(SolveWork &w, int64_t n, int grid) {

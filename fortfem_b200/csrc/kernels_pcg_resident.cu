@@ -65,6 +65,10 @@ struct SliceEnt {
 struct ResShared {
   double red[kVals][16], res[kVals];
   double slot[2][kVals][kMaxCluster];
+  // the wall limit; past_limit, deadline: the first CTA's first thread's own
+  unsigned long long deadline;
+  int past_limit;  // its last look, which it takes while it waits in a phase
+  int late;        // grid: the first CTA's verdict
   unsigned long long mbar[2];
   unsigned long long mbar_all[2];  // the cluster's barrier
   int ok, items, rows;
@@ -111,12 +115,20 @@ __device__ __forceinline__ double block_sums(const double (&v)[kVals]) {
   return x;
 }
 
+// What the first CTA sends for its second sum once the wall limit has passed: a
+// signalling NaN, which no arithmetic
+// returns.  A message or a register of its own for the verdict cost the grid
+// 1.5 us an iteration in spilled registers.
+constexpr long long kLate = 0x7ff4000000000001ll;
+
 // ------------------------------------------------------------ synchronisation
 // sums<NV>(v, out): the sums of the threads' v[0..NV) over all CTAs of the
 // system, the same bits in every thread.  Every load whose value went into a
 // sum has completed before any CTA goes on, but no other memory is ordered.
 // reduce<NV>(v, out) also releases and acquires all earlier writes (NV = 0:
-// the barrier alone).  False: give up.
+// the barrier alone).  False: give up.  With a second sum
+// comes the first CTA's verdict on the wall limit: late(), to be read before the
+// next phase.
 
 // Sums travel by st.async into every CTA's slots, each counting on the
 // receiver's mbarrier, which the receiver alone waits for (with its own
@@ -208,6 +220,8 @@ struct ClusterSync {
       }
     }
     if (warp == 0) {
+      if (NV == 2 && rank == 0 && __shfl_sync(0xffffffffu, gSh.past_limit, 0) && half)
+        x = __longlong_as_double(kLate);
       if (lane == 0)
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar),
                      "r"(phase_bytes(NV, n, base ? gSh.need * slice_bytes : 0u))
@@ -219,6 +233,7 @@ struct ClusterSync {
             "l"(__double_as_longlong(x)), "r"(mapa(mbar, l))
             : "memory");
       __syncwarp();
+      if (rank == 0 && lane == 0) gSh.past_limit = globaltimer() > gSh.deadline;
       // for everything this phase expects
       wait(mbar, ((phase - 1) >> 1) & 1u);
     }
@@ -231,6 +246,9 @@ struct ClusterSync {
       for (int s = 0; s < NV; ++s) out[s] = __shfl_sync(0xffffffffu, x, 16 * s);
     }
     return gSh.ok != 0;
+  }
+  __device__ __forceinline__ bool late() const {
+    return __double_as_longlong(gSh.slot[phase & 1u][1][0]) == kLate;
   }
 
   template <int NV>
@@ -279,7 +297,8 @@ struct GridSync {
         unsigned long long e[4];
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
-          const unsigned long long bits = (unsigned long long)__double_as_longlong(s ? x1 : x);
+          unsigned long long bits = (unsigned long long)__double_as_longlong(s ? x1 : x);
+          if (NV == 2 && s == 1 && rank == 0 && gSh.past_limit) bits = kLate;
           e[2 * s] = (bits << 32) | phase;
           e[2 * s + 1] = (bits & 0xffffffff00000000ull) | phase;
         }
@@ -289,6 +308,7 @@ struct GridSync {
                        "l"(e[2 * s]), "l"(e[2 * s + 1])
                        : "memory");
       }
+      if (rank == 0 && lane == 0) gSh.past_limit = globaltimer() > gSh.deadline;
       __syncwarp();
       __nanosleep(kData ? kNapData : kNapSums);
       unsigned long long e[kPoll][4], t0 = 0;
@@ -338,6 +358,8 @@ struct GridSync {
       if (lane == 0) {
 #pragma unroll
         for (int s = 0; s < NV; ++s) gSh.res[s] = acc[s];
+        // this lane's first message is the first CTA's
+        if (NV == 2) gSh.late = ((e[0][2] >> 32) | (e[0][3] & 0xffffffff00000000ull)) == kLate;
         if (!good) gSh.ok = 0;
       }
     }
@@ -346,6 +368,7 @@ struct GridSync {
     for (int s = 0; s < NV; ++s) out[s] = gSh.res[s];
     return gSh.ok != 0;
   }
+  __device__ __forceinline__ bool late() const { return gSh.late != 0; }
 };
 
 // ------------------------------------------------------------------- a solve
@@ -658,6 +681,7 @@ struct Solve {
   }
 
   __device__ __forceinline__ bool residual_norms(double (&red)[kVals]) {
+    if (tid == 0) gSh.past_limit = 0;  // (b, b) is a sum, not a verdict
     double part[kVals] = {residual<false>(nullptr), 0.0};
     for_rows([&](int, int row) {
       const double bb = gP.b[row];
@@ -671,24 +695,13 @@ struct Solve {
     return S.template reduce<0>(none, out);
   }
 
-  // Whether the wall limit has passed, judged by the first CTA every
-  // kLimitEvery iterations; false in `ok` when the sync gave up.
-  __device__ __forceinline__ bool late(int iteration, unsigned long long t_start, bool &ok) {
-    ok = true;
-    if (iteration % kLimitEvery != 0) return false;
-    double v[kVals] = {0.0, 0.0}, out[kVals];
-    if (S.rank == 0 && tid == 0 && globaltimer() - t_start > gP.limit_ns) v[0] = 1.0;
-    ok = S.template sums<1>(v, out);
-    return ok && out[0] != 0.0;
-  }
-
   __device__ __forceinline__ unsigned long long stamp() const {
     return (S.rank == 0 && tid == 0) ? clock_now() : 0ull;
   }
 
   // cg64 of kernels_pcg.cu: the reference's recurrences (or, after a stagnated
   // mixed solve, its continuation in restarted cycles).
-  __device__ __forceinline__ void fp64(unsigned long long t_start, bool continuation, Outcome &o,
+  __device__ __forceinline__ void fp64(bool continuation, Outcome &o,
                                     Timing &tm) {
     setup<double>(gP.v64);
     double *r = vecs<double>(0), *p = vecs<double>(1), *q = vecs<double>(2), *d = vecs<double>(3),
@@ -764,9 +777,7 @@ struct Solve {
       double rz_new = red[1];
       est2 = red[0];
       const bool reached = est2 <= target2;
-      bool ok;
-      if (late(o.iterations, t_start, ok)) { o.status = FFG_TIMEOUT; break; }
-      if (!ok) { o.aborted = 1; return; }
+      if (S.late()) { o.status = FFG_TIMEOUT; break; }
       if (reached && !continuation) { converged = 1; break; }
       ++cycle_its;
       bool restart = false;
@@ -812,7 +823,7 @@ struct Solve {
   }
 
   // cg_mixed of kernels_pcg.cu.
-  __device__ __forceinline__ void mixed(unsigned long long t_start, Outcome &o, Timing &tm) {
+  __device__ __forceinline__ void mixed(Outcome &o, Timing &tm) {
     setup<float>(gP.v32);
     float *r = vecs<float>(0), *p = vecs<float>(1), *q = vecs<float>(2), *d = vecs<float>(3),
           *xf = vecs<float>(4);
@@ -921,13 +932,11 @@ struct Solve {
       ++o.iterations;
       unfolded = true;
       const double rr = red[0], rz_new = red[1];
-      bool ok;
-      if (late(o.iterations, t_start, ok)) {
+      if (S.late()) {
         o.status = FFG_TIMEOUT;
         true_res = sqrt(rr) * scale;
         break;
       }
-      if (!ok) { o.aborted = 1; return; }
       // the estimate sqrt(rr) * scale against the target, delta and growth, squared
       const bool grew = !(rr < 100.0);
       const bool slow = o.iterations - since > window;
@@ -1072,21 +1081,19 @@ struct Solve {
 };
 
 template <class Sync, int IDX, int NT>
-__device__ __noinline__ Sync run_mixed(Share h, Sync sync, unsigned long long t_start,
-                                           Outcome &out, Timing &tmo) {
+__device__ __noinline__ Sync run_mixed(Share h, Sync sync, Outcome &out, Timing &tmo) {
   Solve<Sync, IDX, NT> X;
   X.init(h, sync);
   Outcome o;
   Timing tm;
-  X.mixed(t_start, o, tm);
+  X.mixed(o, tm);
   out = o;
   tmo = tm;
   return X.S;
 }
 
 template <class Sync, int IDX, int NT>
-__device__ __noinline__ Sync run_fp64(Share h, Sync sync, unsigned long long t_start,
-                                          bool continuation, Outcome &out, Timing &tmo) {
+__device__ __noinline__ Sync run_fp64(Share h, Sync sync, bool continuation, Outcome &out, Timing &tmo) {
   Solve<Sync, IDX, NT> X;
   X.init(h, sync);
   Outcome o = out;
@@ -1095,7 +1102,7 @@ __device__ __noinline__ Sync run_fp64(Share h, Sync sync, unsigned long long t_s
     X.for_rows([&](int, int row) { gP.x[row] = 0.0; });
   }
   if (!X.barrier()) o.aborted = 1;
-  else X.fp64(t_start, continuation, o, tm);
+  else X.fp64(continuation, o, tm);
   out = o;
   tmo = tm;
   return X.S;
@@ -1107,6 +1114,10 @@ __device__ __noinline__ Sync run_fp64(Share h, Sync sync, unsigned long long t_s
 template <class Sync, bool kShared, int NT>
 __device__ __forceinline__ void run_solve(const Share &h, Sync sync) {
   const unsigned long long t_start = globaltimer(), c_start = clock_now();
+  if (threadIdx.x == 0) {
+    gSh.deadline = t_start + gP.limit_ns;
+    gSh.past_limit = 0;
+  }
   Outcome o;
   Timing tm;
   int continued = 0;
@@ -1115,13 +1126,13 @@ __device__ __forceinline__ void run_solve(const Share &h, Sync sync) {
     bool done = false;
     if constexpr (kShared) {
       if (gP.staged & 1) {
-        sync = run_mixed<Sync, kAbs16, NT>(h, sync, t_start, o, tm);
+        sync = run_mixed<Sync, kAbs16, NT>(h, sync, o, tm);
         done = true;
       }
     }
     if (done) {
-    } else if (gP.dcol) sync = run_mixed<Sync, kRel16, NT>(h, sync, t_start, o, tm);
-    else sync = run_mixed<Sync, kAbs32, NT>(h, sync, t_start, o, tm);
+    } else if (gP.dcol) sync = run_mixed<Sync, kRel16, NT>(h, sync, o, tm);
+    else sync = run_mixed<Sync, kAbs32, NT>(h, sync, o, tm);
     if (!o.aborted && o.stagnated && !o.converged && o.status == FFG_OK) {
       continued = o.restart ? 2 : 1;
       fp64 = continuation = true;
@@ -1131,13 +1142,13 @@ __device__ __forceinline__ void run_solve(const Share &h, Sync sync) {
     bool done = false;
     if constexpr (kShared) {
       if (gP.staged & 2) {
-        run_fp64<Sync, kAbs16, NT>(h, sync, t_start, continuation, o, tm);
+        run_fp64<Sync, kAbs16, NT>(h, sync, continuation, o, tm);
         done = true;
       }
     }
     if (done) {
-    } else if (gP.dcol) run_fp64<Sync, kRel16, NT>(h, sync, t_start, continuation, o, tm);
-    else run_fp64<Sync, kAbs32, NT>(h, sync, t_start, continuation, o, tm);
+    } else if (gP.dcol) run_fp64<Sync, kRel16, NT>(h, sync, continuation, o, tm);
+    else run_fp64<Sync, kAbs32, NT>(h, sync, continuation, o, tm);
   }
   if (o.aborted) {
     // a sync gave up: the host reads the status, not an older result

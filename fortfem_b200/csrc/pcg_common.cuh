@@ -78,7 +78,6 @@ __device__ __forceinline__ bool is_finite_d(double x) { return isfinite(x); }
 
 constexpr int kVals = 2;  // values of one reduction, at most
 constexpr int kPoll = 5;            // messages a lane polls: up to 160 CTAs
-constexpr int kLimitEvery = 64;    // iterations between looks at the wall limit
 
 struct Outcome {
   int iterations = 0, updates = 0, converged = 0, status = FFG_OK, stagnated = 0, aborted = 0;

@@ -166,8 +166,6 @@ LOOPS = {
     "update": "P X1 S1 P X2 B P X0 S1 P X1 S1 P X2",
     # the update that changes to the direct form, an iteration, an update in it
     "direct": "P X1 S1 P X2 B P X0 S1 S1 P X0 S1 S2 B S1 S1 P X0 S1 S2",
-    # a look at the wall limit between the phases
-    "limit": "P X0 S1 S2 S1 P X0 S1 S2",
     # the change to the FP64 loop (two barriers on end), its vector in global memory
     "global": "X1 S1 X2 B B S2 B S1 S2 B S1 S2 B B B S1",
 }

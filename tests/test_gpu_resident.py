@@ -174,3 +174,54 @@ def test_cluster_mixed_solve_continues_in_fp64(family, n, relabel):
     assert abs(res - st.true_relative_residual) <= 2 * (terms + 1) * level
     assert st.converged or family == K.FFG_TRIANGLE_P1
     assert res <= max(1.01 * opts.tolerance, 2 * (terms + 2) * level)
+
+
+@pytest.mark.parametrize("precision,n,per_row,span", [
+    ("mixed", 257, 7, 40), ("fp64", 257, 7, 40),                  # cluster
+    ("mixed", 40009, 12, 40000), ("fp64", 40009, 12, 40000),      # grid
+    ("mixed16", 4097, 9, 4000), ("fp64", 900001, 12, 30000),      # streamed
+])
+def test_wall_limit_is_looked_at_every_iteration(precision, n, per_row, span):
+    """Solves of some tens of iterations, with a limit that has passed at the first."""
+    A = dominant(n, per_row, span, n)
+    b = np.random.default_rng(n).standard_normal(n)
+    A.sort_indices()
+    M = ff.CscMatrix(n, n, A.indptr.astype(np.int64), A.indices.astype(np.int32), A.data)
+    opts = ff.solver_options(method="pcg", preconditioner="jacobi", tolerance=TOL,
+                             precision=precision, max_iterations=60, breakdown_guard="spd")
+    st = ff.solve_sparse(M, b, np.zeros(n), opts)
+    assert st.converged and 5 < st.iterations < 60
+    opts.timeout_seconds = 1e-9
+    with pytest.raises(ff.FortfemError) as e:
+        ff.solve_sparse(M, b, np.zeros(n), opts)
+    assert e.value.code == K.FFG_TIMEOUT
+
+
+@pytest.mark.parametrize("mode", ["cta_per_system", "cta_groups", "whole_device"])
+@pytest.mark.parametrize("precision", ["mixed", "mixed16"])
+def test_wall_limit_of_a_batch(mode, precision):
+    import torch
+    from fortfem_b200.api import solve_batch
+    probs, inputs = [], []
+    for k, n in enumerate((9, 14)):
+        v, t = oracle.unit_square_mesh(n)
+        probs.append(ff.Problem(K.FFG_TRIANGLE_P1, 1, t, len(v)))
+        dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+        src = np.ones(probs[-1].sample_points(v).shape[:-1])
+        inputs.append((dev(v), dev(src)))
+    for limit, want in ((1e-9, False), (60.0, True)):
+        opts = ff.SolverOptions(method="pcg", preconditioner="jacobi", tolerance=TOL,
+                                precision=precision, timeout_seconds=limit)
+        out = [torch.empty(p.n_dofs, dtype=torch.float64, device="cuda") for p in probs]
+        solve_batch(probs, [i[0] for i in inputs], out, [1.0, 1.0], [0.0, 0.0],
+                    samples=[i[1] for i in inputs], options=opts, mode=mode)
+        torch.cuda.synchronize()
+        for p in probs:
+            if want:
+                assert p.batch_stats().converged
+            else:
+                with pytest.raises(ff.FortfemError) as e:
+                    p.batch_stats()
+                assert e.value.code == K.FFG_TIMEOUT
+    for p in probs:
+        p.close()
