@@ -201,6 +201,10 @@ __device__ __forceinline__ void slice_range(const PcgParams &P, int &s0, int &s1
   if (P.ncta == 1) {
     s0 = 0;
     s1 = P.n_slices;
+  } else if (!P.cta_slice) {
+    // a CTA group of a batch: equal slice counts
+    s0 = (int)((int64_t)cta_of(P) * P.n_slices / P.ncta);
+    s1 = (int)((int64_t)(cta_of(P) + 1) * P.n_slices / P.ncta);
   } else {
     s0 = P.cta_slice[cta_of(P)];
     s1 = P.cta_slice[cta_of(P) + 1];
@@ -1110,6 +1114,34 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_batch_kernel(const __grid_con
   pcg_body(Ps);
 }
 
+// Independent systems on an FP16 operator (the on-chip kernels have none) side
+// by side in one cooperative launch, system i on CTAs first[i] .. first[i + 1] - 1
+// with its own barrier counter, partial sums and control word.  The launch
+// makes every CTA resident together, so a group's barrier waits only on CTAs
+// that are running; its size depends on the system alone (group_ctas), so its
+// result does not depend on the other systems of the launch.
+constexpr int64_t kGroupRows = 16384;  // rows per CTA of a group
+struct PcgGroups {
+  PcgParams sys[kMaxResidentGroups];
+  int first[kMaxResidentGroups + 1];
+  int count;
+};
+__global__ void __launch_bounds__(kThreads, 1) pcg_group_kernel(const __grid_constant__ PcgGroups B) {
+  __shared__ PcgParams Ps;
+  if (threadIdx.x == 0) {
+    int i = 0;
+    while (i + 1 < B.count && B.first[i + 1] <= (int)blockIdx.x) ++i;
+    Ps = B.sys[i];
+    Ps.cta0 = B.first[i];
+    // the operator's partition is for the whole grid: groups split evenly
+    Ps.cta_slice = nullptr;
+    Ps.wslice = nullptr;
+    Ps.woff = nullptr;
+  }
+  __syncthreads();
+  pcg_body(Ps);
+}
+
 // Drop-in FP64 CSR SpMV, one thread per row (spmv / csc_matvec semantics).
 __global__ void csr_spmv64_kernel(int64_t n, const int64_t *rp, const int *ci, const double *v,
                                   const double *x, double *y) {
@@ -1158,6 +1190,8 @@ bool staged_smem_ready() {
         cudaFuncSetAttribute((const void *)pcg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kStageSmem) == cudaSuccess &&
         cudaFuncSetAttribute((const void *)pcg_batch_kernel,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, kStageSmem) == cudaSuccess &&
+        cudaFuncSetAttribute((const void *)pcg_group_kernel,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, kStageSmem) == cudaSuccess;
     if (!ok) cudaGetLastError();
     state[dev] = ok ? 1 : -1;
@@ -1583,6 +1617,29 @@ int pcg_launch_batch(int count, const DeviceSell *const *A, const double *const 
   return FFG_OK;
 }
 
+namespace {
+int group_ctas(int64_t n, int grid) {
+  const int64_t g = (n + kGroupRows - 1) / kGroupRows;
+  return (int)std::max<int64_t>(2, std::min<int64_t>(g, grid));
+}
+
+cudaError_t launch_half_groups(int count, const PcgParams *sys, cudaStream_t s) {
+  static_assert(sizeof(PcgGroups) <= 32000, "kernel parameter block too large");
+  const int staged = staged_smem_ready() ? 1 : 0;
+  PcgGroups B;
+  B.count = count;
+  B.first[0] = 0;
+  for (int i = 0; i < count; ++i) {
+    B.sys[i] = sys[i];
+    B.sys[i].staged = staged;
+    B.first[i + 1] = B.first[i] + sys[i].ncta;
+  }
+  void *args[] = {&B};
+  return cudaLaunchCooperativeKernel((const void *)pcg_group_kernel, dim3(B.first[count]),
+                                     dim3(kThreads), args, staged ? kStageSmem : 0, s);
+}
+}  // namespace
+
 int pcg_launch_groups(int count, const DeviceSell *const *A, const double *const *b,
                       double *const *x, const ffg_solver_options &opts, SolveWork *const *w,
                       cudaStream_t stream, std::string &msg) {
@@ -1590,10 +1647,12 @@ int pcg_launch_groups(int count, const DeviceSell *const *A, const double *const
   int st = pcg_grid_size(&grid);
   if (st) return st;
   // the CTAs of every system, by the system alone
+  const bool half = opts.precision == FFG_PRECISION_MIXED16;
   std::vector<int> ctas((size_t)count), slices((size_t)count, 0), order((size_t)count);
   for (int i = 0; i < count; ++i) {
     order[i] = i;
-    ctas[i] = pcg_group_shape(*A[i], opts.precision, grid, &slices[i]);
+    ctas[i] = half ? group_ctas(A[i]->n, grid)
+                   : pcg_group_shape(*A[i], opts.precision, grid, &slices[i]);
     if (w[i]->n != A[i]->n || A[i]->n < 1 || w[i]->grid < ctas[i]) {
       msg = "solver workspace mismatch";
       return FFG_INVALID_INPUT;
@@ -1614,7 +1673,8 @@ int pcg_launch_groups(int count, const DeviceSell *const *A, const double *const
       if ((st = pcg_launch(*A[i], b[i], x[i], opts, *w[i], stream, msg))) return st;
       done[i] = 1;
     } else if (!clear_state(*w[i], stream) ||
-               cudaMemsetAsync(w[i]->partial, 0, pcg_message_bytes(ctas[i]), stream) !=
+               (half ? cudaMemsetAsync(w[i]->barrier, 0, 64, stream)
+                     : cudaMemsetAsync(w[i]->partial, 0, pcg_message_bytes(ctas[i]), stream)) !=
                    cudaSuccess) {
       return FFG_CUDA_ERROR;
     }
@@ -1634,7 +1694,8 @@ int pcg_launch_groups(int count, const DeviceSell *const *A, const double *const
       done[i] = 1;
     }
     if (R.empty()) break;
-    const cudaError_t e = pcg_launch_resident_groups((int)R.size(), R.data(), stream);
+    const cudaError_t e = half ? launch_half_groups((int)R.size(), R.data(), stream)
+                               : pcg_launch_resident_groups((int)R.size(), R.data(), stream);
     if (e != cudaSuccess) {
       msg = std::string("cooperative group launch failed: ") + cudaGetErrorString(e);
       cudaGetLastError();

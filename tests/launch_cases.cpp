@@ -87,6 +87,17 @@ void batch_reports_a_wait_that_ran_out(int precision) {
   }
 }
 
+// Systems that fit the grid together share one launch, in every precision.
+void groups_side_by_side(int precision) {
+  std::vector<System> s;
+  for (int k = 0; k < 3; ++k) s.emplace_back(17000 + 500 * k, 7);
+  Batch B(s);
+  std::string msg;
+  CHECK(pcg_launch_groups(3, B.A.data(), B.b.data(), B.x.data(), options(precision), B.w.data(), 0,
+                          msg) == FFG_OK);
+  CHECK(launches.size() == 1 && launches[0].cooperative && launches[0].blocks <= 148);
+}
+
 struct Mesh {
   Topology t;
   ElementTables tab;
@@ -181,6 +192,9 @@ int main(int argc, char **argv) {
   else if (which == "threads_nedelec") assembly_beside_another(FFG_TETRA_NEDELEC, 45, false);
   else if (which == "threads_batch") assembly_beside_another(FFG_TETRA_LAGRANGE, 10, true);
   else if (which == "threads_adjoint") adjoints_of_different_orders();
+  else if (which == "groups_fp64") groups_side_by_side(FFG_PRECISION_FP64);
+  else if (which == "groups_mixed") groups_side_by_side(FFG_PRECISION_MIXED);
+  else if (which == "groups_mixed16") groups_side_by_side(FFG_PRECISION_MIXED16);
   else return 2;
   return 0;
 }

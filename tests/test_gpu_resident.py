@@ -225,3 +225,38 @@ def test_wall_limit_of_a_batch(mode, precision):
                 assert e.value.code == K.FFG_TIMEOUT
     for p in probs:
         p.close()
+
+
+def test_half_precision_groups_match_alone():
+    """MIXED16 systems side by side, each the bits of its own launch and, as a
+    solution, within the residual of the whole device's."""
+    import torch
+    from fortfem_b200.api import solve_batch
+    probs, vs, fs = [], [], []
+    for n in (20, 45, 90, 140):
+        v, t = oracle.unit_square_mesh(n)
+        probs.append(ff.Problem(K.FFG_TRIANGLE_P1, 1, t, len(v)))
+        vs.append(torch.from_numpy(np.ascontiguousarray(v)).cuda())
+        fs.append(torch.ones(probs[-1].sample_points(v).shape[:-1], dtype=torch.float64,
+                             device="cuda"))
+    opts = ff.SolverOptions(method="pcg", preconditioner="jacobi", tolerance=TOL,
+                            precision="mixed16", max_iterations=1000000)
+
+    def run(which, mode):
+        out = [torch.empty(probs[i].n_dofs, dtype=torch.float64, device="cuda") for i in which]
+        one = [1.0] * len(which)
+        solve_batch([probs[i] for i in which], [vs[i] for i in which], out, one, one,
+                    samples=[fs[i] for i in which], options=opts, mode=mode)
+        torch.cuda.synchronize()
+        for i in which:
+            st = probs[i].batch_stats()
+            assert st.converged and st.true_relative_residual <= 1.01 * TOL
+        return [o.cpu().numpy() for o in out]
+
+    together = run(range(4), "cta_groups")
+    for i in range(4):
+        assert np.array_equal(run([i], "cta_groups")[0], together[i])
+        whole = run([i], "whole_device")[0]
+        assert np.linalg.norm(whole - together[i]) <= 1e-6 * np.linalg.norm(whole)
+    for p in probs:
+        p.close()

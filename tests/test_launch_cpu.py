@@ -38,6 +38,11 @@ def test_batch_reports_a_wait_that_ran_out(program, kernel):
     run(program, "batch_status_" + kernel)
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "mixed16"])
+def test_group_batch_is_one_launch(program, precision):
+    run(program, "groups_" + precision)
+
+
 def test_adjoint_beside_another_thread(program):
     """Orders 5 (182 KB of shared memory) and 6 (59 KB) run the same kernel."""
     run(program, "threads_adjoint")
