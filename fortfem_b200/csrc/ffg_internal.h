@@ -248,8 +248,8 @@ int pcg_launch_batch(int count, const DeviceSell *const *A, const double *const 
                      cudaStream_t stream, std::string &msg);
 // Independent systems in shared cooperative launches, each on a group of CTAs
 // whose size depends on the system alone: a k-th of the grid whose shared
-// memory holds the operator (pcg_group_shape); systems that no group holds run
-// one after another on the whole device.
+// memory holds the operator (pcg_group_shape), or, streaming an operator that no
+// group holds or an FP16 one, a CTA for every 16384 rows.
 int pcg_launch_groups(int count, const DeviceSell *const *A, const double *const *b,
                       double *const *x, const ffg_solver_options &opts, SolveWork *const *w,
                       cudaStream_t stream, std::string &msg);

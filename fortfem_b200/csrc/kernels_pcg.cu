@@ -1114,8 +1114,8 @@ __global__ void __launch_bounds__(kThreads, 1) pcg_batch_kernel(const __grid_con
   pcg_body(Ps);
 }
 
-// Independent systems on an FP16 operator (the on-chip kernels have none) side
-// by side in one cooperative launch, system i on CTAs first[i] .. first[i + 1] - 1
+// Independent systems that the on-chip group kernel does not take (an operator
+// too large for it, or one in FP16) side by side in one cooperative launch, system i on CTAs first[i] .. first[i + 1] - 1
 // with its own barrier counter, partial sums and control word.  The launch
 // makes every CTA resident together, so a group's barrier waits only on CTAs
 // that are running; its size depends on the system alone (group_ctas), so its
@@ -1623,7 +1623,7 @@ int group_ctas(int64_t n, int grid) {
   return (int)std::max<int64_t>(2, std::min<int64_t>(g, grid));
 }
 
-cudaError_t launch_half_groups(int count, const PcgParams *sys, cudaStream_t s) {
+cudaError_t launch_streamed_groups(int count, const PcgParams *sys, cudaStream_t s) {
   static_assert(sizeof(PcgGroups) <= 32000, "kernel parameter block too large");
   const int staged = staged_smem_ready() ? 1 : 0;
   PcgGroups B;
@@ -1647,12 +1647,15 @@ int pcg_launch_groups(int count, const DeviceSell *const *A, const double *const
   int st = pcg_grid_size(&grid);
   if (st) return st;
   // the CTAs of every system, by the system alone
-  const bool half = opts.precision == FFG_PRECISION_MIXED16;
   std::vector<int> ctas((size_t)count), slices((size_t)count, 0), order((size_t)count);
+  std::vector<char> streamed((size_t)count, 0);
   for (int i = 0; i < count; ++i) {
     order[i] = i;
-    ctas[i] = half ? group_ctas(A[i]->n, grid)
-                   : pcg_group_shape(*A[i], opts.precision, grid, &slices[i]);
+    ctas[i] = pcg_group_shape(*A[i], opts.precision, grid, &slices[i]);
+    if (!ctas[i]) {
+      streamed[i] = 1;
+      ctas[i] = group_ctas(A[i]->n, grid);
+    }
     if (w[i]->n != A[i]->n || A[i]->n < 1 || w[i]->grid < ctas[i]) {
       msg = "solver workspace mismatch";
       return FFG_INVALID_INPUT;
@@ -1666,44 +1669,42 @@ int pcg_launch_groups(int count, const DeviceSell *const *A, const double *const
     return A[i]->padded < 10 * A[i]->n ? std::sqrt(n) : 1.5 * std::cbrt(n);
   };
   std::stable_sort(order.begin(), order.end(), [&](int i, int j) { return length(i) > length(j); });
-  std::vector<char> done((size_t)count, 0);
-  for (int i : order) {
-    if (!ctas[i]) {
-      // no group holds it on chip: the whole device
-      if ((st = pcg_launch(*A[i], b[i], x[i], opts, *w[i], stream, msg))) return st;
-      done[i] = 1;
-    } else if (!clear_state(*w[i], stream) ||
-               (half ? cudaMemsetAsync(w[i]->barrier, 0, 64, stream)
+  for (int i : order)
+    if (!clear_state(*w[i], stream) ||
+        (streamed[i] ? cudaMemsetAsync(w[i]->barrier, 0, 64, stream)
                      : cudaMemsetAsync(w[i]->partial, 0, pcg_message_bytes(ctas[i]), stream)) !=
-                   cudaSuccess) {
+            cudaSuccess)
       return FFG_CUDA_ERROR;
+  std::vector<char> done((size_t)count, 0);
+  for (const bool stream_them : {true, false})
+    while (true) {
+      // one launch: the first system of the kind not yet launched and, in order,
+      // those that still fit beside it
+      std::vector<PcgParams> R;
+      int used = 0;
+      for (int i : order) {
+        if (done[i] || (streamed[i] != 0) != stream_them ||
+            (int)R.size() == kMaxResidentGroups || used + ctas[i] > grid)
+          continue;
+        PcgParams P = make_params(*A[i], b[i], x[i], opts, *w[i]);
+        P.ncta = ctas[i];
+        P.share_slices = slices[i];
+        R.push_back(P);
+        used += ctas[i];
+        done[i] = 1;
+      }
+      if (R.empty()) break;
+      const cudaError_t e = stream_them
+                                ? launch_streamed_groups((int)R.size(), R.data(), stream)
+                                : pcg_launch_resident_groups((int)R.size(), R.data(), stream);
+      if (e != cudaSuccess) {
+        msg = std::string("cooperative group launch failed: ") + cudaGetErrorString(e);
+        cudaGetLastError();
+        return FFG_CUDA_ERROR;
+      }
     }
-  }
-  while (true) {
-    // one launch: the first system not yet launched and, in order, those that
-    // still fit beside it
-    std::vector<PcgParams> R;
-    int used = 0;
-    for (int i : order) {
-      if (done[i] || (int)R.size() == kMaxResidentGroups || used + ctas[i] > grid) continue;
-      PcgParams P = make_params(*A[i], b[i], x[i], opts, *w[i]);
-      P.ncta = ctas[i];
-      P.share_slices = slices[i];
-      R.push_back(P);
-      used += ctas[i];
-      done[i] = 1;
-    }
-    if (R.empty()) break;
-    const cudaError_t e = half ? launch_half_groups((int)R.size(), R.data(), stream)
-                               : pcg_launch_resident_groups((int)R.size(), R.data(), stream);
-    if (e != cudaSuccess) {
-      msg = std::string("cooperative group launch failed: ") + cudaGetErrorString(e);
-      cudaGetLastError();
-      return FFG_CUDA_ERROR;
-    }
-  }
   for (int k = 0; k < count; ++k)
-    if (ctas[k] && !fetch_state(*w[k], stream)) return FFG_CUDA_ERROR;
+    if (!fetch_state(*w[k], stream)) return FFG_CUDA_ERROR;
   return FFG_OK;
 }
 

@@ -474,8 +474,9 @@ void ffg_problem_phase_times(int handle, double *seconds, int *status);
  * 16th) whose shared memory holds its operator, so that mid-size systems,
  * whose iterations are bound by synchronisation rather than by bandwidth,
  * share the GPU while a system's result still does not depend on the rest of
- * the batch (a system too large for that takes the whole GPU).  A problem may belong to one
- * unfinished batch at a time. */
+ * the batch; a system too large for that, and FFG_PRECISION_MIXED16, stream
+ * the operator on a block for every 16384 rows (at least 2, at most one per
+ * SM).  A problem may belong to one unfinished batch at a time. */
 #define FFG_BATCH_CTA_PER_SYSTEM 0
 #define FFG_BATCH_WHOLE_DEVICE 1
 #define FFG_BATCH_CTA_GROUPS 2

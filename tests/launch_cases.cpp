@@ -88,9 +88,9 @@ void batch_reports_a_wait_that_ran_out(int precision) {
 }
 
 // Systems that fit the grid together share one launch, in every precision.
-void groups_side_by_side(int precision) {
+void groups_side_by_side(int precision, int64_t rows, int width) {
   std::vector<System> s;
-  for (int k = 0; k < 3; ++k) s.emplace_back(17000 + 500 * k, 7);
+  for (int k = 0; k < 3; ++k) s.emplace_back(rows + 500 * k, width);
   Batch B(s);
   std::string msg;
   CHECK(pcg_launch_groups(3, B.A.data(), B.b.data(), B.x.data(), options(precision), B.w.data(), 0,
@@ -192,9 +192,10 @@ int main(int argc, char **argv) {
   else if (which == "threads_nedelec") assembly_beside_another(FFG_TETRA_NEDELEC, 45, false);
   else if (which == "threads_batch") assembly_beside_another(FFG_TETRA_LAGRANGE, 10, true);
   else if (which == "threads_adjoint") adjoints_of_different_orders();
-  else if (which == "groups_fp64") groups_side_by_side(FFG_PRECISION_FP64);
-  else if (which == "groups_mixed") groups_side_by_side(FFG_PRECISION_MIXED);
-  else if (which == "groups_mixed16") groups_side_by_side(FFG_PRECISION_MIXED16);
+  else if (which == "groups_fp64") groups_side_by_side(FFG_PRECISION_FP64, 17000, 7);
+  else if (which == "groups_mixed") groups_side_by_side(FFG_PRECISION_MIXED, 17000, 7);
+  else if (which == "groups_large") groups_side_by_side(FFG_PRECISION_MIXED, 490000, 28);
+  else if (which == "groups_mixed16") groups_side_by_side(FFG_PRECISION_MIXED16, 17000, 7);
   else return 2;
   return 0;
 }

@@ -38,8 +38,9 @@ def test_batch_reports_a_wait_that_ran_out(program, kernel):
     run(program, "batch_status_" + kernel)
 
 
-@pytest.mark.parametrize("precision", ["fp64", "mixed", "mixed16"])
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "mixed16", "large"])
 def test_group_batch_is_one_launch(program, precision):
+    """large: mixed systems that no group of CTAs holds on chip."""
     run(program, "groups_" + precision)
 
 
