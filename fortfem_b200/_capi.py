@@ -160,6 +160,7 @@ SIGNATURES = {
     "ffg_problem_reduced_system": (
         None, [i32, vp, f64, f64, vp, vp, vp, vp, i64, pi64, vp, vp, vp, vp, vp, pi32]),
     "ffg_problem_phase_times": (None, [i32, vp, pi32]),
+    "ffg_problem_group_ctas": (None, [i32, i32, pi32, pi32]),
     "ffg_problem_solve_batch": (
         None, [i32, vp, vp, vp, vp, vp, vp, vp, vp, C.POINTER(SolverOptionsC), vp, i32, vp, pi32]),
     "ffg_problem_batch_stats": (None, [i32, C.POINTER(SolverStatsC), pi32]),

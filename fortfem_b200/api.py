@@ -799,6 +799,20 @@ class Problem:
         return {"fp64_continuation": bool(out[0]), "spmv": out[1], "spmv_barrier": out[2],
                 "vector": out[3], "vector_barrier": out[4], "residual_replacement": out[5]}
 
+    def group_ctas(self, precision: str = "mixed") -> int:
+        """Thread blocks of this system in a "cta_groups" batch that keeps it on chip,
+        0 where it is streamed (ffg_problem_group_ctas)."""
+        ctas = C.c_int(0)
+        st = C.c_int(0)
+        modes = {"fp64": K.FFG_PRECISION_FP64, "mixed": K.FFG_PRECISION_MIXED,
+                 "mixed16": K.FFG_PRECISION_MIXED16}
+        if precision not in modes:
+            raise FortfemError(K.FFG_INVALID_INPUT, f"precision {precision!r}")
+        K.load().ffg_problem_group_ctas(self.handle, modes[precision], C.byref(ctas), C.byref(st))
+        if st.value:
+            raise FortfemError(st.value, "ffg_problem_group_ctas")
+        return ctas.value
+
     def reduced_system(self, vertices, coef_a=1.0, coef_b=0.0, cell_a=None, cell_b=None,
                        samples=None, constrained_values=None):
         """The constrained (free x free) CSC, its lifted right-hand side and the free DoFs."""

@@ -1293,6 +1293,18 @@ void ffg_problem_solve(int handle, const double *vertices, double ca, double cb,
   if (local.converged) *status = FFG_OK;
 }
 
+void ffg_problem_group_ctas(int handle, int precision, int *ctas, int *status) {
+  auto P = find_problem(handle);
+  if (!P) { *status = FFG_BAD_HANDLE; return; }
+  if (!ctas || (precision != FFG_PRECISION_FP64 && precision != FFG_PRECISION_MIXED &&
+                precision != FFG_PRECISION_MIXED16)) {
+    *status = FFG_INVALID_INPUT;
+    return;
+  }
+  *ctas = pcg_group_ctas(P->S, precision);
+  *status = FFG_OK;
+}
+
 void ffg_problem_solve_batch(int count, const int *handles, const double *const *vertices,
                              const double *coef_a, const double *coef_b,
                              const double *const *cell_a, const double *const *cell_b,

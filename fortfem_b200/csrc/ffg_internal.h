@@ -250,6 +250,7 @@ int pcg_launch_batch(int count, const DeviceSell *const *A, const double *const 
 // whose size depends on the system alone: a k-th of the grid whose shared
 // memory holds the operator (pcg_group_shape), or, streaming an operator that no
 // group holds or an FP16 one, a CTA for every 16384 rows.
+int pcg_group_ctas(const DeviceSell &A, int precision);  // on chip; 0: streamed
 int pcg_launch_groups(int count, const DeviceSell *const *A, const double *const *b,
                       double *const *x, const ffg_solver_options &opts, SolveWork *const *w,
                       cudaStream_t stream, std::string &msg);

@@ -1640,6 +1640,11 @@ cudaError_t launch_streamed_groups(int count, const PcgParams *sys, cudaStream_t
 }
 }  // namespace
 
+int pcg_group_ctas(const DeviceSell &A, int precision) {
+  int grid = 0, slices = 0;
+  return pcg_grid_size(&grid) ? 0 : pcg_group_shape(A, precision, grid, &slices);
+}
+
 int pcg_launch_groups(int count, const DeviceSell *const *A, const double *const *b,
                       double *const *x, const ffg_solver_options &opts, SolveWork *const *w,
                       cudaStream_t stream, std::string &msg) {

@@ -39,7 +39,7 @@ import math
 import time
 from collections import Counter, deque
 from dataclasses import dataclass, field
-from typing import Dict, List, Optional, Tuple
+from typing import Callable, Dict, List, Optional, Tuple
 
 import numpy as np
 
@@ -123,7 +123,10 @@ class Scheduler:
     # another on the whole device
     groups: bool = False
     grid: int = 148
-    group_rows: int = 2048
+    # the blocks of a mesh size, 0: alone on the whole device (DeviceEngine.group_ctas);
+    # without it one for every group_rows rows, 2 to grid
+    shape: Optional[Callable] = None
+    group_rows: int = 16384
     max_groups: int = 16
     queue: deque = field(default_factory=deque)
     inflight: List[Batch] = field(default_factory=list)
@@ -132,28 +135,29 @@ class Scheduler:
         return free_dofs(r.key) <= self.small_rows
 
     def group_ctas(self, key) -> int:
-        """Thread blocks of a system in a group launch (ffg_problem_solve_batch's
-        FFG_BATCH_CTA_GROUPS rule: group_rows rows per block, 2 to grid)."""
+        """Thread blocks of a system in a group launch, 0 when it goes alone."""
+        if self.shape is not None:
+            return self.shape(key)
         return max(2, min(-(-free_dofs(key) // self.group_rows), self.grid))
 
     def _large_batch(self, head: Request, can_host) -> Batch:
         picked, counts = [head], Counter({head.key: 1})
-        used = self.group_ctas(head.key)
-        if self.groups:
+        used = self.group_ctas(head.key) if self.groups else 0
+        if used:
             for r in list(self.queue)[1:]:
                 if len(picked) == self.max_groups:
                     break
                 if self.is_small(r):
                     continue
                 g = self.group_ctas(r.key)
-                if used + g > self.grid or not can_host(r.key, counts[r.key] + 1):
+                if not g or used + g > self.grid or not can_host(r.key, counts[r.key] + 1):
                     continue
                 picked.append(r)
                 counts[r.key] += 1
                 used += g
         for r in picked:
             self.queue.remove(r)
-        return Batch("cta_groups" if self.groups else "whole_device", picked, 0)
+        return Batch("cta_groups" if used else "whole_device", picked, 0)
 
     def busy_counts(self) -> Counter:
         return Counter(r.key for b in self.inflight for r in b.requests)
@@ -298,6 +302,7 @@ class DeviceEngine:
         self.idle: Dict[Tuple[str, int], List[_Mesh]] = {}
         self.bytes: Dict[Tuple[str, int], int] = {}
         self.last_use: Dict[Tuple[str, int], float] = {}
+        self.shapes: Dict[Tuple[str, int], int] = {}  # group_ctas by mesh size
         self.max_instances = max_instances
         self.options = options or SolverOptions(method="pcg", preconditioner="jacobi",
                                                 tolerance=1e-10, precision="mixed",
@@ -360,6 +365,15 @@ class DeviceEngine:
                 return False
             self._create(key)
         return True
+
+    def group_ctas(self, key) -> int:
+        """Thread blocks that a "cta_groups" batch gives this mesh size (0: it is
+        not kept on chip), from the library."""
+        if key not in self.shapes:
+            if not self.can_host(key):
+                return 0
+            self.shapes[key] = self.meshes[key][0].problem.group_ctas(self.options.precision)
+        return self.shapes[key]
 
     def prepare(self, requests: List[Request]) -> float:
         """Create the problems of every mesh size in `requests` ahead of time
@@ -457,7 +471,7 @@ def run_requests(reqs: List[Request], small_rows: int = 32768, max_batch: int = 
     setup = eng.prepare(reqs)
     sms = torch.cuda.get_device_properties(device).multi_processor_count
     sch = Scheduler(small_rows=small_rows, max_batch=max_batch, streams=streams, groups=groups,
-                    grid=sms)
+                    grid=sms, shape=eng.group_ctas)
     t0 = time.perf_counter()
     res = serve(reqs, eng, sch) if reqs else []
     wall = time.perf_counter() - t0

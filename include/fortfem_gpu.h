@@ -480,6 +480,9 @@ void ffg_problem_phase_times(int handle, double *seconds, int *status);
 #define FFG_BATCH_CTA_PER_SYSTEM 0
 #define FFG_BATCH_WHOLE_DEVICE 1
 #define FFG_BATCH_CTA_GROUPS 2
+/* The thread blocks that FFG_BATCH_CTA_GROUPS gives this system on chip, in a
+ * solve of this precision; 0 where it streams the operator. */
+void ffg_problem_group_ctas(int handle, int precision, int *ctas, int *status);
 void ffg_problem_solve_batch(int count, const int *handles, const double *const *vertices,
                              const double *coef_a, const double *coef_b,
                              const double *const *cell_a, const double *const *cell_b,

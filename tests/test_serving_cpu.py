@@ -218,3 +218,20 @@ def test_evictions_spare_the_sizes_of_the_batch_being_formed():
     assert eng2.can_host(a)
     assert not eng2.can_host(a, 2)
     assert len(eng2.meshes[a]) == 1
+
+
+def test_scheduler_takes_the_groups_from_the_engine():
+    """Blocks as the library says; a size it keeps off the chip goes alone on the
+    whole device and joins nobody's launch."""
+    shape = {("p1", 50): 24, ("p1", 60): 74, ("p2", 30): 0, ("p2", 12): 37}
+    sch = S.Scheduler(small_rows=100, groups=True, grid=148, shape=shape.get)
+    sizes = [("p1", 50), ("p2", 30), ("p1", 60), ("p2", 12), ("p1", 50), ("p2", 30)]
+    for i, (family, n) in enumerate(sizes):
+        sch.queue.append(S.Request(i, family, n, 1, 0.0))
+    taken = []
+    while sch.queue:
+        b = sch.next_batch(lambda k, c: True)
+        taken.append((b.mode, [r.rid for r in b.requests]))
+    # 24 + 74 + 37 fit, another 24 does not
+    assert taken == [("cta_groups", [0, 2, 3]), ("whole_device", [1]), ("cta_groups", [4]),
+                     ("whole_device", [5])]

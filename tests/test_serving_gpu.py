@@ -127,3 +127,20 @@ def test_same_size_requests_share_a_batch_and_overlap():
     # different seeds on one mesh size give different systems
     assert not np.array_equal(got[0].solution, got[1].solution)
     eng.close()
+
+
+def test_group_sizes_come_from_the_library():
+    """The engine's group is the library's for the operator's bytes: a k-th of the
+    SMs, fewer for the short rows of P1 than for P2 of as many rows, 0 beyond the
+    chip and in FP16."""
+    import torch
+    from fortfem_b200 import api
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    eng = S.DeviceEngine(0)
+    p1, p2 = eng.group_ctas(("p1", 296)), eng.group_ctas(("p2", 22))   # 87,025 and 79,507 rows
+    assert 0 < p1 < p2 and all(g in [sms // k for k in range(1, 17)] for g in (p1, p2))
+    assert eng.group_ctas(("p2", 44)) == 0
+    prob = eng.meshes[("p1", 296)][0].problem
+    assert prob.group_ctas("mixed") == p1 <= prob.group_ctas("fp64")
+    assert prob.group_ctas("mixed16") == 0
+    eng.close()
