@@ -984,7 +984,8 @@ void ffg_problem_autotune(int handle, const double *vertices, double ca, double 
   if ((st = time_assembly(best, best_ms))) goto done;
   rep.default_assembly_ms = best_ms;
   {
-    // element kernel shapes first, then the column gather's block size
+    // element kernel shapes first, then the column gather's block size; only
+    // variants that reach the kernels this problem runs
     std::vector<LaunchTuning> cands;
     if (t.family == FFG_TETRA_NEDELEC && P->assembly_precision == FFG_ASSEMBLY_TF32X3) {
       for (int c : {1, 2}) {
@@ -1006,7 +1007,9 @@ void ffg_problem_autotune(int handle, const double *vertices, double ca, double 
       if (ms < best_ms) { best_ms = ms; best = x; }
     }
     const LaunchTuning base = best;
+    // (the slice gather's block size is its own)
     for (int th : {64, 128, 256}) {
+      if (sell_by_slices(t, P->S)) break;
       LaunchTuning x = base;
       x.col_threads = th;
       double ms = 0;
@@ -1047,7 +1050,9 @@ void ffg_problem_autotune(int handle, const double *vertices, double ca, double 
     if ((st = time_solve(256, sms_best))) goto done;
     rep.default_solve_ms = sms_best;
     int best_cost = 256;
+    // (a cluster's slices are cut without it)
     for (int cost : {16, 64, 128, 512, 1024}) {
+      if (pcg_on_cluster(P->S, o.precision)) break;
       double ms = 0;
       if ((st = time_solve(cost, ms))) goto done;
       if (ms < sms_best) { sms_best = ms; best_cost = cost; }

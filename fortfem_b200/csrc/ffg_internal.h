@@ -251,6 +251,8 @@ int pcg_launch_batch(int count, const DeviceSell *const *A, const double *const 
 // memory holds the operator (pcg_group_shape), or, streaming an operator that no
 // group holds or an FP16 one, a CTA for every 16384 rows.
 int pcg_group_ctas(const DeviceSell &A, int precision);  // on chip; 0: streamed
+// Whether a solve of its own runs on one thread-block cluster.
+bool pcg_on_cluster(const DeviceSell &A, int precision);
 int pcg_launch_groups(int count, const DeviceSell *const *A, const double *const *b,
                       double *const *x, const ffg_solver_options &opts, SolveWork *const *w,
                       cudaStream_t stream, std::string &msg);
@@ -385,6 +387,9 @@ int launch_weighted_weights(const Topology &t, const DeviceTopology &dt, const A
 int launch_nedelec(const Topology &t, const ElementTables &tab, const DeviceTopology &dt,
                    const AssemblyInputs &in, double *elem, double *cell_rhs, int *err,
                    cudaStream_t s, bool load_only = false);
+// Whether an assembly into this operator goes by the slice gather.
+bool sell_by_slices(const Topology &t, const DeviceSell &sell);
+
 // Column-owner gather into the constrained operator (element matrices from
 // `elem`, FP64 nb x nb per cell, or `elem32`, FP32 column-major with leading
 // dimension ld32 and cs32 floats per cell).  With `sell` set the

@@ -896,6 +896,16 @@ int launch_nedelec(const Topology &t, const ElementTables &tab, const DeviceTopo
   return launch_nedelec_oriented(t, *dt.ort, dt, in, elem, cell_rhs, err, s, load_only);
 }
 
+namespace {
+int sell_slice_lanes(const Topology &t, const DeviceSell &sell) {
+  return sell.inc_range ? slice_lanes(t.family, t.nb, t.max_column) : 0;
+}
+}  // namespace
+
+bool sell_by_slices(const Topology &t, const DeviceSell &sell) {
+  return sell_slice_lanes(t, sell) != 0;
+}
+
 int launch_columns(const Topology &t, const ElementTables &tab, const DeviceTopology &dt,
                    const AssemblyInputs &in, const double *geo, int stride,
                    const double *cell_rhs, const double *elem, const int64_t *col_ptr,
@@ -922,7 +932,7 @@ int launch_columns(const Topology &t, const ElementTables &tab, const DeviceTopo
                        col_bytes <= kColSmem;
   const int wpb = by_warp ? std::max(1, std::min(8, kColSmem / col_bytes)) : 0;
   // SELL rows by the slice gather
-  const int lanes = sell && sell->inc_range ? slice_lanes(t.family, t.nb, t.max_column) : 0;
+  const int lanes = sell ? sell_slice_lanes(t, *sell) : 0;
   if (lanes) {
     SliceArgs A;
     A.range = sell->inc_range;

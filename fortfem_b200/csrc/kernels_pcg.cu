@@ -1640,6 +1640,10 @@ cudaError_t launch_streamed_groups(int count, const PcgParams *sys, cudaStream_t
 }
 }  // namespace
 
+bool pcg_on_cluster(const DeviceSell &A, int precision) {
+  return pcg_cluster_size(A, precision, false) != 0;
+}
+
 int pcg_group_ctas(const DeviceSell &A, int precision) {
   int grid = 0, slices = 0;
   return pcg_grid_size(&grid) ? 0 : pcg_group_shape(A, precision, grid, &slices);

@@ -375,9 +375,11 @@ typedef struct {
   int element_threads;     /* Nedelec FP64 element kernels: threads per CTA (256) */
   int element_ctas_per_sm; /* the matrix kernel's grid target in CTAs per SM (the
                               entry range of a cell tile is split to reach it) */
-  int column_threads;      /* column-owner gather: threads per block */
+  int column_threads;      /* column-owner gather (triangle Lagrange, columns too
+                              long for the slice gather, CSC): threads per block */
   int tc_ctas_per_sm;      /* 3xTF32 tensor-core kernel: CTAs per SM (1 or 2) */
-  int slice_cost;          /* PCG work partition: cost of a slice beyond its entries */
+  int slice_cost;          /* PCG work partition of the whole device: cost of a slice
+                              beyond its entries */
   double assembly_ms;         /* best assembly time measured (device-resident inputs) */
   double default_assembly_ms; /* the built-in defaults, same measurement */
   double solve_ms;            /* best time of a fixed 60-iteration mixed PCG run */
@@ -388,8 +390,9 @@ typedef struct {
  * Chooses the problem's launch shapes by measurement on its own inputs (as
  * ffg_problem_solve takes them): the element matrix kernel's grid (Nedelec
  * FP64) or the tensor-core kernel's CTAs per SM (3xTF32), the column
- * gather's block size, then the PCG work partition's slice cost, each
- * candidate timed with CUDA events (best of three) and the fastest kept for
+ * gather's block size, then the PCG work partition's slice cost, where the
+ * problem's assembly and mixed solve run a kernel that has them; each
+ * candidate is timed with CUDA events (best of three) and the fastest kept for
  * every following assembly and solve of the problem.  Results of assembly and
  * solve do not depend on the shapes except through the CTA partition of the
  * PCG dot products (reduced in a fixed order for a given partition).  Fills

@@ -55,3 +55,28 @@ def test_autotune_keeps_results_and_reports_times(family, degree):
             assert np.array_equal(R2.val, R0.val)
         with pytest.raises(ff.FortfemError):
             prob.set_tuning({**tune, "element_threads": 100})
+
+
+@pytest.mark.parametrize("family,degree,n", [
+    (K.FFG_TRIANGLE_P1, 1, 20), (K.FFG_TRIANGLE_P1, 1, 40), (K.FFG_TETRA_LAGRANGE, 1, 6),
+    (K.FFG_TETRA_LAGRANGE, 2, 5), (K.FFG_TETRA_NEDELEC, 1, 5), (K.FFG_TETRA_NEDELEC, 2, 4),
+])
+def test_autotune_leaves_shapes_that_reach_no_kernel(family, degree, n):
+    """Small systems: rows by the slice gather, mixed solves on one cluster.  Neither
+    the column gather's block size nor the slice cost reaches them, so both keep
+    the default and no candidate's noise is taken for a gain."""
+    v, t = oracle.unit_square_mesh(n) if family == K.FFG_TRIANGLE_P1 else oracle.box_mesh([n] * 3)
+    with ff.Problem(family, degree, t, len(v)) as prob:
+        tune = prob.autotune(v, 1.0, 1.0)
+        assert tune["column_threads"] == 0 and tune["slice_cost"] == 256
+        assert tune["solve_ms"] == tune["default_solve_ms"]
+        if family != K.FFG_TETRA_NEDELEC:
+            assert tune["assembly_ms"] == tune["default_assembly_ms"]
+
+
+def test_autotune_times_the_column_gather_of_triangles():
+    v, t = oracle.unit_square_mesh(12)
+    with ff.Problem(K.FFG_TRIANGLE_LAGRANGE, 3, t, len(v)) as prob:
+        tune = prob.autotune(v, 1.0, 1.0)
+        assert tune["column_threads"] in (0, 64, 128, 256)
+        assert tune["assembly_ms"] <= tune["default_assembly_ms"]
