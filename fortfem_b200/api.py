@@ -172,33 +172,43 @@ def unit_square_mesh(n: int):
 _CSC_BOUND_BYTES = 1 << 30
 
 
+def _csc_arrays(n, cap):
+    return np.empty(n + 1, np.int64), np.empty(cap, np.int32), np.empty(cap)
+
+
 def _csc_call(fn, args, where, n_cells=0, nb=0):
     """One call of a CSC entry point.  With the element size nb given, the
     arrays are made for the largest pattern that n_cells elements can have and
-    cut to the one returned: asking for the size first builds the topology
-    twice, which is most of the call."""
+    shrunk to the one returned: asking for the size first builds the topology
+    twice, which is most of the call.  Where there is no address space for
+    them, the size is asked for."""
     lib = K.load()
     nd = C.c_int(0)
     nz = C.c_int64(0)
     st = C.c_int(0)
     cap = n_cells * nb * nb
-    if not (0 < nb and 0 < cap * 12 <= _CSC_BOUND_BYTES):
+    arrays = None
+    if 0 < nb and 0 < cap * 12 <= _CSC_BOUND_BYTES:
+        try:
+            arrays = _csc_arrays(n_cells * nb, cap)
+        except MemoryError:
+            pass
+    if arrays is None:
         getattr(lib, fn)(*args, C.c_int64(0), C.byref(nd), C.byref(nz), None, None, None,
                          C.byref(st))
         if st.value not in (K.FFG_OK, K.FFG_CAPACITY):
             return None, Status.of(st.value, where)
-        n, cap = nd.value, nz.value
-    else:
-        n = n_cells * nb
-    cp = np.empty(n + 1, np.int64)
-    ri = np.empty(cap, np.int32)
-    val = np.empty(cap)
-    getattr(lib, fn)(*args, C.c_int64(cap), C.byref(nd), C.byref(nz), _ptr(cp), _ptr(ri),
-                     _ptr(val), C.byref(st))
+        cap = nz.value
+        arrays = _csc_arrays(nd.value, cap)
+    getattr(lib, fn)(*args, C.c_int64(cap), C.byref(nd), C.byref(nz), *map(_ptr, arrays),
+                     C.byref(st))
     if st.value:
         return None, Status.of(st.value, where)
     n = nd.value
-    return CscMatrix(n, n, cp[:n + 1], ri[:nz.value], val[:nz.value]), Status()
+    # in place: what the result does not need is unmapped
+    for a, size in zip(arrays, (n + 1, nz.value, nz.value)):
+        a.resize(size, refcheck=False)
+    return CscMatrix(n, n, *arrays), Status()
 
 
 def _lagrange_nb(p):
