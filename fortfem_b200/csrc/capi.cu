@@ -358,7 +358,6 @@ int assemble(Problem &P, const double *vertices, double ca, double cb, const dou
     }
     if (P.assembly_precision == FFG_ASSEMBLY_TF32X3) {
       // matrices on the tensor cores (FP32, leading dimension tc.ld), loads in FP64
-      if (!P.tc.bimage && (st = tc_build_plan(t, P.ort, P.tc, s))) return st;
       if (in.samples) {
         st = launch_nedelec(t, P.tab, P.dt, in, P.elem, P.cell_rhs, P.err, s, true);
       } else {
@@ -1087,6 +1086,10 @@ void ffg_problem_set_assembly_precision(int handle, int precision, int *status) 
       (P->topo.family != FFG_TETRA_NEDELEC || !tc_supported_order(P->topo.degree))) {
     *status = FFG_INVALID_INPUT;
     return;
+  }
+  // its tables now, so that no assembly allocates
+  if (precision == FFG_ASSEMBLY_TF32X3 && !P->tc.bimage) {
+    if (const int st = tc_build_plan(P->topo, P->ort, P->tc, 0)) { *status = st; return; }
   }
   P->assembly_precision = precision;
   *status = FFG_OK;

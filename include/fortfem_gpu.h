@@ -412,7 +412,8 @@ void ffg_problem_set_tuning(int handle, const ffg_tuning *tuning, int *status);
  * the contraction as a GEMM on the tensor cores (tcgen05, TF32 hi/lo operand
  * split, three products accumulated in FP32) against the same oriented
  * tensors: entries carry about 1e-7 relative error, the geometry and the
- * loads stay FP64.
+ * loads stay FP64.  Its tables are allocated by this call, at its first use
+ * (FFG_OUT_OF_MEMORY: the precision is as before).
  * Other orders and families return FFG_INVALID_INPUT. */
 void ffg_problem_set_assembly_precision(int handle, int precision, int *status);
 

@@ -157,3 +157,25 @@ def test_tf32x3_solve_is_backward_stable_for_the_fp64_matrix(k):
     print(f"order {k}: ||b - A64 x3|| / ||b|| = {res / np.linalg.norm(rhs):.2e}, "
           f"bound {bound / np.linalg.norm(rhs):.2e}")
     assert res <= bound
+
+
+@pytest.mark.parametrize("k", [4, 6])
+def test_first_tf32x3_assembly_allocates_nothing(k):
+    """The kernel's tables (tens of MB at order 6) come with the selection."""
+    import torch
+    v, t = oracle.box_mesh([2, 2, 2])
+    with ff.Problem(K.FFG_TETRA_NEDELEC, k, t, len(v), boundary="all") as prob:
+        opts = ff.SolverOptions(method="pcg", preconditioner="jacobi", tolerance=1e-6,
+                                precision="mixed", max_iterations=100000)
+        src = synth.trig_vector_source(k)(prob.sample_points(v))
+        prob.solve(v, 1.0, 50.0, None, None, src, None, opts)
+
+        def free():
+            torch.cuda.synchronize()
+            return torch.cuda.mem_get_info()[0]
+
+        start = free()
+        prob.set_assembly_precision("tf32x3")
+        chosen = free()
+        prob.solve(v, 1.0, 50.0, None, None, src, None, opts)
+        assert free() == chosen < start
