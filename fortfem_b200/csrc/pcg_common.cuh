@@ -36,7 +36,9 @@ struct PcgParams {
   float2 *zpf0, *zpf1;       // mixed mode after a switch to direct A p: (z, p) pairs
   double *rd, *qd;
   double2 *zpd0, *zpd1;
-  double *partial;  // partial sums [2][2][grid], or messages (pcg_message_bytes)
+  // partial sums [2][2][grid] and the verdicts on the limit [2], or messages
+  // (pcg_message_bytes)
+  double *partial;
   unsigned int *bar;
   int *control;     // [0] error status
   double *result;   // kResultDoubles
